@@ -169,7 +169,7 @@ __global__ void k_step_tail(const uint32_t *qstart, uint32_t N, DevCounters *cnt
 
 void free_all(glint_ctx *c) {
     void *ptrs[] = {c->d_pts, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj_gid, c->d_obj_lv, c->d_obj_leaf, c->d_order, c->d_grid_count,
-                    c->d_grid_start, c->d_grid_cursor, c->d_sorted, c->d_rank_of, c->d_sxy, c->d_sL, c->d_leaf_work,
+                    c->d_grid_start, c->d_grid_cursor, c->d_sorted, c->d_rank_of, c->d_sxy, c->d_sm, c->d_leaf_work,
                     c->d_nodes, c->d_low, c->d_sstack, c->d_gstack, c->d_split, c->d_evscan, c->d_cand, c->d_newgid,
                     c->d_events, c->d_evpos, c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
                     c->d_qstart, c->d_qlist, c->d_qtmp, c->d_tcount, c->d_tstart, c->d_tcursor, c->d_tlist, c->d_tab,
@@ -219,6 +219,10 @@ Frame make_frame(const glint_box &mbr, const glint_schema_node &root, double r, 
     f.r2 = (float)(r * r);
     f.band0 = (float)(64.0 * std::ldexp(1.0, -24) * r * r);
     f.band1 = (float)(4.0 * r);
+    const double mid = std::fabs(0.5 * (ly + hy));
+    f.a0 = std::isfinite(mid) ? (90.0 - mid) * kPIh / 180.0 : 0.0;
+    f.s0 = std::sin(f.a0);
+    f.c0 = std::cos(f.a0);
     return f;
 }
 
@@ -403,7 +407,7 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     ALLOC(c->d_sorted, N);
     ALLOC(c->d_rank_of, N);
     ALLOC(c->d_sxy, N);
-    ALLOC(c->d_sL, N);
+    ALLOC(c->d_sm, N);
     ALLOC(c->d_leaf_work, G);
     ALLOC(c->d_big, G);
     ALLOC(c->d_nodes, S);

@@ -315,6 +315,7 @@ struct Frame {
     float r2;            /* r^2 */
     float band0;         /* 64 u r^2 */
     float band1;         /* 4 r */
+    double a0, s0, c0;   /* an angle near the map's middle latitude, its sin and cos */
 };
 
 constexpr double kFxLimit = 1152921504606846976.0; /* 2^60 */
@@ -343,6 +344,27 @@ __device__ inline float c_of_lat(double lat, const Frame &f) {
     if (a == 90.0) a = 89.0;
     const float t = (float)__dsub_rn(90.0, a);
     return sinf(t * f.kdeg) * f.kc;
+}
+
+/* metres per degree of longitude at latitude lat in FP64, 1 / L to a few
+ * 2^-50: the FP64 form of the refine stage decides with it outside a band of
+ * 2^-36, and takes the reference's own L inside.  Within 0.02 rad (127 km) of
+ * the frame's middle the sin is its Taylor expansion there to the fifth
+ * power (remainder below 0.02^6 / 720 = 9e-14): 12 FP64 operations where the
+ * library's sin and L's divisions are about 60. */
+__device__ inline double metres_per_degree(double lat, const Frame &f) {
+    const double la = fabs(lat) == 90.0 ? 89.0 : fabs(lat);
+    const double x = __dmul_rn(__dsub_rn(90.0, la), kPI / 180.0), d = __dsub_rn(x, f.a0);
+    double s;
+    if ((unsigned long long)__double_as_longlong(fabs(d)) <= 0x3f947ae147ae147bull) { /* 0.02 */
+        const double d2 = __dmul_rn(d, d);
+        const double ev = __fma_rn(d2, __fma_rn(d2, 1.0 / 24.0, -0.5), 1.0);
+        const double od = __dmul_rn(d, __fma_rn(d2, __fma_rn(d2, 1.0 / 120.0, -1.0 / 6.0), 1.0));
+        s = __fma_rn(f.s0, ev, __dmul_rn(f.c0, od));
+    } else {
+        s = sin(x);
+    }
+    return __dmul_rn(s, 40076000.0 / 360.0);
 }
 
 /* the per-first-point screening limits */

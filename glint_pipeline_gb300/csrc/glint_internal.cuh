@@ -9,7 +9,7 @@
  *   sxy         double2[N]   coordinates gathered in that order (leaf tiles)
  *   sipos, sc   [N]          fixed-point coordinates (i64 pair) and screening scale, same order
  *   sfpos, fpos float2[N]    FP32 coordinates (meeting boxes), sorted and by object id
- *   sL          double[N]    degree_per_meter_longitude with CUDA sin (plain form only)
+ *   sm          double[N]    metres per degree of longitude, FP64 (plain form only)
  *   nodes       DNode[S]     64-byte schema records (comparison keys), low corners in
  *                            low[S], fixed-point boxes in ibox[S]
  *   stacks      u32[S], u32[G]  free schema / grid slots (workbench.h:118-128)
@@ -178,7 +178,7 @@ struct glint_ctx {
     uint32_t *d_sorted = nullptr;          /* [N] */
     uint32_t *d_rank_of = nullptr;         /* [N] sorted position of each object */
     double2 *d_sxy = nullptr;
-    double *d_sL = nullptr;                /* [N] sorted L (plain form only) */
+    double *d_sm = nullptr;                /* [N] sorted metres per degree of longitude (plain form only) */
     longlong2 *d_sipos = nullptr;          /* [N] sorted fixed-point coordinates */
     float2 *d_sfpos = nullptr;             /* [N] sorted f32 coordinates (meeting boxes) */
     float *d_sc = nullptr;                 /* [N] sorted metres per unit along x */

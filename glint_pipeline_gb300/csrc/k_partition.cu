@@ -205,14 +205,15 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
 }
 
 /* per object, in leaf-major order: the coordinates, their fixed-point and
- * FP32 forms and the screening scale cx; L with CUDA sin for the plain form;
+ * FP32 forms and the screening scale cx; metres per degree of longitude in
+ * FP64 for the plain form;
  * each object's sorted position */
 struct GatherOut {
     double2 *sxy;
     longlong2 *sipos;
     float2 *sfpos;
     float *sc;
-    double *sL;        /* null: not needed */
+    double *sm;        /* null: not needed */
     float2 *fpos;      /* by object id */
     uint32_t *rank_of;
 };
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(256) k_gather(const uint32_t *__restrict__ sor
         const float2 fp = make_float2((float)p.x, (float)p.y);
         o.sfpos[i] = fp;
         o.fpos[pid] = fp;
-        if (o.sL) o.sL[i] = dpm_lon_fast(p.y);
+        if (o.sm) o.sm[i] = metres_per_degree(p.y, f);
         o.rank_of[pid] = i;
     }
 }
@@ -258,7 +259,7 @@ cudaError_t launch_partition(glint_ctx *c, uint32_t /*cur_time*/) {
     o.sipos = c->d_sipos;
     o.sfpos = c->d_sfpos;
     o.sc = c->d_sc;
-    o.sL = c->cfg.precision_mode == 1 ? nullptr : c->d_sL;
+    o.sm = c->cfg.precision_mode == 1 ? nullptr : c->d_sm;
     o.fpos = c->d_fpos;
     o.rank_of = c->d_rank_of;
     k_gather<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_sorted, N, c->d_pts, o, c->frame);

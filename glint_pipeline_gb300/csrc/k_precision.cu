@@ -1,16 +1,21 @@
 /*
  * k_precision.cu -- the precision form of the refine stage: every candidate
- * pair is first screened in FP32 on exact fixed-point coordinate differences
- * (the Frame of glint_device.cuh), and only the pairs whose screened squared
- * distance lies inside the guard band around r^2 are re-tested with the
- * reference's FP64 arithmetic (point_le_exact), so the contact set - and every
- * meeting - stays identical to the reference's.
+ * pair is screened in FP32 on offsets from its leaf (refine_common.cuh), and
+ * only the pairs whose screened squared distance lies inside the guard band
+ * around r^2 are re-tested with the reference's FP64 arithmetic
+ * (point_le_exact), so the contact set - and every meeting - stays identical
+ * to the reference's.
  *
  * The reference's test (tracing/refinement.cpp:19-31 with Point::distance,
  * geometry/geometry.h:40-48) divides the longitude difference by L(y1) of the
- * checking object; the screen multiplies the integer difference by that
+ * checking object; the screen multiplies the offset difference by that
  * object's cx = 1/(L(y1) S).  No FP64 instruction runs per pair outside the
  * band: on sm_103a FP64 issues at a small fraction of the FP32 rate.
+ *
+ * Bound: issue slots at small tables, random record access at large ones.
+ * Dealing pairs to lanes by number and loading 32 checks at a time took 1M
+ * objects from 290 to 215 us, 2M in dense spots from 1562 to 1414 us and 10M
+ * (34-GB table) from 10.4 to 9.5 ms.
  */
 #include <algorithm>
 #include <cstring>
@@ -23,184 +28,21 @@ namespace glint {
 
 constexpr int kPrecWarps = 4;
 
-/* one screened test; p1 scale cx, p2 scale c2 (a NaN in either forces the
- * exact path) */
-__device__ inline int screen_pair(long long dx, long long dy, float cx, float c2, const Frame &f) {
-    const Screen s = make_screen(__fmaf_rn(0.0f, c2, cx), f);
-    return fx_screen(dx, dy, s, f.cy);
-}
-
-/* one warp's shared memory: its leaf's members (X Y as i64; cx fx fy as f32;
- * id) and its contact queue */
-struct PrecSmem {
-    long long *sX, *sY;
-    float *sC, *sFx, *sFy;
-    uint32_t *sid;
-    QEntry *Q;
-};
-
-__host__ __device__ inline size_t prec_warp_bytes(uint32_t cap) {
-    const size_t per_warp = (size_t)cap * 32 + sizeof(QEntry) * kQueue + 64;
-    return (per_warp + 63) & ~(size_t)63;
-}
-
-__device__ inline PrecSmem prec_smem(unsigned char *base, uint32_t cap) {
-    PrecSmem m;
-    m.sX = reinterpret_cast<long long *>(base);
-    m.sY = m.sX + cap;
-    m.sC = reinterpret_cast<float *>(m.sY + cap);
-    m.sFx = m.sC + cap;
-    m.sFy = m.sFx + cap;
-    m.sid = reinterpret_cast<uint32_t *>(m.sFy + cap);
-    m.Q = reinterpret_cast<QEntry *>(((uintptr_t)(m.sid + cap) + 15) & ~(uintptr_t)15);
-    return m;
-}
-
-/* a warp's tests and contacts of one context, added to its totals on flush */
-struct PrecTally {
-    unsigned long long cand = 0, hits = 0;
-    uint32_t band = 0;
-};
-
-/* warp-collective: the queued contacts into context a's table, and the
- * warp's counts into its totals */
-__device__ inline void prec_flush(const RefineArgs &a, QEntry *Q, uint32_t &qn, uint32_t tag, PrecTally &t) {
-    drain_queue(a, Q, qn, tag);
-    qn = 0;
-    for (int o = 16; o > 0; o >>= 1) {
-        t.cand += __shfl_down_sync(0xffffffffu, t.cand, o);
-        t.hits += __shfl_down_sync(0xffffffffu, t.hits, o);
-        t.band += __shfl_down_sync(0xffffffffu, t.band, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&a.cnt->candidates, t.cand);
-        atomicAdd(&a.cnt->contacts, t.hits);
-        if (t.band) atomicAdd(&a.cnt->band_pairs, t.band);
-    }
-    t = PrecTally();
-}
-
-/* warp-collective: one work item (leaf g, chunk) of context a */
-__device__ inline void prec_item(const RefineArgs &a, uint32_t g, uint32_t chunk, const PrecSmem &m,
-                                 uint32_t &staged, PrecTally &t, uint32_t &qn, uint32_t tag) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t cap = a.cap;
-    const Frame &f = a.f;
-    long long *sX = m.sX, *sY = m.sY;
-    float *sC = m.sC, *sFx = m.sFx, *sFy = m.sFy;
-    uint32_t *sid = m.sid;
-    QEntry *Q = m.Q;
-    const uint32_t s0 = a.grid_start[g];
-    const uint32_t cnt_g = a.grid_count[g];
-    const uint32_t k = cnt_g < cap ? cnt_g : cap;
-    if (g != staged) {
-        for (uint32_t i = lane; i < k; i += 32) {
-            const longlong2 ip = a.sipos[s0 + i];
-            const float2 fp = a.sfpos[s0 + i];
-            sX[i] = ip.x;
-            sY[i] = ip.y;
-            sC[i] = a.sc[s0 + i];
-            sFx[i] = fp.x;
-            sFy[i] = fp.y;
-            sid[i] = a.sorted[s0 + i];
-        }
-        __syncwarp();
-        staged = g;
-    }
-    /* inside checks: p1 = member i, p2 = member j > i */
-    for (uint32_t i = 0; chunk == 0 && i + 1 < k; ++i) {
-        const long long Xi = sX[i], Yi = sY[i];
-        const float ci = sC[i];
-        const uint32_t p1 = sid[i];
-        for (uint32_t jb = i + 1; jb < k; jb += 32) {
-            const uint32_t j = jb + lane;
-            bool hit = false;
-            unsigned long long pw = 0;
-            if (j < k) {
-                ++t.cand;
-                int r = screen_pair(Xi - sX[j], Yi - sY[j], ci, sC[j], f);
-                if (r < 0) {
-                    ++t.band;
-                    const double2 P = a.sxy[s0 + i], Q2 = a.sxy[s0 + j];
-                    r = point_le_exact(P.x, P.y, Q2.x, Q2.y, dpm_lon_fast(P.y), a.ex) ? 1 : 0;
-                }
-                hit = r == 1;
-                if (hit) {
-                    ++t.hits;
-                    pw = pair_word(p1, sid[j]);
-                }
-            }
-            enqueue(a, Q, qn, hit, pw, prio_pack(0, p1, 0, j), sFx[i], sFy[i], hit ? sFx[j] : 0.f,
-                    hit ? sFy[j] : 0.f, tag);
-        }
-    }
-    /* cross-leaf checks that target this leaf, this item's chunk: p1 = the
-     * querier */
-    uint32_t tb, te;
-    item_checks(a, g, chunk, tb, te);
-    for (uint32_t tt = tb; tt < te; ++tt) {
-        const uint2 qe = a.tlist[tt];
-        const uint32_t q = qe.x;
-        const uint32_t qr = a.rank_of[q];
-        const longlong2 qi = a.sipos[qr];
-        const float cq = a.sc[qr];
-        const float2 qf = a.sfpos[qr];
-        const uint32_t qgid = a.obj_gid[q];
-        const bool qstored = (qr - a.grid_start[qgid]) < cap;
-        for (uint32_t jb = 0; jb < k; jb += 32) {
-            const uint32_t j = jb + lane;
-            bool hit = false;
-            unsigned long long pw = 0;
-            if (j < k) {
-                ++t.cand;
-                const long long dx = qi.x - sX[j], dy = qi.y - sY[j];
-                int r = screen_pair(dx, dy, cq, sC[j], f);
-                if (r < 0) {
-                    ++t.band;
-                    const double2 P = a.sxy[qr], M = a.sxy[s0 + j];
-                    r = point_le_exact(P.x, P.y, M.x, M.y, dpm_lon_fast(P.y), a.ex) ? 1 : 0;
-                }
-                hit = r == 1;
-                if (hit) {
-                    ++t.hits;
-                    const uint32_t mm = sid[j];
-                    /* the same pair tested from mm's side comes first in the
-                     * reference's order when mm < q; keep only one event */
-                    if (q > mm && qstored && has_check(a, mm, qgid)) {
-                        int r2 = screen_pair(dx, dy, sC[j], cq, f);
-                        if (r2 < 0) {
-                            ++t.band;
-                            const double2 P = a.sxy[qr], M = a.sxy[s0 + j];
-                            r2 = point_le_exact(M.x, M.y, P.x, P.y, dpm_lon_fast(M.y), a.ex) ? 1 : 0;
-                        }
-                        if (r2 == 1) hit = false;
-                    }
-                    if (hit) pw = pw_of(q, mm);
-                }
-            }
-            enqueue(a, Q, qn, hit, pw, prio_pack(1, q, qe.y, j), qf.x, qf.y, hit ? sFx[j] : 0.f,
-                    hit ? sFy[j] : 0.f, tag);
-        }
-    }
-    __syncwarp();
-}
-
 __global__ void __launch_bounds__(32 * kPrecWarps) k_refine_fp32(RefineArgs a) {
-    extern __shared__ unsigned char smem_raw[];
-    const int w = threadIdx.x >> 5;
-    const PrecSmem m = prec_smem(smem_raw + (size_t)w * prec_warp_bytes(a.cap), a.cap);
-    PrecTally t;
+    extern __shared__ __align__(64) unsigned char smem_raw[];
+    const LeafTile m = leaf_tile(smem_raw + (size_t)(threadIdx.x >> 5) * tile_warp_bytes(a.cap), a.cap);
+    RefineTally t;
     uint32_t qn = 0;
     const uint32_t nwork = a.cnt->n_leaf_work, n_extra = a.cnt->n_extra;
     const uint32_t tag = a.cnt->step_tag;
     bool extra_done = n_extra == 0;
-    uint32_t staged = ~0u;
+    LeafOrigin o;
     for (;;) {
         uint32_t g, chunk;
         if (!claim_item(a, nwork, n_extra, extra_done, g, chunk)) break;
-        prec_item(a, g, chunk, m, staged, t, qn, tag);
+        refine_item<false>(a, g, chunk, m, o, t, qn, tag);
     }
-    prec_flush(a, m.Q, qn, tag, t);
+    refine_flush<false>(a, m.Q, qn, tag, t);
 }
 
 /* ---- the refine stage of many contexts in one launch ---------------------
@@ -239,15 +81,16 @@ __global__ void __launch_bounds__(32 * kPrecWarps) k_refine_fp32_batch(const Ref
                                                                        const uint32_t *__restrict__ ex_off,
                                                                        const uint32_t *__restrict__ wk_off,
                                                                        unsigned int *next, uint32_t cap_max) {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(64) unsigned char smem_raw[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr size_t kArgBytes = (sizeof(RefineArgs) + 63) & ~(size_t)63;
-    unsigned char *base = smem_raw + (size_t)w * (kArgBytes + prec_warp_bytes(cap_max));
+    unsigned char *base = smem_raw + (size_t)w * (kArgBytes + tile_warp_bytes(cap_max));
     RefineArgs *sa = reinterpret_cast<RefineArgs *>(base);
-    const PrecSmem m = prec_smem(base + kArgBytes, cap_max);
+    const LeafTile m = leaf_tile(base + kArgBytes, cap_max);
     const uint32_t E = ex_off[R], W = wk_off[R];
-    PrecTally t;
-    uint32_t qn = 0, tag = 0, staged = ~0u, cur = ~0u;
+    RefineTally t;
+    LeafOrigin o;
+    uint32_t qn = 0, tag = 0, cur = ~0u;
     for (;;) {
         uint32_t v = 0;
         if (lane == 0) v = atomicAdd(next, 1u);
@@ -265,7 +108,7 @@ __global__ void __launch_bounds__(32 * kPrecWarps) k_refine_fp32_batch(const Ref
             chunk = 0;
         }
         if (r != cur) {
-            if (cur != ~0u) prec_flush(*sa, m.Q, qn, tag, t);
+            if (cur != ~0u) refine_flush<false>(*sa, m.Q, qn, tag, t);
             __syncwarp();
             static_assert(sizeof(RefineArgs) % 4 == 0, "RefineArgs words");
             const uint32_t *src = reinterpret_cast<const uint32_t *>(&args[r]);
@@ -273,19 +116,19 @@ __global__ void __launch_bounds__(32 * kPrecWarps) k_refine_fp32_batch(const Ref
             for (uint32_t i = lane; i < sizeof(RefineArgs) / 4; i += 32) dst[i] = src[i];
             __syncwarp();
             cur = r;
-            staged = ~0u;
+            o.g = ~0u;
             tag = sa->cnt->step_tag;
         }
-        prec_item(*sa, g, chunk, m, staged, t, qn, tag);
+        refine_item<false>(*sa, g, chunk, m, o, t, qn, tag);
     }
-    if (cur != ~0u) prec_flush(*sa, m.Q, qn, tag, t);
+    if (cur != ~0u) refine_flush<false>(*sa, m.Q, qn, tag, t);
 }
 
 int refine_prec_warps(uint32_t cap) {
-    return (int)std::max<size_t>(1, std::min<size_t>(kPrecWarps, kMaxBlockSmem / prec_warp_bytes(cap)));
+    return (int)std::max<size_t>(1, std::min<size_t>(kPrecWarps, kMaxBlockSmem / tile_warp_bytes(cap)));
 }
 
-size_t refine_prec_smem_bytes(uint32_t cap) { return (size_t)refine_prec_warps(cap) * prec_warp_bytes(cap); }
+size_t refine_prec_smem_bytes(uint32_t cap) { return (size_t)refine_prec_warps(cap) * tile_warp_bytes(cap); }
 
 cudaError_t launch_refine_precision(glint_ctx *c, const RefineArgs &a) {
     k_refine_fp32<<<152 * 8, 32 * refine_prec_warps(c->cap), refine_prec_smem_bytes(c->cap), c->stream>>>(a);
@@ -298,7 +141,7 @@ cudaError_t launch_refine_precision_batch(const RefineArgs *d_args, uint32_t R, 
                                           uint32_t *wk_off, unsigned int *next, cudaStream_t s) {
     k_refine_batch_prep<<<1, 1, 0, s>>>(d_args, R, ex_off, wk_off, next);
     constexpr size_t kArgBytes = (sizeof(RefineArgs) + 63) & ~(size_t)63;
-    const size_t per_warp = kArgBytes + prec_warp_bytes(cap_max);
+    const size_t per_warp = kArgBytes + tile_warp_bytes(cap_max);
     const int warps = (int)std::max<size_t>(1, std::min<size_t>(kPrecWarps, kMaxBlockSmem / per_warp));
     k_refine_fp32_batch<<<152 * 8, 32 * warps, warps * per_warp, s>>>(d_args, R, ex_off, wk_off, next, cap_max);
     return cudaGetLastError();

@@ -10,12 +10,22 @@
  *
  * Device form: one warp per leaf.  The leaf's stored members (its first
  * min(count, capacity) objects in id order) are staged in shared memory as
- * SoA x / y / L / id; the warp runs the inside pairs i < j and then every
- * cross-leaf check that targets the leaf against the staged members.  Pairs
- * within reach go through the contact queue (refine_common.cuh): a pair found
- * in the table as it stood at the start of the step is touched there, which is
- * what the reference does for it; a pair not found goes to the new list with
- * its position in the reference's sequential check order as priority.
+ * FP32 offsets from the leaf; the warp runs the inside pairs i < j and then
+ * every cross-leaf check that targets the leaf against the staged members
+ * (refine_common.cuh).  A pair whose FP32 distance is beyond reach by more
+ * than the screen's proven error is ruled out there; every other pair goes
+ * through the contact queue and is decided by the FP64 test when the queue is
+ * drained, 32 pairs to a warp instruction.  A contact found in the table as it
+ * stood at the start of the step is touched there, which is what the
+ * reference does for it; a pair not found goes to the new list with its
+ * position in the reference's sequential check order as priority.
+ *
+ * Bound: FP64 issues at 1/64 of the FP32 rate, so the reference's expression
+ * on every candidate (two divisions, a square root: about 45 FP64 operations)
+ * was the whole kernel.  1M objects, 18.7M candidates, 3.0M contacts, GB300:
+ * 4832 us with FP64 on every candidate, 263 us with the bound, the queue and
+ * the division-free test (215 us in the form that accepts by the screen too);
+ * 100k objects, 1.4M candidates: 525 and 22 us.
  *
  * Duplicate pairs: a cross-leaf pair (a, b) is tested from both sides when a
  * has a check on b's leaf and b one on a's leaf.  The reference's second test
@@ -33,127 +43,28 @@ namespace glint {
 constexpr int kRefineWarps = 4;
 
 __global__ void __launch_bounds__(32 * kRefineWarps) k_refine_fp64(RefineArgs a) {
-    extern __shared__ unsigned char smem_raw[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t cap = a.cap;
-    /* per-warp layout: x[cap] y[cap] L[cap] (double), id[cap] (u32), queue */
-    const size_t per_warp = (size_t)cap * 28 + sizeof(QEntry) * kQueue + 64;
-    unsigned char *base = smem_raw + (size_t)w * ((per_warp + 63) & ~(size_t)63);
-    double *sx = reinterpret_cast<double *>(base);
-    double *sy = sx + cap;
-    double *sLm = sy + cap;
-    uint32_t *sid = reinterpret_cast<uint32_t *>(sLm + cap);
-    QEntry *Q = reinterpret_cast<QEntry *>(((uintptr_t)(sid + cap) + 15) & ~(uintptr_t)15);
-
-    unsigned long long cand = 0, hits = 0;
+    extern __shared__ __align__(64) unsigned char smem_raw[];
+    const LeafTile m = leaf_tile(smem_raw + (size_t)(threadIdx.x >> 5) * tile_warp_bytes(a.cap), a.cap);
+    RefineTally t;
     uint32_t qn = 0;
     const uint32_t nwork = a.cnt->n_leaf_work, n_extra = a.cnt->n_extra;
     const uint32_t tag = a.cnt->step_tag;
     bool extra_done = n_extra == 0;
-    uint32_t staged = ~0u;
+    LeafOrigin o;
     for (;;) {
         uint32_t g, chunk;
         if (!claim_item(a, nwork, n_extra, extra_done, g, chunk)) break;
-        const uint32_t s0 = a.grid_start[g];
-        const uint32_t cnt_g = a.grid_count[g];
-        const uint32_t k = cnt_g < cap ? cnt_g : cap;
-        if (g != staged) {
-            for (uint32_t i = lane; i < k; i += 32) {
-                const double2 p = a.sxy[s0 + i];
-                sx[i] = p.x;
-                sy[i] = p.y;
-                sLm[i] = a.sL[s0 + i];
-                sid[i] = a.sorted[s0 + i];
-            }
-            __syncwarp();
-            staged = g;
-        }
-        /* inside checks: p1 = member i, p2 = member j > i (ids ascend with rank) */
-        for (uint32_t i = 0; chunk == 0 && i + 1 < k; ++i) {
-            const double x1 = sx[i], y1 = sy[i], L1 = sLm[i];
-            const uint32_t p1 = sid[i];
-            const float fx1 = (float)x1, fy1 = (float)y1;
-            for (uint32_t jb = i + 1; jb < k; jb += 32) {
-                const uint32_t j = jb + lane;
-                bool hit = false;
-                unsigned long long pw = 0;
-                float fx2 = 0.f, fy2 = 0.f;
-                if (j < k) {
-                    ++cand;
-                    const double x2 = sx[j], y2 = sy[j];
-                    hit = point_le_exact(x1, y1, x2, y2, L1, a.ex);
-                    if (hit) {
-                        ++hits;
-                        pw = pair_word(p1, sid[j]);
-                        fx2 = (float)x2;
-                        fy2 = (float)y2;
-                    }
-                }
-                enqueue(a, Q, qn, hit, pw, prio_pack(0, p1, 0, j), fx1, fy1, fx2, fy2, tag);
-            }
-        }
-        /* cross-leaf checks that target this leaf: this item's chunk */
-        uint32_t tb, te;
-        item_checks(a, g, chunk, tb, te);
-        for (uint32_t t = tb; t < te; ++t) {
-            const uint2 qe = a.tlist[t];
-            const uint32_t q = qe.x;
-            const uint32_t qr = a.rank_of[q];
-            const double2 qp = a.sxy[qr];
-            const double Lq = a.sL[qr];
-            const uint32_t qgid = a.obj_gid[q];
-            const bool qstored = (qr - a.grid_start[qgid]) < cap;
-            const float fqx = (float)qp.x, fqy = (float)qp.y;
-            for (uint32_t jb = 0; jb < k; jb += 32) {
-                const uint32_t j = jb + lane;
-                bool hit = false;
-                unsigned long long pw = 0;
-                float fx2 = 0.f, fy2 = 0.f;
-                if (j < k) {
-                    ++cand;
-                    const double x2 = sx[j], y2 = sy[j];
-                    hit = point_le_exact(qp.x, qp.y, x2, y2, Lq, a.ex);
-                    if (hit) {
-                        ++hits;
-                        const uint32_t m = sid[j];
-                        /* the same pair tested from m's side comes first in the
-                         * reference's order when m < q; keep only one event */
-                        if (q > m && qstored && has_check(a, m, qgid) && point_le_exact(x2, y2, qp.x, qp.y, sLm[j], a.ex))
-                            hit = false;
-                        if (hit) {
-                            pw = pw_of(q, m);
-                            fx2 = (float)x2;
-                            fy2 = (float)y2;
-                        }
-                    }
-                }
-                enqueue(a, Q, qn, hit, pw, prio_pack(1, q, qe.y, j), fqx, fqy, fx2, fy2, tag);
-            }
-        }
-        __syncwarp();
+        refine_item<true>(a, g, chunk, m, o, t, qn, tag);
     }
-    drain_queue(a, Q, qn, tag);
-    for (int o = 16; o > 0; o >>= 1) {
-        cand += __shfl_down_sync(0xffffffffu, cand, o);
-        hits += __shfl_down_sync(0xffffffffu, hits, o);
-    }
-    if (lane == 0) {
-        atomicAdd(&a.cnt->candidates, cand);
-        atomicAdd(&a.cnt->contacts, hits);
-    }
+    refine_flush<true>(a, m.Q, qn, tag, t);
 }
 
-/* shared memory per warp (its leaf's members and its contact queue), and the
- * warps per block that fit the per-block limit (large leaf buffers run with
- * fewer warps per block) */
-static size_t refine_warp_bytes(uint32_t cap) {
-    const size_t per_warp = (size_t)cap * 28 + sizeof(QEntry) * kQueue + 64;
-    return (per_warp + 63) & ~(size_t)63;
-}
+/* the warps per block whose leaf tiles and contact queues fit the per-block
+ * limit of shared memory (large leaf buffers run with fewer) */
 int refine_warps(uint32_t cap) {
-    return (int)std::max<size_t>(1, std::min<size_t>(kRefineWarps, kMaxBlockSmem / refine_warp_bytes(cap)));
+    return (int)std::max<size_t>(1, std::min<size_t>(kRefineWarps, kMaxBlockSmem / tile_warp_bytes(cap)));
 }
-size_t refine_smem_bytes(uint32_t cap) { return (size_t)refine_warps(cap) * refine_warp_bytes(cap); }
+size_t refine_smem_bytes(uint32_t cap) { return (size_t)refine_warps(cap) * tile_warp_bytes(cap); }
 
 /* the chunks beyond the first of every leaf's cross-leaf checks */
 __global__ void __launch_bounds__(256) k_refine_extra(const uint32_t *__restrict__ work,
@@ -179,7 +90,9 @@ RefineArgs refine_args(glint_ctx *c) {
     a.grid_count = c->d_grid_count;
     a.sorted = c->d_sorted;
     a.sxy = c->d_sxy;
-    a.sL = c->d_sL;
+    a.sm = c->d_sm;
+    a.obj_leaf = c->d_obj_leaf;
+    a.ibox = c->d_ibox;
     a.tstart = c->d_tstart;
     a.tlist = c->d_tlist;
     a.sipos = c->d_sipos;
@@ -201,6 +114,9 @@ RefineArgs refine_args(glint_ctx *c) {
     a.chunk = c->chunk;
     a.extra_cap = (uint32_t)std::min<uint64_t>(c->rextra_cap, 0xffffffffu);
     a.ex = make_exact(c);
+    a.m_lat = 1.0 / c->dpm_lat;
+    a.r2 = c->cfg.reach_distance * c->cfg.reach_distance;
+    a.tol = 4.0 * c->cfg.reach_distance * c->band;
     a.cnt = c->d_cnt;
     return a;
 }

@@ -81,7 +81,8 @@ typedef struct glint_config {
     uint32_t CTF_count;            /* configuration::CTF_count (100); must be a square */
     double dProbFalse;             /* workbench::dProbFalse: object-box area above which keys go to the oversize buffer */
     /* ---- this implementation ---- */
-    uint32_t precision_mode;       /* 0: FP64 test on every candidate; 1: FP32 leaf-relative guard band */
+    uint32_t precision_mode;       /* 0: FP64 test on every candidate that an FP32 bound cannot rule out;
+                                      1: FP32 leaf-relative guard band, FP64 inside it */
     uint32_t device;               /* CUDA device ordinal */
     uint64_t new_capacity;         /* per-step new-contact buffer (entries); 0 -> automatic */
     uint64_t check_capacity;       /* cross-leaf check buffer (entries); 0 -> automatic */

@@ -29,9 +29,9 @@ size_t refine_smem_bytes(uint32_t cap);
 uint64_t identify_tiles(uint64_t B);
 cudaError_t noalloc_setup(int device);
 /* stamps cover a whole number of identify tiles (the padding stays empty) */
-inline uint64_t stamp_bytes(uint64_t B) { return identify_tiles(B) * 8192 + 64; }
+inline uint64_t stamp_bytes(uint64_t B) { return (B + 8191) / 8192 * 8192 + 64; }
 /* the new-line bitmap: one bit per 4 slots over the same tiles */
-inline uint64_t newline_words(uint64_t B) { return identify_tiles(B) * (8192 / 128); }
+inline uint64_t newline_words(uint64_t B) { return (B + 8191) / 8192 * (8192 / 128); }
 } // namespace glint
 
 using namespace glint;
@@ -162,9 +162,16 @@ __global__ void k_iota(uint32_t *a, uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = i;
 }
 
-__global__ void k_step_tail(const uint32_t *qstart, uint32_t N, DevCounters *cnt) {
+/* the step's last counts, and its reports join the log */
+__global__ void k_step_tail(const uint32_t *qstart, uint32_t N, const uint32_t *reports, uint64_t log_cap,
+                            DevCounters *cnt) {
     cnt->cross_checks = qstart[N];
     cnt->total_checks = N + qstart[N];
+    const uint32_t total = *reports;
+    cnt->meetings = total;
+    cnt->log_step_begin = cnt->log_head;
+    cnt->log_head += total;
+    if (total > log_cap) atomicOr(&cnt->error_flags, GLINT_EF_LOG_OVERFLOW);
 }
 
 void free_all(glint_ctx *c) {
@@ -542,6 +549,8 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     init_sin_coef(&coef);
     cudaMemcpy(c->d_coef, &coef, sizeof(coef), cudaMemcpyHostToDevice);
     k_fill_empty<<<grid_for(c->B, 256, 152u * 16u), 256, 0, c->stream>>>(c->d_tab, c->B);
+    cudaMemsetAsync(c->d_scan_tmp, 0, c->scan_tmp_bytes, c->stream);
+    cudaMemsetAsync(c->d_scan_tmp_side, 0, c->scan_tmp_bytes, c->stream);
     cudaMemsetAsync(c->d_stamp, 0, stamp_bytes(c->B), c->stream);
     cudaMemsetAsync(c->d_newline, 0, sizeof(uint32_t) * newline_words(c->B), c->stream);
     cudaMemsetAsync(c->d_grid_count, 0, sizeof(uint32_t) * ((size_t)G + 1), c->stream);
@@ -639,7 +648,7 @@ void launch_step_back(glint_ctx *c) {
     launch_keys(c);
     if (tm) cudaEventRecord(c->timers.ev[6], s);
     if (schema) cudaStreamWaitEvent(s, c->join_ev, 0);
-    k_step_tail<<<1, 1, 0, s>>>(c->d_qstart, c->N, c->d_cnt);
+    k_step_tail<<<1, 1, 0, s>>>(c->d_qstart, c->N, c->d_tile_off + c->n_tiles, c->log_cap, c->d_cnt);
     if (tm) cudaEventRecord(c->timers.ev[7], s);
     cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
 }
@@ -737,10 +746,9 @@ static void fill_stats(glint_ctx *c, glint_step_stats *st) {
     st->band_pairs = h.band_pairs;
     st->box_band = h.box_band;
     st->error_flags = h.error_flags;
-    /* kernels per step: partition 9, filter 9, refine 2 (work items, pairs),
-     * insert 1, identify 6 + keys 1, schema update 11, tail 1 (scans count
-     * three each) */
-    st->launches = 9 + 9 + 2 + 1 + 7 + (c->cfg.dynamic_schema ? 11 : 0) + 1;
+    /* kernels per step: partition 7, filter 5, refine 2 (work items, pairs),
+     * insert 1, identify 3 + keys 1, schema update 9, tail 1 */
+    st->launches = 7 + 5 + 2 + 1 + 4 + (c->cfg.dynamic_schema ? 9 : 0) + 1;
     st->meeting_log_size = h.log_head;
     st->kv_count = h.kv_count;
     st->flushed = c->last_flushed ? 1u : 0u;

@@ -285,7 +285,9 @@ namespace glint {
 
 /* ---- utilities (k_util.cu) ---- */
 size_t scan_tmp_bytes(size_t n);
-/* exclusive scan of n u32 values into out[0..n], out[n] = total */
+/* exclusive scan of n u32 values into out[0..n], out[n] = total; tmp holds
+ * scan_tmp_bytes(n) bytes that were zero before its first scan, and in and out
+ * do not overlap */
 cudaError_t scan_u32(const uint32_t *in, uint32_t *out, size_t n, void *tmp, cudaStream_t s);
 void init_sin_coef(SinCoef *host);
 

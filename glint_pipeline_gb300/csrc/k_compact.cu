@@ -703,7 +703,8 @@ extern "C" glint_status glint_store_compact(glint_ctx *c, uint32_t first, uint32
     uint32_t *sval = sc.get<uint32_t>(R), *sval2 = sc.get<uint32_t>(R);
     const uint64_t sort_n = std::max<uint64_t>(std::max<uint64_t>(R, N), O_src + R);
     void *rs_tmp = sc.get<uint8_t>(radix_tmp_bytes(sort_n));
-    void *scan_tmp = sc.get<uint8_t>(scan_tmp_bytes(256 * ((sort_n + 1023) / 1024) + 1 + N + 1));
+    const size_t scan_bytes = scan_tmp_bytes(256 * ((sort_n + 1023) / 1024) + 1 + N + 1);
+    void *scan_tmp = sc.get<uint8_t>(scan_bytes);
     uint32_t *rfirst = sc.get<uint32_t>(N), *rend = sc.get<uint32_t>(N), *nkeys = sc.get<uint32_t>(N);
     float4 *obox = sc.get<float4>(N);
     uint2 *ostart = sc.get<uint2>(N);
@@ -713,6 +714,7 @@ extern "C" glint_status glint_store_compact(glint_ctx *c, uint32_t first, uint32
     if (sc.e != cudaSuccess) return cuda_fail(sc.e, "scratch");
     cudaMemcpyAsync(d_src, hs.data(), sizeof(SrcBlock) * count, cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long) * kNumCounters, s);
+    cudaMemsetAsync(scan_tmp, 0, scan_bytes, s);
     cudaMemsetAsync(rfirst, 0, sizeof(uint32_t) * N, s);
     cudaMemsetAsync(rend, 0, sizeof(uint32_t) * N, s);
 

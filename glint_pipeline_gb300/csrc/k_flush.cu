@@ -78,9 +78,10 @@ struct KeyArgs {
 
 /* the meetings this step wrote to the log become keys */
 __global__ void __launch_bounds__(256) k_keys_append(const glint_meeting *__restrict__ log, uint64_t log_cap,
-                                                     KeyArgs a, DevCounters *cnt) {
-    const uint32_t total = cnt->meetings;
-    const unsigned long long begin = cnt->log_step_begin;
+                                                     const uint32_t *__restrict__ reports, KeyArgs a,
+                                                     DevCounters *cnt) {
+    const uint32_t total = *reports;
+    const unsigned long long begin = cnt->log_head; /* moved in the step's tail */
     const uint32_t end_time_min = cnt->end_time_min;
     const int lane = threadIdx.x & 31;
     for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 - lane < total; i0 += gridDim.x * blockDim.x) {
@@ -842,7 +843,8 @@ KeyArgs key_args(glint_ctx *c) {
 
 /* after identify: this step's meetings become keys */
 cudaError_t launch_keys(glint_ctx *c) {
-    k_keys_append<<<152 * 4, 256, 0, c->stream>>>(c->d_log, c->log_cap, key_args(c), c->d_cnt);
+    k_keys_append<<<152 * 4, 256, 0, c->stream>>>(c->d_log, c->log_cap, c->d_tile_off + c->n_tiles, key_args(c),
+                                                  c->d_cnt);
     return cudaGetLastError();
 }
 

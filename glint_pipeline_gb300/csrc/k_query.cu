@@ -24,11 +24,11 @@
 
 namespace glint {
 
-uint64_t identify_tiles(uint64_t B);
-
 constexpr int kSearchThreads = 512;
 constexpr int kSearchItems = 16;
-constexpr uint32_t kSearchTile = kSearchThreads * kSearchItems; /* = the identify tile */
+constexpr uint32_t kSearchTile = kSearchThreads * kSearchItems;
+
+static uint64_t search_tiles(uint64_t B) { return (B + kSearchTile - 1) / kSearchTile; }
 
 struct SearchArgs {
     const TRec *tab;
@@ -169,7 +169,7 @@ cudaError_t launch_active_search(const glint_ctx *c, uint32_t *bits, uint32_t *t
                                  Scan scan, const uint32_t *d_pids, uint32_t npids, glint_search_info *d_out,
                                  uint64_t cap, unsigned long long *d_n) {
     cudaStream_t s = c->stream;
-    const uint64_t tiles = identify_tiles(c->B);
+    const uint64_t tiles = search_tiles(c->B);
     cudaError_t e = cudaMemsetAsync(bits, 0, sizeof(uint32_t) * (((size_t)c->N + 31) / 32), s);
     if (e != cudaSuccess) return e;
     if (npids) k_search_set_bits<<<grid_for(npids, 256, 152u * 4u), 256, 0, s>>>(d_pids, npids, bits, c->N);
@@ -322,7 +322,7 @@ extern "C" glint_status glint_active_search_noalloc(glint_ctx *c, const uint32_t
         c->last_error = "active search before the first step";
         return GLINT_ERR_STATE;
     }
-    if (c->N > kNaMaxObjects || identify_tiles(c->B) > kNaMaxTiles) {
+    if (c->N > kNaMaxObjects || search_tiles(c->B) > kNaMaxTiles) {
         c->last_error = "glint_active_search_noalloc: context larger than its fixed scratch (objects <= 2^24, "
                         "buckets <= 2^30); use glint_active_search";
         return GLINT_ERR_UNSUPPORTED;

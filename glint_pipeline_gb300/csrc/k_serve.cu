@@ -533,7 +533,9 @@ static cudaError_t server_result_space(glint_server *v, uint64_t n, uint32_t act
     if (e == cudaSuccess) e = cudaMalloc((void **)&v->rv2, sizeof(uint32_t) * cap);
     if (e == cudaSuccess) e = cudaMalloc((void **)&v->rids, sizeof(uint32_t) * cap);
     if (e == cudaSuccess) e = cudaMalloc(&v->rs_tmp, radix_tmp_bytes(cap));
-    if (e == cudaSuccess) e = cudaMalloc(&v->rscan, scan_tmp_bytes(256 * ((cap + 1023) / 1024) + 1));
+    const size_t scan_bytes = scan_tmp_bytes(256 * ((cap + 1023) / 1024) + 1);
+    if (e == cudaSuccess) e = cudaMalloc(&v->rscan, scan_bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(v->rscan, 0, scan_bytes, v->ctx->stream);
     if (e == cudaSuccess && !v->roff) e = cudaMalloc((void **)&v->roff, sizeof(unsigned long long) * (v->slots + 1));
     if (e == cudaSuccess) v->r_cap = cap;
     (void)act;

@@ -159,7 +159,7 @@ cudaError_t radix_sort_u64(unsigned long long *keys, uint32_t *vals, unsigned lo
     const uint64_t tiles = (n + kRsTile - 1) / kRsTile;
     if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
     uint32_t *cnt = static_cast<uint32_t *>(rs_tmp);
-    uint32_t *off = cnt + (size_t)kRsDigits * tiles + 1;
+    uint32_t *off = cnt + (size_t)kRsDigits * tiles; /* 16-byte aligned: whole scan words */
     unsigned long long *src_k = keys, *dst_k = tmp_k;
     uint32_t *src_v = vals, *dst_v = tmp_v;
     int passes = 0;
@@ -188,7 +188,7 @@ cudaError_t radix_sort_u64_varying(unsigned long long *keys, uint32_t *vals, uns
     const uint64_t tiles = (n + kRsTile - 1) / kRsTile;
     if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
     uint32_t *cnt = static_cast<uint32_t *>(rs_tmp);
-    uint32_t *off = cnt + (size_t)kRsDigits * tiles + 1;
+    uint32_t *off = cnt + (size_t)kRsDigits * tiles; /* 16-byte aligned: whole scan words */
     unsigned long long *orand =
         reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(rs_tmp) + radix_tmp_bytes(n) - 16);
     cudaMemsetAsync(orand, 0, sizeof(unsigned long long), s);

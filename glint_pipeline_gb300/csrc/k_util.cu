@@ -2,6 +2,7 @@
  * k_util.cu -- device-wide exclusive scan, the double-double sin
  * coefficients, and the device side of the synthetic trajectory generator.
  */
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -11,96 +12,141 @@
 
 namespace glint {
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
+/* Exclusive scan in one launch: a tile per block, the tiles' running sums
+ * passed on by look-back over status words.  The step runs five scans, most
+ * of them over a few hundred thousand words at most, so launches bound them:
+ * the reduce / scan / down form took three (36 us for the five at 20k
+ * objects), this takes one (26 us) and reads the input once instead of twice.
+ * The scratch starts zeroed.  Its status words carry the scan's number
+ * (epoch), so they need no reset between scans: a word of an earlier scan
+ * reads as not there yet.  Tiles are taken by ticket, so a tile waits only for
+ * tiles that already run; a wait that outlasts kScanPolls adds up the input
+ * before its tile itself. */
+constexpr int kScanThreads = 512;
+constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr uint32_t kScanPolls = 1u << 20;
+
+struct ScanHead {
+    uint32_t epoch, ticket, done, pad;
+};
 
 size_t scan_tmp_bytes(size_t n) {
-    size_t tiles = (n + kScanTile - 1) / kScanTile + 1;
-    return (tiles + 1) * sizeof(uint32_t);
+    const size_t tiles = (n + kScanTile - 1) / kScanTile + 1;
+    return sizeof(ScanHead) + tiles * sizeof(unsigned long long);
 }
 
-__device__ inline uint32_t block_exclusive_scan(uint32_t v, uint32_t *warp_sums, uint32_t &block_total) {
+__device__ inline unsigned long long scan_status(uint32_t epoch, uint32_t flag, uint32_t value) {
+    return ((unsigned long long)((epoch << 2) | flag) << 32) | value;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
+                                                       size_t n, ScanHead *head, uint32_t tiles, bool vec) {
+    constexpr uint32_t kSum = 1, kPrefix = 2;
+    __shared__ uint32_t ws[kScanThreads / 32];
+    __shared__ uint32_t s_tile, s_epoch, s_before;
+    volatile unsigned long long *status = reinterpret_cast<unsigned long long *>(head + 1);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t x = v;
+    if (threadIdx.x == 0) {
+        /* the epoch moves when the last tile is done: all tiles read the same */
+        s_epoch = (*(volatile uint32_t *)&head->epoch + 1) & 0x3fffffffu;
+        s_tile = atomicAdd(&head->ticket, 1u);
+    }
+    __syncthreads();
+    const uint32_t tile = s_tile, epoch = s_epoch;
+    const size_t base = (size_t)tile * kScanTile + (size_t)threadIdx.x * kScanItems;
+    uint32_t v[kScanItems];
+    if (vec && base + kScanItems <= n) {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k += 4) {
+            const uint4 x = *reinterpret_cast<const uint4 *>(in + base + k);
+            v[k] = x.x;
+            v[k + 1] = x.y;
+            v[k + 2] = x.z;
+            v[k + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) v[k] = base + k < n ? in[base + k] : 0u;
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) mine += v[k];
+    uint32_t incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
     }
-    if (lane == 31) warp_sums[wid] = x;
+    if (lane == 31) ws[wid] = incl;
     __syncthreads();
     if (wid == 0) {
-        uint32_t w = (lane < (int)(blockDim.x >> 5)) ? warp_sums[lane] : 0u;
+        uint32_t w = lane < kScanThreads / 32 ? ws[lane] : 0u;
+        const uint32_t own = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
             if (lane >= o) w += y;
         }
-        warp_sums[lane] = w;
+        const uint32_t sum = __shfl_sync(0xffffffffu, w, 31);
+        if (lane < kScanThreads / 32) ws[lane] = w - own;
+        if (lane == 0) status[tile] = scan_status(epoch, tile == 0 ? kPrefix : kSum, sum);
+        uint32_t before = 0;
+        for (long long at = (long long)tile - 1; at >= 0; at -= 32) {
+            /* 32 earlier tiles at once, the nearest on lane 0 */
+            const long long t = at - lane;
+            unsigned long long st = scan_status(epoch, kPrefix, 0);
+            uint32_t polls = 0;
+            if (t >= 0) {
+                do {
+                    st = status[t];
+                } while ((st >> 34) != epoch && ++polls < kScanPolls);
+            }
+            if (__any_sync(0xffffffffu, (st >> 34) != epoch)) {
+                before = 0;
+                for (size_t i = lane; i < (size_t)tile * kScanTile; i += 32) before += in[i];
+                before = __reduce_add_sync(0xffffffffu, before);
+                break;
+            }
+            const unsigned full = __ballot_sync(0xffffffffu, ((uint32_t)(st >> 32) & 3u) == kPrefix);
+            const int upto = full ? __ffs(full) - 1 : 31;
+            before += __reduce_add_sync(0xffffffffu, lane <= upto ? (uint32_t)st : 0u);
+            if (full) break;
+        }
+        if (lane == 0) {
+            if (tile) status[tile] = scan_status(epoch, kPrefix, before + sum);
+            s_before = before;
+            if (tile == tiles - 1) out[n] = before + sum;
+            if (atomicAdd(&head->done, 1u) == tiles - 1) {
+                head->ticket = 0;
+                head->done = 0;
+                head->epoch = epoch;
+            }
+        }
     }
     __syncthreads();
-    uint32_t prefix = (wid > 0 ? warp_sums[wid - 1] : 0u) + x - v;
-    block_total = warp_sums[(blockDim.x >> 5) - 1];
-    __syncthreads();
-    return prefix;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t *in, size_t n, uint32_t *tile_sums) {
-    __shared__ uint32_t ws[32];
-    size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + k < n) s += in[base + k];
-    uint32_t tot;
-    block_exclusive_scan(s, ws, tot);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = tot;
-}
-
-/* one block: exclusive scan of the tile sums in place; total into tile_sums[tiles] */
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t *tile_sums, size_t tiles) {
-    __shared__ uint32_t ws[32];
-    uint32_t carry = 0;
-    for (size_t base = 0; base < tiles; base += kScanThreads) {
-        size_t i = base + threadIdx.x;
-        uint32_t v = i < tiles ? tile_sums[i] : 0u;
-        uint32_t tot;
-        uint32_t p = block_exclusive_scan(v, ws, tot);
-        if (i < tiles) tile_sums[i] = carry + p;
-        carry += tot;
-    }
-    if (threadIdx.x == 0) tile_sums[tiles] = carry;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t *in, uint32_t *out, size_t n,
-                                                           const uint32_t *tile_off, size_t tiles) {
-    __shared__ uint32_t ws[32];
-    size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t s = 0;
+    uint32_t p = s_before + ws[wid] + incl - mine;
+    uint32_t o[kScanItems];
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        v[k] = (base + k < n) ? in[base + k] : 0u;
-        s += v[k];
-    }
-    uint32_t tot;
-    uint32_t p = block_exclusive_scan(s, ws, tot) + tile_off[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < n) out[base + k] = p;
+        o[k] = p;
         p += v[k];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = tile_off[tiles];
+    if (vec && base + kScanItems <= n) {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k += 4)
+            *reinterpret_cast<uint4 *>(out + base + k) = make_uint4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
+            if (base + k < n) out[base + k] = o[k];
+    }
 }
 
 cudaError_t scan_u32(const uint32_t *in, uint32_t *out, size_t n, void *tmp, cudaStream_t s) {
-    size_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles == 0) tiles = 1;
-    uint32_t *ts = (uint32_t *)tmp;
-    k_scan_reduce<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, ts);
-    k_scan_tiles<<<1, kScanThreads, 0, s>>>(ts, tiles);
-    k_scan_down<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, ts, tiles);
+    const uint32_t tiles = (uint32_t)std::max<size_t>(1, (n + kScanTile - 1) / kScanTile);
+    const bool vec = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+    k_scan<<<tiles, kScanThreads, 0, s>>>(in, out, n, (ScanHead *)tmp, tiles, vec);
     return cudaGetLastError();
 }
 

@@ -24,7 +24,6 @@ namespace glint {
 void partition_set_attributes();
 void refine_set_attributes(uint32_t cap);
 void refine_prec_set_attributes(uint32_t cap);
-void schema_set_attributes();
 size_t refine_smem_bytes(uint32_t cap);
 uint64_t identify_tiles(uint64_t B);
 cudaError_t noalloc_setup(int device);
@@ -162,24 +161,31 @@ __global__ void k_iota(uint32_t *a, uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = i;
 }
 
-/* the step's last counts, and its reports join the log */
-__global__ void k_step_tail(const uint32_t *qstart, uint32_t N, const uint32_t *reports, uint64_t log_cap,
-                            DevCounters *cnt) {
-    cnt->cross_checks = qstart[N];
-    cnt->total_checks = N + qstart[N];
-    const uint32_t total = *reports;
-    cnt->meetings = total;
-    cnt->log_step_begin = cnt->log_head;
-    cnt->log_head += total;
-    if (total > log_cap) atomicOr(&cnt->error_flags, GLINT_EF_LOG_OVERFLOW);
+/* the step's last counts; its reports join the log; the counters go to the
+ * host (page-locked memory, read there after the stream is synchronised) */
+__global__ void __launch_bounds__(64) k_step_tail(uint32_t N, const uint32_t *reports, uint64_t log_cap,
+                                                  DevCounters *cnt, DevCounters *host) {
+    if (threadIdx.x == 0) {
+        cnt->total_checks = N + cnt->cross_checks;
+        const uint32_t total = *reports;
+        cnt->meetings = total;
+        cnt->log_step_begin = cnt->log_head;
+        cnt->log_head += total;
+        if (total > log_cap) cnt->error_flags |= GLINT_EF_LOG_OVERFLOW;
+    }
+    __syncthreads();
+    static_assert(sizeof(DevCounters) % 4 == 0, "counter words");
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(cnt);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(host);
+    for (uint32_t i = threadIdx.x; i < sizeof(DevCounters) / 4; i += blockDim.x) dst[i] = src[i];
 }
 
 void free_all(glint_ctx *c) {
-    void *ptrs[] = {c->d_pts, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj_gid, c->d_obj_lv, c->d_obj_leaf, c->d_order, c->d_grid_count,
-                    c->d_grid_start, c->d_grid_cursor, c->d_sorted, c->d_rank_of, c->d_sxy, c->d_sm, c->d_leaf_work,
+    void *ptrs[] = {c->d_pts, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj_gid, c->d_obj_lv, c->d_obj_leaf, c->d_obj_pos, c->d_grid_count,
+                    c->d_grid_start, c->d_sorted, c->d_rank_of, c->d_sxy, c->d_sm, c->d_leaf_work,
                     c->d_nodes, c->d_low, c->d_sstack, c->d_gstack, c->d_split, c->d_evscan, c->d_cand, c->d_newgid,
-                    c->d_events, c->d_evpos, c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
-                    c->d_qstart, c->d_qlist, c->d_qtmp, c->d_tcount, c->d_tstart, c->d_tcursor, c->d_tlist, c->d_tab,
+                    c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
+                    c->d_qstart, c->d_qlist, c->d_qslot, c->d_tcount, c->d_tstart, c->d_tlist, c->d_tab,
                     c->d_stamp, c->d_newline, c->d_new, c->d_rextra, c->d_tile_cnt, c->d_tile_off, c->d_log, c->d_cnt, c->d_coef,
                     c->d_scan_tmp, c->d_scan_tmp_side, c->d_qbits, c->d_qpids, c->d_qout, c->d_qn};
     for (void *p : ptrs)
@@ -220,7 +226,11 @@ Frame make_frame(const glint_box &mbr, const glint_schema_node &root, double r, 
     f.ox = std::isfinite(lx) ? lx : 0.0;
     f.oy = std::isfinite(ly) ? ly : 0.0;
     f.S = std::ldexp(1.0, k);
-    f.kdeg = (float)(kPIh / 180.0);
+    f.k = k;
+    f.X0 = fx_round(f.ox, k, nullptr);
+    f.Y0 = fx_round(f.oy, k, nullptr);
+    f.ksh = std::max(0, k - 36);
+    f.kang = (float)std::ldexp(kPIh / 180.0, f.ksh - k);
     f.kc = (float)(40076000.0 / (360.0 * f.S));
     f.cy = (float)(1.0 / (dpm_lat * f.S));
     f.r2 = (float)(r * r);
@@ -407,10 +417,9 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     ALLOC(c->d_obj_gid, N);
     ALLOC(c->d_obj_lv, N);
     ALLOC(c->d_obj_leaf, N);
-    ALLOC(c->d_order, N);
+    ALLOC(c->d_obj_pos, N);
     ALLOC(c->d_grid_count, (size_t)G + 1);
     ALLOC(c->d_grid_start, (size_t)G + 1);
-    ALLOC(c->d_grid_cursor, G);
     ALLOC(c->d_sorted, N);
     ALLOC(c->d_rank_of, N);
     ALLOC(c->d_sxy, N);
@@ -426,18 +435,15 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     ALLOC(c->d_evscan, S);
     ALLOC(c->d_cand, S);
     ALLOC(c->d_newgid, S);
-    ALLOC(c->d_events, (size_t)S + 1);
-    ALLOC(c->d_evpos, (size_t)S + 1);
     ALLOC(c->d_evlist, S);
     ALLOC(c->d_evdata, 2 * (size_t)S);
     ALLOC(c->d_evlevel, S);
     ALLOC(c->d_qcount, (size_t)N + 1);
     ALLOC(c->d_qstart, (size_t)N + 1);
     ALLOC(c->d_qlist, c->check_cap);
-    ALLOC(c->d_qtmp, (size_t)N * 8);
+    ALLOC(c->d_qslot, c->check_cap);
     ALLOC(c->d_tcount, (size_t)G + 1);
     ALLOC(c->d_tstart, (size_t)G + 1);
-    ALLOC(c->d_tcursor, G);
     ALLOC(c->d_tlist, c->check_cap);
     ALLOC(c->d_tab, c->B);
     ALLOC(c->d_stamp, stamp_bytes(c->B));
@@ -544,6 +550,22 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     std::memset(&hc, 0, sizeof(hc));
     hc.ssi = ssi;
     hc.gsi = gsi;
+    /* ids from here on sit at their own places of the free stacks and in no
+     * node, so they are first used when the stack index reaches them */
+    uint32_t su = std::max(1u, ssi), gu = std::max(1u, gsi);
+    for (uint32_t i = 0; i < S; ++i) {
+        if (sch[i].type == 0) continue;
+        su = std::max(su, i + 1);
+        if (sch[i].type == 1)
+            for (uint32_t ch : sch[i].children) su = std::max(su, ch < S ? ch + 1 : S);
+        gu = std::max(gu, sch[i].grid_id < G ? sch[i].grid_id + 1 : G);
+    }
+    for (uint32_t i = ssi; i < S; ++i)
+        if (sstack[i] != i) su = std::max({su, i + 1, sstack[i] < S ? sstack[i] + 1 : S});
+    for (uint32_t i = gsi; i < G; ++i)
+        if (gstack[i] != i) gu = std::max({gu, i + 1, gstack[i] < G ? gstack[i] + 1 : G});
+    hc.slots_used = su;
+    hc.grids_used = gu;
     cudaMemcpy(c->d_cnt, &hc, sizeof(hc), cudaMemcpyHostToDevice);
     SinCoef coef;
     init_sin_coef(&coef);
@@ -553,15 +575,16 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     cudaMemsetAsync(c->d_scan_tmp_side, 0, c->scan_tmp_bytes, c->stream);
     cudaMemsetAsync(c->d_stamp, 0, stamp_bytes(c->B), c->stream);
     cudaMemsetAsync(c->d_newline, 0, sizeof(uint32_t) * newline_words(c->B), c->stream);
+    cudaMemsetAsync(c->d_tcount, 0, sizeof(uint32_t) * ((size_t)G + 1), c->stream);
+    cudaMemsetAsync(c->d_split, 0, (size_t)S + 4, c->stream);
     cudaMemsetAsync(c->d_grid_count, 0, sizeof(uint32_t) * ((size_t)G + 1), c->stream);
-    k_iota<<<grid_for(N, 256, 152u * 8u), 256, 0, c->stream>>>(c->d_order, N);
+    k_iota<<<grid_for(N, 256, 152u * 8u), 256, 0, c->stream>>>(c->d_sorted, N);
     /* scratch address of glint_active_search_noalloc, once per device, with
      * this device current; a failure is reported by that call */
     noalloc_setup(c->device);
     partition_set_attributes();
     refine_set_attributes(c->cap);
     refine_prec_set_attributes(c->cap);
-    schema_set_attributes();
     flush_set_attributes();
     for (auto &ev : c->timers.ev) cudaEventCreate(&ev);
     for (auto &ev : c->flush_ev) cudaEventCreate(&ev);
@@ -611,8 +634,7 @@ namespace glint {
 void launch_step_front(glint_ctx *c, const double *points, bool host) {
     cudaStream_t s = c->stream;
     const bool tm = c->cfg.timing != 0 && !c->cfg.use_graph;
-    cudaMemsetAsync(c->d_cnt, 0, kStepCounterBytes, s);
-    cudaMemcpyAsync(&c->d_cnt->step_time, c->h_params, sizeof(StepParams), cudaMemcpyHostToDevice, s);
+    launch_step_begin(c);
     if (tm) cudaEventRecord(c->timers.ev[0], s);
     if (host) {
         cudaMemcpyAsync(c->d_pts, points, sizeof(double2) * c->N, cudaMemcpyHostToDevice, s);
@@ -624,7 +646,6 @@ void launch_step_front(glint_ctx *c, const double *points, bool host) {
     if (tm) cudaEventRecord(c->timers.ev[2], s);
     launch_filter(c);
     if (tm) cudaEventRecord(c->timers.ev[3], s);
-    launch_refine_items(c);
 }
 
 void launch_step_back(glint_ctx *c) {
@@ -648,9 +669,8 @@ void launch_step_back(glint_ctx *c) {
     launch_keys(c);
     if (tm) cudaEventRecord(c->timers.ev[6], s);
     if (schema) cudaStreamWaitEvent(s, c->join_ev, 0);
-    k_step_tail<<<1, 1, 0, s>>>(c->d_qstart, c->N, c->d_tile_off + c->n_tiles, c->log_cap, c->d_cnt);
+    k_step_tail<<<1, 64, 0, s>>>(c->N, c->d_tile_off + c->n_tiles, c->log_cap, c->d_cnt, c->h_cnt);
     if (tm) cudaEventRecord(c->timers.ev[7], s);
-    cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
 }
 
 static void launch_step(glint_ctx *c, const double *points, bool host) {
@@ -746,9 +766,9 @@ static void fill_stats(glint_ctx *c, glint_step_stats *st) {
     st->band_pairs = h.band_pairs;
     st->box_band = h.box_band;
     st->error_flags = h.error_flags;
-    /* kernels per step: partition 7, filter 5, refine 2 (work items, pairs),
-     * insert 1, identify 3 + keys 1, schema update 9, tail 1 */
-    st->launches = 7 + 5 + 2 + 1 + 4 + (c->cfg.dynamic_schema ? 9 : 0) + 1;
+    /* kernels per step: begin 1, partition 5, filter 3, refine 1, insert 1,
+     * identify 3 + keys 1, schema update 4, tail 1 */
+    st->launches = 1 + 5 + 3 + 1 + 1 + 4 + (c->cfg.dynamic_schema ? 4 : 0) + 1;
     st->meeting_log_size = h.log_head;
     st->kv_count = h.kv_count;
     st->flushed = c->last_flushed ? 1u : 0u;

@@ -288,10 +288,10 @@ __device__ inline bool box_le_exact(double lx, double ly, double hx, double hy, 
 }
 
 /* ---- fixed-point frame for screening tests ----------------------------------
- * Every coordinate is also held as a 64-bit integer X = rn((x - ox) * S) with
+ * Every coordinate is also held as a 64-bit integer X = rn(x S) - rn(ox S) with
  * S = 2^k (k chosen so the map spans about 2^40 units), so differences of
- * coordinates are exact integers, each within 1 + 2^-12 units of the exact
- * scaled difference.  A screening test converts the differences to FP32,
+ * coordinates are exact integers, each within 1 unit of the exact scaled
+ * difference.  A screening test converts the differences to FP32,
  * scales them to metres with cx = 1/(L S) (L = degree_per_meter_longitude of
  * the first point) and cy = 1/(dpm_lat S), and compares q = mx^2 + my^2 with
  * r^2.  With u = 2^-24: cx is within 9u of exact (the FP64 angle rounded
@@ -309,7 +309,10 @@ __device__ inline bool box_le_exact(double lx, double ly, double hx, double hy, 
 struct Frame {
     double ox, oy;       /* map low corner */
     double S;            /* units per degree, 2^k */
-    float kdeg;          /* fl32(kPI / 180) */
+    long long X0, Y0;    /* rn(ox S), rn(oy S) */
+    int k;
+    int ksh;             /* angles are taken in units of 2^(ksh - k) degrees: 90 degrees below 2^43 */
+    float kang;          /* radians per such unit */
     float kc;            /* fl32(40076000 / (360 S)): cx = sin(angle) * kc */
     float cy;            /* metres per unit along y: 1/(dpm_lat S) */
     float r2;            /* r^2 */
@@ -318,32 +321,76 @@ struct Frame {
     double a0, s0, c0;   /* an angle near the map's middle latitude, its sin and cos */
 };
 
-constexpr double kFxLimit = 1152921504606846976.0; /* 2^60 */
-
 /* a node box in fixed point: low x, low y, high x, high y */
 struct __align__(32) IBox {
     long long x, y, z, w;
 };
 
-__host__ __device__ inline long long fx_coord(double v, double o, double S, bool *clamped) {
-    double t = (v - o) * S; /* S is a power of two: the product is exact */
-    bool c = false;
-    if (!(t < kFxLimit)) { t = kFxLimit; c = true; }
-    if (t < -kFxLimit) { t = -kFxLimit; c = true; }
-    if (clamped) *clamped = *clamped || c;
-#if defined(__CUDA_ARCH__)
-    return __double2ll_rn(t);
-#else
-    return llrint(t);
-#endif
+/* rn(v 2^k) from the bits of v, with integer instructions: FP64 adds,
+ * multiplies, compares and conversions all issue on the narrow pipe of
+ * sm_103a (15 of them per object made the gather's 37 us per 1M objects).
+ * Exact to half a unit, so the difference of two coordinates is within one
+ * unit of the exact difference.  Beyond 2^60 units, infinite or NaN: clamped. */
+constexpr long long kFxLimit = 1ll << 60;
+__host__ __device__ inline long long fx_round(double v, int k, bool *clamped) {
+    const uint64_t b = dbits(v);
+    const int e = (int)((b >> 52) & 0x7ff);
+    const uint64_t m = (b & 0xfffffffffffffull) | 0x10000000000000ull; /* 1.m 2^52 */
+    const int sh = 1075 - e - k; /* v 2^k = m 2^-sh */
+    long long r;
+    if (e == 0 || sh > 54) r = 0;          /* below half a unit (or zero) */
+    else if (sh < -7) r = kFxLimit;        /* 2^53 2^8 and more, infinities, NaN */
+    else if (sh <= 0) r = (long long)(m << -sh);
+    else r = (long long)((m + (1ull << (sh - 1))) >> sh);
+    if (r >= kFxLimit) {
+        r = kFxLimit;
+        if (clamped) *clamped = true;
+    }
+    return (b >> 63) ? -r : r;
+}
+__host__ __device__ inline long long fx_coord(double v, int k, long long origin, bool *clamped) {
+    return fx_round(v, k, clamped) - origin;
 }
 
-/* metres per unit along x at latitude lat, FP32 (within 9u of exact) */
+/* integer -> FP32 on the FP32 pipe (I2F issues on the narrow FP64 pipe of
+ * sm_103a): for |v| < 2^22 the bits 0x4B400000 + v are the float
+ * 1.5*2^23 + v exactly, so one subtraction recovers v */
+__device__ inline float small_to_f(int v) { return __fsub_rn(__int_as_float(0x4B400000 + v), 12582912.0f); }
+
+/* correctly rounded FP32 value of d for |d| < 2^44; NaN beyond (2^13
+ * map widths apart), which sends the test to the exact path */
+__device__ inline float fx_to_f(long long d) {
+    /* d = hi 2^22 + lo with lo in [0, 2^22): one rounding in the fma; for
+     * |d| < 2^22, hi is 0 or -1 and the fma is exact */
+    const long long w = 1ll << 44;
+    const int hi = (int)(d >> 22), lo = (int)(d & 0x3FFFFF);
+    const float f = __fmaf_rn(small_to_f(hi), 4194304.0f, small_to_f(lo));
+    return (d > -w && d < w) ? f : __int_as_float(0x7fc00000);
+}
+
+/* FP32 value of d, correctly rounded, with integer instructions where the
+ * result is a normal number and not the largest */
+__device__ inline float f_of_d(double d) {
+    const uint64_t b = dbits(d), m = b & 0x7fffffffffffffffull;
+    const uint64_t r = m - (896ull << 52); /* exponent rebiased: 1023 - 127 */
+    if (m >= (897ull << 52) && r < (254ull << 52)) {
+        const uint32_t keep = (uint32_t)(r >> 29), low = (uint32_t)r & 0x1fffffffu;
+        const uint32_t f = keep + (low + (keep & 1u) > 0x10000000u ? 1u : 0u);
+        return __uint_as_float(f | ((uint32_t)(b >> 32) & 0x80000000u));
+    }
+    return (float)d;
+}
+
+/* metres per unit along x at latitude lat, FP32 (within 9u of exact): the
+ * angle from the pole as an integer, converted with one rounding */
 __device__ inline float c_of_lat(double lat, const Frame &f) {
-    double a = fabs(lat);
-    if (a == 90.0) a = 89.0;
-    const float t = (float)__dsub_rn(90.0, a);
-    return sinf(t * f.kdeg) * f.kc;
+    bool clamped = false;
+    long long a = fx_round(lat, f.k, &clamped);
+    a = a < 0 ? -a : a;
+    const long long ninety = 90ll << f.k;
+    if (a == ninety && fabs(lat) == 90.0) a = 89ll << f.k;
+    const float t = fx_to_f((ninety - a) >> f.ksh);
+    return clamped ? __int_as_float(0x7fc00000) : sinf(t * f.kang) * f.kc;
 }
 
 /* metres per degree of longitude at latitude lat in FP64, 1 / L to a few
@@ -380,22 +427,6 @@ __device__ inline Screen make_screen(float cx, const Frame &f) {
     return s;
 }
 
-/* integer -> FP32 on the FP32 pipe (I2F issues on the narrow FP64 pipe of
- * sm_103a): for |v| < 2^22 the bits 0x4B400000 + v are the float
- * 1.5*2^23 + v exactly, so one subtraction recovers v */
-__device__ inline float small_to_f(int v) { return __fsub_rn(__int_as_float(0x4B400000 + v), 12582912.0f); }
-
-/* correctly rounded FP32 value of d for |d| < 2^44; NaN beyond (2^13
- * map widths apart), which sends the test to the exact path */
-__device__ inline float fx_to_f(long long d) {
-    /* d = hi 2^22 + lo with lo in [0, 2^22): one rounding in the fma; for
-     * |d| < 2^22, hi is 0 or -1 and the fma is exact */
-    const long long w = 1ll << 44;
-    const int hi = (int)(d >> 22), lo = (int)(d & 0x3FFFFF);
-    const float f = __fmaf_rn(small_to_f(hi), 4194304.0f, small_to_f(lo));
-    return (d > -w && d < w) ? f : __int_as_float(0x7fc00000);
-}
-
 /* 1 within reach, 0 beyond, -1 inside the guard band (or a NaN scale);
  * dx, dy in units */
 __device__ inline int fx_screen(long long dx, long long dy, const Screen &s, float cy) {
@@ -408,21 +439,17 @@ __device__ inline int fx_screen(long long dx, long long dy, const Screen &s, flo
 
 __host__ __device__ inline IBox fx_box(double lx, double ly, double hx, double hy, const Frame &f) {
     IBox b;
-    b.x = fx_coord(lx, f.ox, f.S, nullptr);
-    b.y = fx_coord(ly, f.oy, f.S, nullptr);
-    b.z = fx_coord(hx, f.ox, f.S, nullptr);
-    b.w = fx_coord(hy, f.oy, f.S, nullptr);
+    b.x = fx_coord(lx, f.k, f.X0, nullptr);
+    b.y = fx_coord(ly, f.k, f.Y0, nullptr);
+    b.z = fx_coord(hx, f.k, f.X0, nullptr);
+    b.w = fx_coord(hy, f.k, f.Y0, nullptr);
     return b;
 }
 
 /* box distance screening: the gap from the point to the box along each axis */
 __device__ inline int fx_box_screen(const IBox &b, long long px, long long py, const Screen &s, float cy) {
-    /* the gaps are taken after the conversion: rounding is monotonic, so the
-     * FP32 maximum is the rounded integer maximum (and needs no 64-bit max) */
-    const float x1 = fx_to_f(b.x - px), x2 = fx_to_f(px - b.z);
-    const float y1 = fx_to_f(b.y - py), y2 = fx_to_f(py - b.w);
-    if (!(x1 == x1 && x2 == x2 && y1 == y1 && y2 == y2)) return -1; /* beyond fx_to_f's range */
-    const float gx = fmaxf(fmaxf(x1, x2), 0.0f), gy = fmaxf(fmaxf(y1, y2), 0.0f);
+    const long long x1 = b.x - px, x2 = px - b.z, y1 = b.y - py, y2 = py - b.w;
+    const float gx = fx_to_f(x1 > 0 ? x1 : (x2 > 0 ? x2 : 0)), gy = fx_to_f(y1 > 0 ? y1 : (y2 > 0 ? y2 : 0));
     const float mx = gx * s.cx, my = gy * cy;
     const float q = mx * mx + my * my;
     if (q < s.lo) return 1;

@@ -65,7 +65,11 @@ struct DevCounters {
     unsigned int sid_count;                /* objects with at least one pending key */
     unsigned int oversize_oid_count;
     unsigned int keys_outside;             /* meetings outside the map box (not keyed) */
-    unsigned int pad2[3];
+    /* schema slots and grids ever in use: ids from there on are free and never
+     * were anything else (0: not known, the whole arrays are in use) */
+    unsigned int slots_used;
+    unsigned int grids_used;
+    unsigned int pad2;
     /* this step's parameters, copied in at the start of the step so that a
      * captured step graph reads them from here */
     unsigned int step_time;                /* cur_time */
@@ -171,11 +175,10 @@ struct glint_ctx {
     /* objects */
     double2 *d_pts = nullptr;
     uint32_t *d_obj_gid = nullptr, *d_obj_lv = nullptr, *d_obj_leaf = nullptr;
-    uint32_t *d_order = nullptr;           /* processing order of the descent */
     uint32_t *d_grid_count = nullptr;      /* [G+1] */
     uint32_t *d_grid_start = nullptr;      /* [G+1] */
-    uint32_t *d_grid_cursor = nullptr;     /* [G] */
-    uint32_t *d_sorted = nullptr;          /* [N] */
+    uint32_t *d_obj_pos = nullptr;         /* [N] each object's place in its leaf's segment */
+    uint32_t *d_sorted = nullptr;          /* [N] leaf-major order; the next descent's processing order */
     uint32_t *d_rank_of = nullptr;         /* [N] sorted position of each object */
     double2 *d_sxy = nullptr;
     double *d_sm = nullptr;                /* [N] sorted metres per degree of longitude (plain form only) */
@@ -193,20 +196,18 @@ struct glint_ctx {
     uint32_t *d_sstack = nullptr;
     uint32_t *d_gstack = nullptr;
     uint8_t *d_split = nullptr;            /* [S] per-slot event flags */
-    uint32_t *d_evscan = nullptr;          /* [S] candidate leaf-children sums */
+    uint32_t *d_evscan = nullptr;          /* [S] candidate leaf-children sums, then each stack cell's last event */
     uint32_t *d_cand = nullptr;            /* [S] merge candidates */
     uint32_t *d_newgid = nullptr;          /* [S] grid id a merged node takes */
-    uint32_t *d_events = nullptr;          /* [S+1] per-slot event indicator */
-    uint32_t *d_evpos = nullptr;           /* [S+1] its exclusive scan */
     uint32_t *d_evlist = nullptr;          /* [S] event slots in slot order */
     uint4 *d_evdata = nullptr;             /* [2S] per-event replay data */
-    int32_t *d_evlevel = nullptr;          /* [S] stack level before each event */
+    int32_t *d_evlevel = nullptr;          /* [S] the stack cell each event crosses */
     uint32_t *d_big = nullptr;             /* [G] leaves sorted by a whole block */
 
     /* filter */
     uint32_t *d_qcount = nullptr, *d_qstart = nullptr, *d_qlist = nullptr;
-    uint32_t *d_qtmp = nullptr;            /* [N*8] first targets of each border object */
-    uint32_t *d_tcount = nullptr, *d_tstart = nullptr, *d_tcursor = nullptr;
+    uint32_t *d_qslot = nullptr;           /* each check's place among its target leaf's */
+    uint32_t *d_tcount = nullptr, *d_tstart = nullptr;
     uint2 *d_tlist = nullptr;
 
     /* table */
@@ -292,10 +293,9 @@ cudaError_t scan_u32(const uint32_t *in, uint32_t *out, size_t n, void *tmp, cud
 void init_sin_coef(SinCoef *host);
 
 /* ---- stages ---- */
+cudaError_t launch_step_begin(glint_ctx *c);
 cudaError_t launch_partition(glint_ctx *c, uint32_t cur_time);
 cudaError_t launch_filter(glint_ctx *c);
-cudaError_t launch_refine(glint_ctx *c, uint32_t cur_time);
-cudaError_t launch_refine_items(glint_ctx *c);
 cudaError_t launch_refine_pairs(glint_ctx *c);
 struct RefineArgs;
 RefineArgs refine_args(glint_ctx *c);

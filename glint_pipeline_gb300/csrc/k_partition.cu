@@ -12,11 +12,12 @@
  * members are its smallest ids.
  *
  * Here the leaf buffers are replaced by a stable sort of objects by
- * (grid id, object id): a count per grid, an exclusive scan, a scatter and a
- * per-leaf sort of each segment.  The first min(count, capacity) entries of a
+ * (grid id, object id): a count per grid, which gives every object a place in
+ * its grid's segment, an exclusive scan, a scatter and a per-leaf sort of each
+ * segment.  The first min(count, capacity) entries of a
  * segment are exactly the reference's stored members, in the same order.
  */
-#include "glint_internal.cuh"
+#include "scan.cuh"
 
 namespace glint {
 
@@ -26,8 +27,8 @@ __global__ void __launch_bounds__(256) k_descend(const double2 *__restrict__ pts
                                                  uint32_t N, const DNode *__restrict__ nodes, uint32_t S, uint32_t G,
                                                  double xb, double yb,
                                                  uint32_t *__restrict__ obj_gid, uint32_t *__restrict__ obj_lv,
-                                                 uint32_t *__restrict__ obj_leaf, uint32_t *__restrict__ grid_count,
-                                                 DevCounters *cnt) {
+                                                 uint32_t *__restrict__ obj_leaf, uint32_t *__restrict__ obj_pos,
+                                                 uint32_t *__restrict__ grid_count, DevCounters *cnt) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         const uint32_t pid = order[i];
         const double2 p = pts[pid];
@@ -62,47 +63,90 @@ __global__ void __launch_bounds__(256) k_descend(const double2 *__restrict__ pts
         obj_lv[pid] = lv;
         obj_leaf[pid] = cur;
         /* objects come in the previous step's leaf order, so the lanes of a
-         * warp mostly share a leaf: one atomic per leaf and warp */
+         * warp mostly share a leaf: one atomic per leaf and warp, which also
+         * gives each object its place in the leaf's segment */
         const unsigned peers = __match_any_sync(__activemask(), gid);
-        if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&grid_count[gid], (uint32_t)__popc(peers));
+        const int leader = __ffs(peers) - 1;
+        uint32_t at = 0;
+        if ((threadIdx.x & 31) == leader) at = atomicAdd(&grid_count[gid], (uint32_t)__popc(peers));
+        at = __shfl_sync(peers, at, leader);
+        obj_pos[pid] = at + __popc(peers & ((1u << (threadIdx.x & 31)) - 1u));
     }
 }
 
-__global__ void __launch_bounds__(256) k_scatter(const uint32_t *__restrict__ obj_gid, uint32_t N,
+__global__ void __launch_bounds__(256) k_scatter(const uint32_t *__restrict__ obj_gid,
+                                                 const uint32_t *__restrict__ obj_pos, uint32_t N,
                                                  const uint32_t *__restrict__ grid_start,
-                                                 uint32_t *__restrict__ grid_cursor, uint32_t *__restrict__ sorted) {
-    for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < N; pid += gridDim.x * blockDim.x) {
-        uint32_t g = obj_gid[pid];
-        uint32_t pos = grid_start[g] + atomicAdd(&grid_cursor[g], 1u);
-        sorted[pos] = pid;
-    }
+                                                 uint32_t *__restrict__ sorted) {
+    for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < N; pid += gridDim.x * blockDim.x)
+        sorted[grid_start[obj_gid[pid]] + obj_pos[pid]] = pid;
 }
 
-/* leaves that hold objects, and the objects their buffers drop */
-__global__ void __launch_bounds__(256) k_leaf_work(const uint32_t *__restrict__ grid_count, uint32_t G, uint32_t cap,
-                                                   uint32_t *__restrict__ work, uint32_t *__restrict__ big,
-                                                   uint32_t warp_limit, DevCounters *cnt) {
-    const int lane = threadIdx.x & 31;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < G; base += gridDim.x * blockDim.x) {
-        uint32_t g = base + threadIdx.x;
-        uint32_t c = g < G ? grid_count[g] : 0u;
-        bool has = c > 0;
-        unsigned m = __ballot_sync(0xffffffffu, has);
-        uint32_t off = 0;
-        if (lane == 0 && m) off = atomicAdd(&cnt->n_leaf_work, (unsigned)__popc(m));
-        off = __shfl_sync(0xffffffffu, off, 0);
-        if (has) work[off + __popc(m & ((1u << lane) - 1u))] = g;
-        uint32_t drop = c > cap ? c - cap : 0u;
-        for (int o = 16; o > 0; o >>= 1) drop += __shfl_down_sync(0xffffffffu, drop, o);
+/* the scan of the leaf counts: segment starts, and on the way the leaves that
+ * hold objects (work, in any order), those whose segment is too long for one
+ * warp (big) and the objects that their buffers drop */
+struct LeafScan {
+    ScanStore start;
+    uint32_t *work, *big;
+    uint32_t cap, warp_limit;
+    DevCounters *cnt;
+    __device__ void total(uint32_t n, uint32_t sum) const { start.total(n, sum); }
+    __device__ void store(uint32_t base, uint32_t n, const uint32_t (&v)[kScanItems],
+                          const uint32_t (&o)[kScanItems]) const {
+        start.store(base, n, v, o);
+        const int lane = threadIdx.x & 31;
+        uint32_t have = 0, drop = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            have += v[k] ? 1u : 0u;
+            drop += v[k] > cap ? v[k] - cap : 0u;
+        }
+        uint32_t incl = have;
+        for (int s = 1; s < 32; s <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, s);
+            if (lane >= s) incl += y;
+        }
+        uint32_t at = 0;
+        if (lane == 31 && incl) at = atomicAdd(&cnt->n_leaf_work, incl);
+        at = __shfl_sync(0xffffffffu, at, 31) + incl - have;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (!v[k]) continue;
+            work[at++] = base + k;
+            if (v[k] > warp_limit) big[atomicAdd(&cnt->n_big, 1u)] = base + k;
+        }
+        drop = __reduce_add_sync(0xffffffffu, drop);
         if (lane == 0 && drop) atomicAdd(&cnt->dropped, drop);
-        /* segments too long for one warp go to the block sorter */
-        bool isbig = c > warp_limit;
-        unsigned mb = __ballot_sync(0xffffffffu, isbig);
-        uint32_t boff = 0;
-        if (lane == 0 && mb) boff = atomicAdd(&cnt->n_big, (unsigned)__popc(mb));
-        boff = __shfl_sync(0xffffffffu, boff, 0);
-        if (isbig) big[boff + __popc(mb & ((1u << lane) - 1u))] = g;
     }
+};
+
+/* per object, in leaf-major order: the coordinates, their fixed-point and
+ * FP32 forms and the screening scale cx; metres per degree of longitude in
+ * FP64 for the plain form; each object's sorted position */
+struct GatherOut {
+    double2 *sxy;
+    longlong2 *sipos;
+    float2 *sfpos;
+    float *sc;
+    double *sm;        /* null: not needed */
+    float2 *fpos;      /* by object id */
+    uint32_t *rank_of;
+};
+
+__device__ inline void gather_one(const GatherOut &o, const Frame &f, const double2 *__restrict__ pts, uint32_t i,
+                                  uint32_t pid) {
+    const double2 p = pts[pid];
+    o.sxy[i] = p;
+    bool clamped = false;
+    const long long X = fx_coord(p.x, f.k, f.X0, &clamped);
+    const long long Y = fx_coord(p.y, f.k, f.Y0, &clamped);
+    o.sipos[i] = make_longlong2(X, Y);
+    o.sc[i] = clamped ? __int_as_float(0x7fc00000) : c_of_lat(p.y, f);
+    const float2 fp = make_float2(f_of_d(p.x), f_of_d(p.y));
+    o.sfpos[i] = fp;
+    o.fpos[pid] = fp;
+    if (o.sm) o.sm[i] = metres_per_degree(p.y, f);
+    o.rank_of[pid] = i;
 }
 
 /* bitonic sort of n (<= 1024) keys in a warp's shared buffer, padded with ~0u */
@@ -130,36 +174,49 @@ __device__ inline void warp_bitonic(uint32_t *buf, uint32_t n) {
 constexpr int kSortWarps = 8;
 constexpr uint32_t kWarpSortMax = 1024;
 
-/* one warp per leaf segment of up to kWarpSortMax objects */
+/* One warp per leaf segment of up to kWarpSortMax objects: its ids in order,
+ * and each object's gathered arrays while the ids are still at hand.  (As a
+ * sort and a gather of their own: 31 + 37 us at 1M objects; together and
+ * without FP64 instructions 49 us.) */
 __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t *__restrict__ work,
                                                                   const uint32_t *__restrict__ grid_start,
                                                                   const uint32_t *__restrict__ grid_count,
-                                                                  uint32_t *__restrict__ sorted, const DevCounters *cnt) {
+                                                                  uint32_t *__restrict__ sorted,
+                                                                  const double2 *__restrict__ pts, GatherOut o,
+                                                                  Frame f, const DevCounters *cnt) {
     __shared__ uint32_t buf[kSortWarps][kWarpSortMax];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nwork = cnt->n_leaf_work;
     for (uint32_t li = blockIdx.x * kSortWarps + w; li < nwork; li += gridDim.x * kSortWarps) {
         const uint32_t g = work[li];
         const uint32_t n = grid_count[g];
-        if (n <= 1 || n > kWarpSortMax) continue;
-        uint32_t *seg = sorted + grid_start[g];
+        if (n > kWarpSortMax) continue;
+        const uint32_t s0 = grid_start[g];
+        uint32_t *seg = sorted + s0;
         if (n <= 32) {
             uint32_t v = lane < (int)n ? seg[lane] : 0xffffffffu;
             /* register bitonic sort across the warp */
             for (int k = 2; k <= 32; k <<= 1) {
                 for (int j = k >> 1; j > 0; j >>= 1) {
-                    uint32_t o = __shfl_xor_sync(0xffffffffu, v, j);
+                    uint32_t x = __shfl_xor_sync(0xffffffffu, v, j);
                     bool up = (lane & k) == 0;
                     bool lower = (lane & j) == 0;
-                    v = (lower == up) ? min(v, o) : max(v, o);
+                    v = (lower == up) ? min(v, x) : max(v, x);
                 }
+                if (k >= (int)n) break; /* the padding sorts last: done */
             }
-            if (lane < (int)n) seg[lane] = v;
+            if (lane < (int)n) {
+                seg[lane] = v;
+                gather_one(o, f, pts, s0 + lane, v);
+            }
         } else {
             for (uint32_t i = lane; i < n; i += 32) buf[w][i] = seg[i];
             __syncwarp();
             warp_bitonic(buf[w], n);
-            for (uint32_t i = lane; i < n; i += 32) seg[i] = buf[w][i];
+            for (uint32_t i = lane; i < n; i += 32) {
+                seg[i] = buf[w][i];
+                gather_one(o, f, pts, s0 + i, buf[w][i]);
+            }
         }
         __syncwarp();
     }
@@ -171,14 +228,20 @@ constexpr uint32_t kBlockSortMax = 16384;
 __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restrict__ big,
                                                         const uint32_t *__restrict__ grid_start,
                                                         const uint32_t *__restrict__ grid_count,
-                                                        uint32_t *__restrict__ sorted, DevCounters *cnt) {
+                                                        uint32_t *__restrict__ sorted,
+                                                        const double2 *__restrict__ pts, GatherOut o, Frame f,
+                                                        DevCounters *cnt) {
     extern __shared__ uint32_t sbuf[];
     const uint32_t nbig = cnt->n_big;
     for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
         const uint32_t g = big[bi];
         const uint32_t n = grid_count[g];
         if (n > kBlockSortMax) {
+            /* reported; the arrays are filled all the same, so that what
+             * follows in this step reads objects */
             if (threadIdx.x == 0) atomicOr(&cnt->error_flags, GLINT_EF_SEGMENT_TOO_LARGE);
+            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+                gather_one(o, f, pts, grid_start[g] + i, sorted[grid_start[g] + i]);
             continue;
         }
         uint32_t P = 1024;
@@ -199,61 +262,53 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
                 __syncthreads();
             }
         }
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) seg[i] = sbuf[i];
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            seg[i] = sbuf[i];
+            gather_one(o, f, pts, grid_start[g] + i, sbuf[i]);
+        }
         __syncthreads();
     }
 }
 
-/* per object, in leaf-major order: the coordinates, their fixed-point and
- * FP32 forms and the screening scale cx; metres per degree of longitude in
- * FP64 for the plain form;
- * each object's sorted position */
-struct GatherOut {
-    double2 *sxy;
-    longlong2 *sipos;
-    float2 *sfpos;
-    float *sc;
-    double *sm;        /* null: not needed */
-    float2 *fpos;      /* by object id */
-    uint32_t *rank_of;
-};
-
-__global__ void __launch_bounds__(256) k_gather(const uint32_t *__restrict__ sorted, uint32_t N,
-                                                const double2 *__restrict__ pts, GatherOut o, Frame f) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        const uint32_t pid = sorted[i];
-        const double2 p = pts[pid];
-        o.sxy[i] = p;
-        bool clamped = false;
-        const long long X = fx_coord(p.x, f.ox, f.S, &clamped);
-        const long long Y = fx_coord(p.y, f.oy, f.S, &clamped);
-        o.sipos[i] = make_longlong2(X, Y);
-        o.sc[i] = clamped ? __int_as_float(0x7fc00000) : c_of_lat(p.y, f);
-        const float2 fp = make_float2((float)p.x, (float)p.y);
-        o.sfpos[i] = fp;
-        o.fpos[pid] = fp;
-        if (o.sm) o.sm[i] = metres_per_degree(p.y, f);
-        o.rank_of[pid] = i;
+/* the start of a step: its counters cleared, its parameters (host memory)
+ * taken in, and the counts of the leaves in use cleared */
+__global__ void __launch_bounds__(256) k_step_begin(const StepParams *__restrict__ params,
+                                                    uint32_t *__restrict__ grid_count, uint32_t *__restrict__ tcount,
+                                                    uint32_t G, DevCounters *cnt) {
+    const uint32_t n = cnt->grids_used && cnt->grids_used < G ? cnt->grids_used : G;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        grid_count[i] = 0;
+        tcount[i] = 0;
     }
+    if (blockIdx.x == 0) {
+        uint32_t *w = reinterpret_cast<uint32_t *>(cnt);
+        for (uint32_t i = threadIdx.x; i < kStepCounterBytes / 4; i += blockDim.x) w[i] = 0;
+        if (threadIdx.x == 0) *reinterpret_cast<StepParams *>(&cnt->step_time) = *params;
+    }
+}
+
+cudaError_t launch_step_begin(glint_ctx *c) {
+    k_step_begin<<<grid_for(c->G, 256, 152u * 4u), 256, 0, c->stream>>>(c->h_params, c->d_grid_count, c->d_tcount, c->G,
+                                                                       c->d_cnt);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_partition(glint_ctx *c, uint32_t /*cur_time*/) {
     cudaStream_t s = c->stream;
     const uint32_t N = c->N, G = c->G;
-    cudaMemsetAsync(c->d_grid_count, 0, sizeof(uint32_t) * (G + 1), s);
-    cudaMemsetAsync(c->d_grid_cursor, 0, sizeof(uint32_t) * G, s);
-    k_descend<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_pts, c->d_order, N, c->d_nodes, c->S, G, c->x_buffer,
+    /* the last step's leaf-major order is the descent's processing order */
+    k_descend<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_pts, c->d_sorted, N, c->d_nodes, c->S, G, c->x_buffer,
                                                            c->y_buffer, c->d_obj_gid, c->d_obj_lv, c->d_obj_leaf,
-                                                           c->d_grid_count, c->d_cnt);
-    scan_u32(c->d_grid_count, c->d_grid_start, G, c->d_scan_tmp, s);
-    k_scatter<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_obj_gid, N, c->d_grid_start, c->d_grid_cursor,
-                                                           c->d_sorted);
-    k_leaf_work<<<grid_for(G, 256, 152u * 8u), 256, 0, s>>>(c->d_grid_count, G, c->cap, c->d_leaf_work, c->d_big,
-                                                             kWarpSortMax, c->d_cnt);
-    k_segsort_warp<<<152 * 8, 32 * kSortWarps, 0, s>>>(c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted,
-                                                       c->d_cnt);
-    k_segsort_block<<<152, 1024, kBlockSortMax * sizeof(uint32_t), s>>>(c->d_big, c->d_grid_start, c->d_grid_count,
-                                                                        c->d_sorted, c->d_cnt);
+                                                           c->d_obj_pos, c->d_grid_count, c->d_cnt);
+    LeafScan ls;
+    ls.start = ScanStore{c->d_grid_start, true};
+    ls.work = c->d_leaf_work;
+    ls.big = c->d_big;
+    ls.cap = c->cap;
+    ls.warp_limit = kWarpSortMax;
+    ls.cnt = c->d_cnt;
+    scan_launch(ScanWords{c->d_grid_count, true}, ls, G, &c->d_cnt->grids_used, c->d_scan_tmp, s);
+    k_scatter<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_obj_gid, c->d_obj_pos, N, c->d_grid_start, c->d_sorted);
     GatherOut o;
     o.sxy = c->d_sxy;
     o.sipos = c->d_sipos;
@@ -262,9 +317,10 @@ cudaError_t launch_partition(glint_ctx *c, uint32_t /*cur_time*/) {
     o.sm = c->cfg.precision_mode == 1 ? nullptr : c->d_sm;
     o.fpos = c->d_fpos;
     o.rank_of = c->d_rank_of;
-    k_gather<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_sorted, N, c->d_pts, o, c->frame);
-    /* this step's leaf-major order is the next descent's processing order */
-    cudaMemcpyAsync(c->d_order, c->d_sorted, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, s);
+    k_segsort_warp<<<grid_for(N, 16 * kSortWarps, 152u * 8u), 32 * kSortWarps, 0, s>>>(
+        c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_pts, o, c->frame, c->d_cnt);
+    k_segsort_block<<<152, 1024, kBlockSortMax * sizeof(uint32_t), s>>>(
+        c->d_big, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_pts, o, c->frame, c->d_cnt);
     return cudaGetLastError();
 }
 

@@ -66,23 +66,6 @@ int refine_warps(uint32_t cap) {
 }
 size_t refine_smem_bytes(uint32_t cap) { return (size_t)refine_warps(cap) * tile_warp_bytes(cap); }
 
-/* the chunks beyond the first of every leaf's cross-leaf checks */
-__global__ void __launch_bounds__(256) k_refine_extra(const uint32_t *__restrict__ work,
-                                                      const uint32_t *__restrict__ tstart, uint2 *__restrict__ extra,
-                                                      uint64_t cap, uint32_t per_item, DevCounters *cnt) {
-    const uint32_t nwork = cnt->n_leaf_work;
-    for (uint32_t li = blockIdx.x * blockDim.x + threadIdx.x; li < nwork; li += gridDim.x * blockDim.x) {
-        const uint32_t g = work[li];
-        const uint32_t cross = tstart[g + 1] - tstart[g];
-        const uint32_t chunks = (cross + per_item - 1) / per_item;
-        for (uint32_t ch = 1; ch < chunks; ++ch) {
-            const uint32_t idx = atomicAdd(&cnt->n_extra, 1u);
-            if (idx < cap) extra[idx] = make_uint2(g, ch);
-            else atomicOr(&cnt->error_flags, GLINT_EF_CHECKS_OVERFLOW);
-        }
-    }
-}
-
 RefineArgs refine_args(glint_ctx *c) {
     RefineArgs a;
     a.work = c->d_leaf_work;
@@ -102,6 +85,7 @@ RefineArgs refine_args(glint_ctx *c) {
     a.obj_gid = c->d_obj_gid;
     a.rank_of = c->d_rank_of;
     a.qstart = c->d_qstart;
+    a.qcount = c->d_qcount;
     a.qlist = c->d_qlist;
     a.extra = c->d_rextra;
     a.tab = c->d_tab;
@@ -123,24 +107,12 @@ RefineArgs refine_args(glint_ctx *c) {
 
 cudaError_t launch_refine_precision(glint_ctx *c, const RefineArgs &a);
 
-/* the refine stage's work items: each leaf's chunks beyond its first */
-cudaError_t launch_refine_items(glint_ctx *c) {
-    k_refine_extra<<<grid_for(c->G, 256), 256, 0, c->stream>>>(c->d_leaf_work, c->d_tstart, c->d_rextra,
-                                                               c->rextra_cap, c->chunk, c->d_cnt);
-    return cudaGetLastError();
-}
-
 /* the refine stage's pair tests over its work items */
 cudaError_t launch_refine_pairs(glint_ctx *c) {
     RefineArgs a = refine_args(c);
     if (c->cfg.precision_mode == 1) return launch_refine_precision(c, a);
     k_refine_fp64<<<152 * 8, 32 * refine_warps(c->cap), refine_smem_bytes(c->cap), c->stream>>>(a);
     return cudaGetLastError();
-}
-
-cudaError_t launch_refine(glint_ctx *c, uint32_t /*cur_time*/) {
-    cudaError_t e = launch_refine_items(c);
-    return e != cudaSuccess ? e : launch_refine_pairs(c);
 }
 
 /* The limit is a property of the kernel, shared by every context of the

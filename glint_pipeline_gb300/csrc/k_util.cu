@@ -8,146 +8,19 @@
 #include <cstring>
 
 #include "glint_internal.cuh"
+#include "scan.cuh"
 #include "tracegen.h"
 
 namespace glint {
-
-/* Exclusive scan in one launch: a tile per block, the tiles' running sums
- * passed on by look-back over status words.  The step runs five scans, most
- * of them over a few hundred thousand words at most, so launches bound them:
- * the reduce / scan / down form took three (36 us for the five at 20k
- * objects), this takes one (26 us) and reads the input once instead of twice.
- * The scratch starts zeroed.  Its status words carry the scan's number
- * (epoch), so they need no reset between scans: a word of an earlier scan
- * reads as not there yet.  Tiles are taken by ticket, so a tile waits only for
- * tiles that already run; a wait that outlasts kScanPolls adds up the input
- * before its tile itself. */
-constexpr int kScanThreads = 512;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;
-constexpr uint32_t kScanPolls = 1u << 20;
-
-struct ScanHead {
-    uint32_t epoch, ticket, done, pad;
-};
 
 size_t scan_tmp_bytes(size_t n) {
     const size_t tiles = (n + kScanTile - 1) / kScanTile + 1;
     return sizeof(ScanHead) + tiles * sizeof(unsigned long long);
 }
 
-__device__ inline unsigned long long scan_status(uint32_t epoch, uint32_t flag, uint32_t value) {
-    return ((unsigned long long)((epoch << 2) | flag) << 32) | value;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
-                                                       size_t n, ScanHead *head, uint32_t tiles, bool vec) {
-    constexpr uint32_t kSum = 1, kPrefix = 2;
-    __shared__ uint32_t ws[kScanThreads / 32];
-    __shared__ uint32_t s_tile, s_epoch, s_before;
-    volatile unsigned long long *status = reinterpret_cast<unsigned long long *>(head + 1);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        /* the epoch moves when the last tile is done: all tiles read the same */
-        s_epoch = (*(volatile uint32_t *)&head->epoch + 1) & 0x3fffffffu;
-        s_tile = atomicAdd(&head->ticket, 1u);
-    }
-    __syncthreads();
-    const uint32_t tile = s_tile, epoch = s_epoch;
-    const size_t base = (size_t)tile * kScanTile + (size_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    if (vec && base + kScanItems <= n) {
-#pragma unroll
-        for (int k = 0; k < kScanItems; k += 4) {
-            const uint4 x = *reinterpret_cast<const uint4 *>(in + base + k);
-            v[k] = x.x;
-            v[k + 1] = x.y;
-            v[k + 2] = x.z;
-            v[k + 3] = x.w;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) v[k] = base + k < n ? in[base + k] : 0u;
-    }
-    uint32_t mine = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) mine += v[k];
-    uint32_t incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) ws[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        uint32_t w = lane < kScanThreads / 32 ? ws[lane] : 0u;
-        const uint32_t own = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        const uint32_t sum = __shfl_sync(0xffffffffu, w, 31);
-        if (lane < kScanThreads / 32) ws[lane] = w - own;
-        if (lane == 0) status[tile] = scan_status(epoch, tile == 0 ? kPrefix : kSum, sum);
-        uint32_t before = 0;
-        for (long long at = (long long)tile - 1; at >= 0; at -= 32) {
-            /* 32 earlier tiles at once, the nearest on lane 0 */
-            const long long t = at - lane;
-            unsigned long long st = scan_status(epoch, kPrefix, 0);
-            uint32_t polls = 0;
-            if (t >= 0) {
-                do {
-                    st = status[t];
-                } while ((st >> 34) != epoch && ++polls < kScanPolls);
-            }
-            if (__any_sync(0xffffffffu, (st >> 34) != epoch)) {
-                before = 0;
-                for (size_t i = lane; i < (size_t)tile * kScanTile; i += 32) before += in[i];
-                before = __reduce_add_sync(0xffffffffu, before);
-                break;
-            }
-            const unsigned full = __ballot_sync(0xffffffffu, ((uint32_t)(st >> 32) & 3u) == kPrefix);
-            const int upto = full ? __ffs(full) - 1 : 31;
-            before += __reduce_add_sync(0xffffffffu, lane <= upto ? (uint32_t)st : 0u);
-            if (full) break;
-        }
-        if (lane == 0) {
-            if (tile) status[tile] = scan_status(epoch, kPrefix, before + sum);
-            s_before = before;
-            if (tile == tiles - 1) out[n] = before + sum;
-            if (atomicAdd(&head->done, 1u) == tiles - 1) {
-                head->ticket = 0;
-                head->done = 0;
-                head->epoch = epoch;
-            }
-        }
-    }
-    __syncthreads();
-    uint32_t p = s_before + ws[wid] + incl - mine;
-    uint32_t o[kScanItems];
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        o[k] = p;
-        p += v[k];
-    }
-    if (vec && base + kScanItems <= n) {
-#pragma unroll
-        for (int k = 0; k < kScanItems; k += 4)
-            *reinterpret_cast<uint4 *>(out + base + k) = make_uint4(o[k], o[k + 1], o[k + 2], o[k + 3]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k)
-            if (base + k < n) out[base + k] = o[k];
-    }
-}
-
 cudaError_t scan_u32(const uint32_t *in, uint32_t *out, size_t n, void *tmp, cudaStream_t s) {
-    const uint32_t tiles = (uint32_t)std::max<size_t>(1, (n + kScanTile - 1) / kScanTile);
     const bool vec = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
-    k_scan<<<tiles, kScanThreads, 0, s>>>(in, out, n, (ScanHead *)tmp, tiles, vec);
-    return cudaGetLastError();
+    return scan_launch(ScanWords{in, vec}, ScanStore{out, vec}, (uint32_t)n, nullptr, tmp, s);
 }
 
 /* ---- double-double Taylor coefficients (-1)^k/(2k+1)!, computed on the host

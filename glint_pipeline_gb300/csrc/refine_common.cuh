@@ -39,7 +39,7 @@ struct RefineArgs {
     const float *sc;           /* screening scale cx, leaf-major */
     const uint32_t *obj_gid;
     const uint32_t *rank_of;
-    const uint32_t *qstart;
+    const uint32_t *qstart, *qcount;
     const uint32_t *qlist;
     const uint32_t *obj_leaf;
     const IBox *ibox;
@@ -131,7 +131,9 @@ static __device__ __noinline__ bool pair_exact(const double2 *__restrict__ sxy, 
 
 /* does object obj have a cross-leaf check on grid gid */
 __device__ inline bool has_check(const RefineArgs &a, uint32_t obj, uint32_t gid) {
-    const uint32_t b = a.qstart[obj], e = a.qstart[obj + 1];
+    const uint32_t n = a.qcount[obj];
+    if (!n) return false;
+    const uint32_t b = a.qstart[obj], e = b + n;
     for (uint32_t k = b; k < e; ++k)
         if (a.qlist[k] == gid) return true;
     return false;

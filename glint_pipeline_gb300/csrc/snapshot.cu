@@ -178,7 +178,7 @@ extern "C" glint_status glint_snapshot_save(glint_ctx *c, const char *path) {
     if (e == cudaSuccess) e = w.dev(kSecSstack, c->d_sstack, sizeof(uint32_t) * c->S);
     if (e == cudaSuccess) e = w.dev(kSecGstack, c->d_gstack, sizeof(uint32_t) * c->G);
     if (e == cudaSuccess) e = w.dev(kSecGridCount, c->d_grid_count, sizeof(uint32_t) * ((size_t)c->G + 1));
-    if (e == cudaSuccess) e = w.dev(kSecOrder, c->d_order, sizeof(uint32_t) * N);
+    if (e == cudaSuccess) e = w.dev(kSecOrder, c->d_sorted, sizeof(uint32_t) * N);
     /* the table as runs, one per transfer chunk: a count, its slots, its
      * records; then a zero count */
     const uint64_t runs = (c->B + kTableChunk - 1) / kTableChunk;
@@ -309,7 +309,7 @@ extern "C" glint_status glint_snapshot_load(const char *path, int device, glint_
     if (e == cudaSuccess) e = r.dev(kSecSstack, c->d_sstack, sizeof(uint32_t) * c->S);
     if (e == cudaSuccess) e = r.dev(kSecGstack, c->d_gstack, sizeof(uint32_t) * c->G);
     if (e == cudaSuccess) e = r.dev(kSecGridCount, c->d_grid_count, sizeof(uint32_t) * ((size_t)c->G + 1));
-    if (e == cudaSuccess) e = r.dev(kSecOrder, c->d_order, sizeof(uint32_t) * N);
+    if (e == cudaSuccess) e = r.dev(kSecOrder, c->d_sorted, sizeof(uint32_t) * N);
     /* the table (empty after create); every occupied bucket is committed
      * between steps */
     uint64_t tbytes = 0;

@@ -312,22 +312,25 @@ class DeviceBench:
             keep.append(sd)
             qs[i].seeds = sd.ctypes.data_as(ctypes.c_void_p).value if sd.size else None
             qs[i].n_seeds, qs[i].hops, qs[i].t_start, qs[i].t_end = sd.size, int(hops), int(t0), int(t1)
-            rs[i].ids, rs[i].cap = None, 0
-        st = self.lib.glint_query_batch(self.h, qs, n, rs)
-        if st != 0:
-            raise GlintError(st, self.last_error())
-        bufs = []
-        for i in range(n):
-            b = np.zeros(max(int(rs[i].n), 1), np.uint32)
-            bufs.append(b)
-            rs[i].ids, rs[i].cap = b.ctypes.data_as(ctypes.c_void_p).value, b.size
-        st = self.lib.glint_query_batch(self.h, qs, n, rs)
-        if st != 0:
-            raise GlintError(st, self.last_error())
+        # A query reaches at most every object: with room for that the batch
+        # runs once.  (Untouched pages cost nothing; results are copied out.)
+        # Very large batches run once for the sizes and once for the ids.
+        once = n * self.n <= 1 << 28
+        bufs = [np.empty(self.n, np.uint32) if once else None for _ in range(n)]
+        for _ in range(1 if once else 2):
+            for i in range(n):
+                if bufs[i] is None and rs[i].n:
+                    bufs[i] = np.empty(int(rs[i].n), np.uint32)
+                rs[i].ids = bufs[i].ctypes.data if bufs[i] is not None else None
+                rs[i].cap = bufs[i].size if bufs[i] is not None else 0
+            st = self.lib.glint_query_batch(self.h, qs, n, rs)
+            if st != 0:
+                raise GlintError(st, self.last_error())
         out = []
         for i, (seeds, hops, t0, t1) in enumerate(queries):
+            ids = bufs[i][:int(rs[i].n)].copy() if bufs[i] is not None else np.zeros(0, np.uint32)
             ends = [0] + [int(rs[i].hop_end[h]) for h in range(int(hops))]
-            out.append([bufs[i][ends[h]:ends[h + 1]] for h in range(int(hops))])
+            out.append([ids[ends[h]:ends[h + 1]] for h in range(int(hops))])
         return out, sum(int(rs[i].keys_scanned) for i in range(n))
 
     # -- state ------------------------------------------------------------------
@@ -519,6 +522,7 @@ class Server:
         self.h = h
         self.slots = int(self.lib.glint_server_slots(h))
         self._keep = {}
+        self._buf = np.empty(1, np.uint32)
 
     def submit(self, seeds, hops: int, t_start: int = 0, t_end: int = 0) -> int:
         sd = np.ascontiguousarray(seeds, dtype=np.uint32)
@@ -541,9 +545,11 @@ class Server:
 
     def poll(self, ticket: int, cap: int = 1 << 20):
         """None while running; else (per-hop id arrays, keys scanned)"""
-        buf = np.zeros(max(cap, 1), np.uint32)
+        cap = max(cap, 1)
+        if self._buf.size < cap:
+            self._buf = np.empty(cap, np.uint32)
         r = _abi.GlintQueryResult()
-        r.ids, r.cap = buf.ctypes.data_as(ctypes.c_void_p).value, buf.size
+        r.ids, r.cap = self._buf.ctypes.data, cap
         done = ctypes.c_int()
         st = self.lib.glint_server_poll(self.h, int(ticket), ctypes.byref(r), ctypes.byref(done))
         if st != 0:
@@ -551,8 +557,9 @@ class Server:
         if not done.value:
             return None
         hops = self._keep.pop(int(ticket))
-        ends = [0] + [min(int(r.hop_end[h]), buf.size) for h in range(hops)]
-        return [buf[ends[h]:ends[h + 1]] for h in range(hops)], int(r.keys_scanned), int(r.n)
+        ids = self._buf[:min(int(r.n), cap)].copy()
+        ends = [0] + [min(int(r.hop_end[h]), cap) for h in range(hops)]
+        return [ids[ends[h]:ends[h + 1]] for h in range(hops)], int(r.keys_scanned), int(r.n)
 
     def close(self):
         if getattr(self, "h", None):

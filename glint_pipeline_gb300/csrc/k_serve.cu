@@ -9,16 +9,24 @@
  * rest (tracing/step_merge.cpp:67-115, 501-568); the targets of one hop are
  * the search list of the next (search_multi_pid, tracing/process.cpp:476-495).
  *
- * Device form: every query owns a slot, a visited bitmap over objects and
- * two object lists (frontier, next).  One launch advances every active slot
- * by one hop: its items are (slot, frontier object, kept block) triples,
+ * Device form: every query owns a slot: a bitmap of the objects it has reached
+ * and one of those the current hop reaches.  One launch advances every active
+ * slot by one hop: its items are (slot, frontier object, kept block) triples,
  * over the kept blocks whose time span can meet the slot's window; the
  * object's sid, first and count in the block locate its keys, which are
  * decoded as CTF::parse_key does (tracing/step_merge.cpp:335-345), and each
- * target inside the time window that the slot has not visited joins its next
- * list.  Between launches the host retires finished queries and admits
- * waiting ones into free slots (continuous batching); a slot's result only
- * depends on its own query.
+ * target inside the time window that the slot has not reached is marked.  A
+ * scan over the slots' marks then lists them, ascending, slot after slot: that
+ * list is the hop's result and the next hop's frontiers.  Between launches the
+ * host retires finished queries and admits waiting ones into free slots
+ * (continuous batching); a slot's result only depends on its own query.
+ *
+ * Bound: the hop's dependent reads, and around it launches and copies.  With
+ * each new object appended to its slot's list by an atomic, the lists then
+ * radix-sorted by (slot, id), 10 separate copies of control arrays and a
+ * synchronisation of its own for the seeds, a 2-hop query from 1000 seeds over
+ * 16 blocks of 3M objects took 97 operations on the stream (820 us); marks, the
+ * scan and one control copy take @OPS@.
  */
 #include <algorithm>
 #include <cstring>
@@ -26,7 +34,7 @@
 #include <unordered_map>
 #include <vector>
 
-#include "glint_internal.cuh"
+#include "scan.cuh"
 #include "store_codec.cuh"
 
 namespace glint {
@@ -34,21 +42,20 @@ namespace glint {
 constexpr uint32_t kMaxHops = 8;
 
 struct SlotParam {
-    uint32_t t_start, t_end, window, cur;  /* cur: which list holds the frontier */
+    uint32_t t_start, t_end, window, pad;
 };
 
 struct HopArgs {
     const StoreBlockDev *blocks;
-    uint32_t nblocks;
     uint32_t N;
-    uint64_t words;                        /* bitmap words per slot */
-    uint32_t *visited;                     /* [slot][words] */
-    uint32_t *lists;                       /* [slot][2][N] */
+    uint32_t words;                        /* bitmap words per slot, a multiple of a scan thread's items */
+    uint32_t *visited;                     /* [slot][words] reached so far */
+    uint32_t *fresh;                       /* [slot][words] reached by this hop */
     const SlotParam *param;                /* [slot] */
-    uint32_t *counts;                      /* [slot] next-list sizes */
     unsigned long long *scanned;           /* [slot] keys read */
     const uint32_t *active;                /* [A] slots taking part in this launch */
     const uint32_t *front;                 /* [A] their frontier sizes */
+    const uint32_t *const *front_ids;      /* [A] their frontiers */
     const unsigned long long *prefix;      /* [A + 1] their items (frontier x blocks), prefix sums */
     const uint32_t *rel;                   /* each active slot's blocks, concatenated */
     const uint32_t *rel_off;               /* [A + 1] where each active slot's blocks start in rel */
@@ -60,29 +67,14 @@ __device__ inline uint32_t visited_word(const HopArgs &a, uint32_t s, uint32_t t
     return target < a.N ? __ldcg(&a.visited[(size_t)s * a.words + (target >> 5)]) : ~0u;
 }
 
-/* marks target reached for slot s and appends it to the slot's next list
- * when it is new, given its reached-set word `seen` (visited_word); the
- * lanes that call together and append to the same slot take their places
- * with one atomic (a slot's counter is one address that every new object of
- * a large frontier would otherwise hit) */
-__device__ inline void visit_seen(const HopArgs &a, uint32_t s, uint32_t next_list, uint32_t target, uint32_t seen) {
-    const unsigned calling = __activemask();
-    bool fresh = false;
-    if (target < a.N) {
-        /* a query's bits only go from 0 to 1, so a set bit read from L2 is
-         * final and saves the atomic; a clear one is settled by the atomic */
-        const uint32_t bit = 1u << (target & 31);
-        if (!(seen & bit)) fresh = !(atomicOr(&a.visited[(size_t)s * a.words + (target >> 5)], bit) & bit);
-    }
-    const unsigned appending = __ballot_sync(calling, fresh);
-    if (!fresh) return;
-    const unsigned peers = __match_any_sync(appending, s);
-    const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(&a.counts[s], (uint32_t)__popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    const uint32_t idx = base + __popc(peers & ((1u << lane) - 1u));
-    if (idx < a.N) a.lists[((size_t)s * 2 + next_list) * a.N + idx] = target;
+/* marks target reached by this hop for slot s, given its reached-set word
+ * `seen` (visited_word).  A query's bits only go from 0 to 1, so a set bit
+ * read from L2 is final and saves the atomic; a clear one is settled by it. */
+__device__ inline void visit_seen(const HopArgs &a, uint32_t s, uint32_t target, uint32_t seen) {
+    if (target >= a.N) return;
+    const uint32_t bit = 1u << (target & 31);
+    const size_t w = (size_t)s * a.words + (target >> 5);
+    if (!(seen & bit) && !(atomicOr(&a.visited[w], bit) & bit)) atomicOr(&a.fresh[w], bit);
 }
 
 /* one item's keys as the hop reads them: where they start, how many, and
@@ -92,7 +84,7 @@ __device__ inline void visit_seen(const HopArgs &a, uint32_t s, uint32_t next_li
 struct HopItem {
     const uint8_t *base;
     const uint8_t *end;      /* the end of the block's packed keys */
-    uint32_t n, s, nl, kind;
+    uint32_t n, s, kind, pad;
     uint32_t kb, off, fast, mbr_bit;
     uint32_t end_bit, dur_bit, end_mask, dur_mask;
     uint32_t id_mask, etm, window, t_start;
@@ -165,11 +157,10 @@ __global__ void __launch_bounds__(kHopThreads) k_serve_hop(HopArgs a) {
             const uint32_t b = a.rel[a.rel_off[lo] + bi];
             const uint32_t s = a.active[lo];
             const SlotParam sp = a.param[s];
-            const uint32_t obj = a.lists[((size_t)s * 2 + sp.cur) * a.N + f];
+            const uint32_t obj = a.front_ids[lo][f];
             const StoreBlockDev &blk = a.blocks[b];
             const uint32_t sid = blk.sids[obj];
             h.s = s;
-            h.nl = sp.cur ^ 1u;
             h.window = sp.window;
             h.t_start = sp.t_start;
             h.t_end = sp.t_end;
@@ -218,13 +209,12 @@ __global__ void __launch_bounds__(kHopThreads) k_serve_hop(HopArgs a) {
         /* kHopKeys keys per lane in flight: their loads, then their bitmap
          * words, then the (rare) atomics and appends */
         for (uint32_t k0 = 0; k0 < T; k0 += 32 * kHopKeys) {
-            uint32_t tg[kHopKeys], sl[kHopKeys], nx[kHopKeys], seen[kHopKeys];
+            uint32_t tg[kHopKeys], sl[kHopKeys], seen[kHopKeys];
 #pragma unroll
             for (int u = 0; u < kHopKeys; ++u) {
                 const uint32_t k = k0 + u * 32 + lane;
                 tg[u] = 0xffffffffu;
                 sl[u] = 0;
-                nx[u] = 0;
                 if (k < T) {
                     /* the last item whose first key is at or before k: it has
                      * keys, since an item without keys shares its offset with
@@ -236,7 +226,6 @@ __global__ void __launch_bounds__(kHopThreads) k_serve_hop(HopArgs a) {
                     const HopItem &x = wi[lo];
                     const uint32_t j = k - wo[lo];
                     sl[u] = x.s;
-                    nx[u] = x.nl;
                     uint32_t end, duration, t;
                     if (x.kind == 2 && x.fast) {
                         /* end, duration and target from one 64-bit window */
@@ -268,7 +257,7 @@ __global__ void __launch_bounds__(kHopThreads) k_serve_hop(HopArgs a) {
 #pragma unroll
             for (int u = 0; u < kHopKeys; ++u) seen[u] = visited_word(a, sl[u], tg[u]);
 #pragma unroll
-            for (int u = 0; u < kHopKeys; ++u) visit_seen(a, sl[u], nx[u], tg[u], seen[u]);
+            for (int u = 0; u < kHopKeys; ++u) visit_seen(a, sl[u], tg[u], seen[u]);
         }
         __syncwarp();
     }
@@ -283,176 +272,170 @@ __global__ void __launch_bounds__(kHopThreads) k_serve_hop(HopArgs a) {
  * times, so u has a key to a reached object v exactly when v has one to u;
  * and v was reached at the previous hop, since a v reached earlier would have
  * reached u already.  The reached set is read as it stood before the hop
- * (its bits are set after it, k_serve_mark), so the hop's result is the one
+ * (its marks join it after it, MarkOut), so the hop's result is the one
  * the frontier's own walk gives, and u stops at its first such key. */
 
-/* the unreached objects of pull slot blockIdx.y into its frontier list,
- * ascending within each warp's 1024 ids */
-__global__ void __launch_bounds__(256) k_serve_unvisited(HopArgs b, unsigned int *ucount) {
-    const uint32_t s = b.active[blockIdx.y];
-    const uint32_t *vis = b.visited + (size_t)s * b.words;
-    uint32_t *out = b.lists + ((size_t)s * 2 + b.param[s].cur) * b.N;
-    const int lane = threadIdx.x & 31;
-    const uint32_t nw = (b.N + 31) / 32;
-    for (uint32_t w0 = blockIdx.x * blockDim.x; w0 < nw; w0 += gridDim.x * blockDim.x) {
-        const uint32_t w = w0 + threadIdx.x;
-        uint32_t inv = 0;
-        if (w < nw) {
-            inv = ~vis[w];
-            if (w == nw - 1 && (b.N & 31)) inv &= (1u << (b.N & 31)) - 1u;
-        }
-        const uint32_t k = __popc(inv);
-        uint32_t incl = k;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        uint32_t base = 0;
-        if (lane == 31 && incl) base = atomicAdd(&ucount[s], incl);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        uint32_t at = base + incl - k;
-        while (inv) {
-            const int bit = __ffs(inv) - 1;
-            inv &= inv - 1u;
-            if (at < b.N) out[at] = w * 32 + (uint32_t)bit;
-            ++at;
-        }
-    }
-}
-
-/* one warp per unreached object: its keys in the slot's blocks, 32 blocks
- * at a time, until one reaches an object reached before this hop */
+/* one warp per bitmap word: for each of its unreached objects, the object's
+ * keys in the slot's blocks, 32 blocks at a time, until one reaches an object
+ * reached before this hop */
 __global__ void __launch_bounds__(256) k_serve_pull(HopArgs b) {
     const int lane = threadIdx.x & 31;
-    const unsigned long long total = b.prefix[b.A];
+    const uint32_t nw = (b.N + 31) / 32;
+    const unsigned long long total = (unsigned long long)b.A * nw;
     const unsigned long long nwarps = (unsigned long long)gridDim.x * (blockDim.x / 32);
     for (unsigned long long w = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) / 32; w < total;
          w += nwarps) {
-        uint32_t lo = 0, hi = b.A; /* prefix[lo] <= w < prefix[lo + 1] */
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) / 2;
-            if (b.prefix[mid] <= w) lo = mid;
-            else hi = mid;
-        }
+        const uint32_t lo = (uint32_t)(w / nw), word = (uint32_t)(w - (unsigned long long)lo * nw);
         const uint32_t s = b.active[lo];
-        const SlotParam sp = b.param[s];
-        const uint32_t u = b.lists[((size_t)s * 2 + sp.cur) * b.N + (w - b.prefix[lo])];
         const uint32_t *vis = b.visited + (size_t)s * b.words;
+        uint32_t left = ~vis[word];
+        if (word == nw - 1 && (b.N & 31)) left &= (1u << (b.N & 31)) - 1u;
+        if (!left) continue;
+        const SlotParam sp = b.param[s];
         const uint32_t r0 = b.rel_off[lo], nrel = b.rel_off[lo + 1] - r0;
-        bool found = false;
+        uint32_t got = 0;
         unsigned long long keys = 0;
-        for (uint32_t r = 0; r < nrel && !found; r += 32) {
-            bool hit = false;
-            if (r + lane < nrel) {
-                const StoreBlockDev &blk = b.blocks[b.rel[r0 + r + lane]];
-                const uint32_t sid = blk.sids[u];
-                uint32_t n = 0;
-                if (sid == 1) {
-                    n = blk.count[u];
-                    const ulonglong2 *k = blk.okeys + blk.first[u];
-                    for (uint32_t j = 0; j < n && !hit; ++j) {
-                        const ulonglong2 kk = k[j];
-                        const uint32_t end = (uint32_t)kk.x + blk.end_time_min, dur = (uint32_t)(kk.x >> 32);
-                        const uint32_t t = (uint32_t)kk.y & ((1u << 26) - 1);
-                        ++keys;
-                        if (sp.window && !((end - dur) < sp.t_end && sp.t_start < end)) continue;
-                        if (t < b.N && ((vis[t >> 5] >> (t & 31)) & 1u)) hit = true;
-                    }
-                } else if (sid >= 2 && sid - 2 < blk.C) {
-                    const uint32_t c = sid - 2;
-                    const glint_ctf_meta &m = blk.ctfs[c];
-                    const uint32_t kb = m.key_bit / 8;
-                    n = blk.count[u];
-                    const uint8_t *base =
-                        blk.keys + blk.byte_index[c] + (unsigned long long)(blk.first[u] - blk.key_index[c]) * kb;
-                    const uint8_t *kend = blk.keys + blk.key_bytes;
-                    for (uint32_t j = 0; j < n && !hit; ++j) {
-                        unsigned __int128 v = load_key(base + (size_t)j * kb, kb, kend);
-                        v >>= m.mbr_bit;
-                        const uint32_t end = (uint32_t)(v & ((1ull << m.end_bit) - 1)) + blk.end_time_min;
-                        v >>= m.end_bit;
-                        const uint32_t dur = (uint32_t)(v & ((1ull << m.duration_bit) - 1));
-                        v >>= m.duration_bit;
-                        const uint32_t t = (uint32_t)(v & ((1ull << m.id_bit) - 1));
-                        ++keys;
-                        if (sp.window && !((end - dur) < sp.t_end && sp.t_start < end)) continue;
-                        if (t < b.N && ((vis[t >> 5] >> (t & 31)) & 1u)) hit = true;
+        for (; left; left &= left - 1) {
+            const uint32_t u = word * 32 + (uint32_t)__ffs(left) - 1;
+            bool found = false;
+            for (uint32_t r = 0; r < nrel && !found; r += 32) {
+                bool hit = false;
+                if (r + lane < nrel) {
+                    const StoreBlockDev &blk = b.blocks[b.rel[r0 + r + lane]];
+                    const uint32_t sid = blk.sids[u];
+                    uint32_t n = 0;
+                    if (sid == 1) {
+                        n = blk.count[u];
+                        const ulonglong2 *k = blk.okeys + blk.first[u];
+                        for (uint32_t j = 0; j < n && !hit; ++j) {
+                            const ulonglong2 kk = k[j];
+                            const uint32_t end = (uint32_t)kk.x + blk.end_time_min, dur = (uint32_t)(kk.x >> 32);
+                            const uint32_t t = (uint32_t)kk.y & ((1u << 26) - 1);
+                            ++keys;
+                            if (sp.window && !((end - dur) < sp.t_end && sp.t_start < end)) continue;
+                            if (t < b.N && ((vis[t >> 5] >> (t & 31)) & 1u)) hit = true;
+                        }
+                    } else if (sid >= 2 && sid - 2 < blk.C) {
+                        const uint32_t c = sid - 2;
+                        const glint_ctf_meta &m = blk.ctfs[c];
+                        const uint32_t kb = m.key_bit / 8;
+                        n = blk.count[u];
+                        const uint8_t *base =
+                            blk.keys + blk.byte_index[c] + (unsigned long long)(blk.first[u] - blk.key_index[c]) * kb;
+                        const uint8_t *kend = blk.keys + blk.key_bytes;
+                        for (uint32_t j = 0; j < n && !hit; ++j) {
+                            unsigned __int128 v = load_key(base + (size_t)j * kb, kb, kend);
+                            v >>= m.mbr_bit;
+                            const uint32_t end = (uint32_t)(v & ((1ull << m.end_bit) - 1)) + blk.end_time_min;
+                            v >>= m.end_bit;
+                            const uint32_t dur = (uint32_t)(v & ((1ull << m.duration_bit) - 1));
+                            v >>= m.duration_bit;
+                            const uint32_t t = (uint32_t)(v & ((1ull << m.id_bit) - 1));
+                            ++keys;
+                            if (sp.window && !((end - dur) < sp.t_end && sp.t_start < end)) continue;
+                            if (t < b.N && ((vis[t >> 5] >> (t & 31)) & 1u)) hit = true;
+                        }
                     }
                 }
+                found = __any_sync(0xffffffffu, hit);
             }
-            found = __any_sync(0xffffffffu, hit);
+            if (found) got |= 1u << (u & 31);
         }
         for (int o = 16; o > 0; o >>= 1) keys += __shfl_down_sync(0xffffffffu, keys, o);
         if (lane == 0) {
             if (keys) atomicAdd(&b.scanned[s], keys);
-            if (found) {
-                const uint32_t idx = atomicAdd(&b.counts[s], 1u);
-                if (idx < b.N) b.lists[((size_t)s * 2 + (sp.cur ^ 1u)) * b.N + idx] = u;
-            }
+            if (got) b.fresh[(size_t)s * b.words + word] = got;
         }
     }
 }
 
-/* the objects a pull hop reached join the reached set of pull slot blockIdx.y */
-__global__ void k_serve_mark(HopArgs b) {
-    const uint32_t s = b.active[blockIdx.y];
-    const uint32_t n = min(b.counts[s], b.N);
-    const uint32_t *next = b.lists + ((size_t)s * 2 + (b.param[s].cur ^ 1u)) * b.N;
-    uint32_t *vis = b.visited + (size_t)s * b.words;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t u = next[i];
-        atomicOr(&vis[u >> 5], 1u << (u & 31));
-    }
-}
-
-/* the new ids of the active slots as (slot rank, id) keys: slot rank r's
- * count[r] ids start at off[r] */
-__global__ void k_serve_collect(const uint32_t *__restrict__ lists, uint32_t N, const uint32_t *__restrict__ act,
-                                const SlotParam *__restrict__ param, const unsigned long long *__restrict__ off,
-                                uint32_t A, unsigned long long *__restrict__ keys, uint32_t *__restrict__ vals) {
-    const unsigned long long total = off[A];
+/* the start of a round: the reached sets of the slots just admitted (their
+ * indices among the active ones come first in `admitted`) and the marks of
+ * every active slot cleared */
+__global__ void __launch_bounds__(256) k_serve_begin(HopArgs a, const uint32_t *__restrict__ admitted,
+                                                     uint32_t n_admitted) {
+    const unsigned long long per = a.words / 4, na = per * n_admitted, total = na + per * a.A;
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < total;
          i += (unsigned long long)gridDim.x * blockDim.x) {
-        uint32_t lo = 0, hi = A; /* off[lo] <= i < off[lo + 1] */
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) / 2;
-            if (off[mid] <= i) lo = mid;
-            else hi = mid;
-        }
-        const uint32_t s = act[lo];
-        const uint32_t id = lists[((size_t)s * 2 + param[s].cur) * N + (i - off[lo])];
-        keys[i] = ((unsigned long long)lo << 32) | id;
-        vals[i] = 0;
+        const bool adm = i < na;
+        const unsigned long long j = adm ? i : i - na;
+        const uint32_t r = (uint32_t)(j / per);
+        const uint32_t s = adm ? admitted[r] : a.active[r];
+        uint4 *w = reinterpret_cast<uint4 *>((adm ? a.visited : a.fresh) + (size_t)s * a.words);
+        w[j - (unsigned long long)r * per] = make_uint4(0, 0, 0, 0);
+        if (adm && j == (unsigned long long)r * per) a.scanned[s] = 0;
     }
 }
 
-__global__ void k_serve_ids(const unsigned long long *__restrict__ keys, uint64_t n, uint32_t *__restrict__ ids) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        ids[i] = (uint32_t)keys[i];
-}
-
-/* the seeds of newly admitted slots: visited, and listed as their frontier */
-__global__ void k_serve_seed(const uint32_t *__restrict__ seeds, const unsigned long long *__restrict__ sprefix,
+/* the seeds of newly admitted slots are reached */
+__global__ void k_serve_seed(const uint32_t *__restrict__ seeds, const uint32_t *__restrict__ sprefix,
                              const uint32_t *__restrict__ slots, uint32_t n_slots, HopArgs a) {
-    const unsigned long long total = sprefix[n_slots];
-    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < total;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
+    const uint32_t total = sprefix[n_slots];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = n_slots;
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) / 2;
             if (sprefix[mid] <= i) lo = mid;
             else hi = mid;
         }
-        const uint32_t s = slots[lo];
         const uint32_t p = seeds[i];
-        if (p >= a.N) continue;
-        uint32_t *vis = a.visited + (size_t)s * a.words;
-        const uint32_t bit = 1u << (p & 31);
-        if (atomicOr(&vis[p >> 5], bit) & bit) continue;
-        const uint32_t idx = atomicAdd(&a.counts[s], 1u);
-        a.lists[((size_t)s * 2 + a.param[s].cur) * a.N + idx] = p;
+        atomicOr(&a.visited[(size_t)slots[lo] * a.words + (p >> 5)], 1u << (p & 31));
     }
 }
+
+/* the marks of all active slots, slot after slot, as one scan: each word's
+ * count of marks, then its ids at its place of the result list; a slot's first
+ * place is where its ids start.  Pull hops read the reached sets as they stood
+ * before the hop, so their marks join them here (a walk's marks are in). */
+struct MarkIn {
+    const uint32_t *fresh;
+    const uint32_t *active;
+    uint32_t words;
+    __device__ const uint32_t *word(uint32_t i) const {
+        const uint32_t r = i / words;
+        return fresh + (size_t)active[r] * words + (i - r * words);
+    }
+    __device__ uint32_t at(uint32_t i) const { return __popc(*word(i)); }
+    __device__ void load(uint32_t base, uint32_t n, uint32_t (&v)[kScanItems]) const {
+        /* n and words are multiples of kScanItems: a thread's words are of
+         * one slot, and aligned */
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) v[k] = 0;
+        if (base >= n) return;
+        const uint4 *w = reinterpret_cast<const uint4 *>(word(base));
+#pragma unroll
+        for (int k = 0; k < kScanItems; k += 4) {
+            const uint4 x = w[k / 4];
+            v[k] = __popc(x.x);
+            v[k + 1] = __popc(x.y);
+            v[k + 2] = __popc(x.z);
+            v[k + 3] = __popc(x.w);
+        }
+    }
+};
+struct MarkOut {
+    MarkIn in;
+    uint32_t *visited;
+    uint32_t *ids;             /* the result list */
+    unsigned long long *off;   /* [A + 1] */
+    uint32_t A;
+    __device__ void total(uint32_t, uint32_t sum) const { off[A] = sum; }
+    __device__ void store(uint32_t base, uint32_t n, const uint32_t (&v)[kScanItems],
+                          const uint32_t (&o)[kScanItems]) const {
+        if (base >= n) return;
+        const uint32_t r = base / in.words, w0 = base - r * in.words;
+        if (w0 == 0) off[r] = o[0];
+        const uint32_t *f = in.word(base);
+        uint32_t *vis = visited + (size_t)in.active[r] * in.words + w0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (!v[k]) continue;
+            uint32_t m = f[k], at = o[k];
+            vis[k] |= m;
+            for (; m; m &= m - 1) ids[at++] = (w0 + k) * 32 + (uint32_t)__ffs(m) - 1;
+        }
+    }
+};
 
 } // namespace glint
 
@@ -467,7 +450,8 @@ struct PendingQuery {
 struct SlotState {
     bool busy = false;
     uint64_t ticket = 0;
-    uint32_t hops = 0, hop = 0, cur = 0, frontier = 0;
+    uint32_t hops = 0, hop = 0, frontier = 0;
+    const uint32_t *front_ids = nullptr; /* device: the last hop's part of the result list, or the seeds */
     uint64_t reached = 0; /* seeds and every hop's new objects so far */
     std::vector<uint32_t> ids;
     uint64_t hop_end[kMaxHops] = {};
@@ -482,65 +466,73 @@ struct FinishedQuery {
 struct glint_server {
     glint_ctx *ctx = nullptr;
     uint32_t slots = 0;
-    uint64_t words = 0;
-    uint32_t *visited = nullptr, *lists = nullptr, *counts = nullptr, *active = nullptr, *seed_slots = nullptr;
-    SlotParam *param = nullptr;
-    unsigned long long *scanned = nullptr, *prefix = nullptr, *sprefix = nullptr;
-    uint32_t *front = nullptr;
-    unsigned long long *pprefix = nullptr; /* pull slots' items (their unreached objects), prefix sums */
-    unsigned int *ucount = nullptr;        /* [slot] unreached objects listed */
-    uint32_t *seeds = nullptr;
-    uint64_t seeds_cap = 0;
-    StoreBlockDev *blocks = nullptr;
-    uint32_t blocks_cap = 0;
-    uint32_t *rel = nullptr, *rel_off = nullptr;   /* each active slot's blocks (the window's) */
-    uint64_t rel_cap = 0, rel_off_cap = 0;
+    uint32_t words = 0;
+    uint32_t *visited = nullptr, *fresh = nullptr;
+    uint32_t *ids[2] = {nullptr, nullptr}; /* the result lists of this round and the last: [slots * N] */
+    uint32_t side = 0;                     /* which of them the next round writes */
+    unsigned long long *out = nullptr;     /* keys read per slot [slots], the result list's offsets [slots + 1] */
+    unsigned long long *h_out = nullptr;   /* page-locked: the same */
+    uint8_t *ctl = nullptr, *h_ctl = nullptr; /* a round's control arrays: device, page-locked */
+    uint64_t ctl_cap = 0;
+    uint32_t *h_ids = nullptr;             /* page-locked: results on their way to the queries */
+    void *scan_tmp = nullptr;
     uint64_t next_ticket = 1;
     std::deque<PendingQuery> queue;
     std::vector<SlotState> state;
     std::vector<SlotParam> hparam;
     std::unordered_map<uint64_t, FinishedQuery> done;
-    std::vector<uint32_t> buf;
-    /* a hop's new ids of all active slots, sorted by (slot, id) on the device */
-    unsigned long long *rk = nullptr, *rk2 = nullptr, *roff = nullptr;
-    uint32_t *rv = nullptr, *rv2 = nullptr, *rids = nullptr;
-    void *rs_tmp = nullptr, *rscan = nullptr;
-    uint64_t r_cap = 0;
 };
 
+constexpr uint64_t kIdsStage = 1u << 20; /* ids per copy to the host */
+
 static void server_release(glint_server *v) {
-    void *ps[] = {v->visited, v->lists, v->counts, v->active, v->seed_slots, v->param, v->scanned, v->prefix,
-                  v->sprefix, v->seeds, v->blocks, v->rk, v->rk2, v->roff, v->rv, v->rv2, v->rids, v->rs_tmp,
-                  v->rscan, v->rel, v->rel_off, v->front, v->pprefix, v->ucount};
+    void *ps[] = {v->visited, v->fresh, v->ids[0], v->ids[1], v->out, v->ctl, v->scan_tmp};
     for (void *p : ps)
         if (p) cudaFree(p);
+    void *hs[] = {v->h_out, v->h_ctl, v->h_ids};
+    for (void *p : hs)
+        if (p) cudaFreeHost(p);
+    v->visited = v->fresh = v->ids[0] = v->ids[1] = v->h_ids = nullptr;
+    v->out = v->h_out = nullptr;
+    v->ctl = v->h_ctl = nullptr;
+    v->ctl_cap = 0;
+    v->scan_tmp = nullptr;
 }
 
-/* the results' sort buffers for n ids over `act` slots (grown, never shrunk) */
-static cudaError_t server_result_space(glint_server *v, uint64_t n, uint32_t act) {
-    if (n <= v->r_cap && v->roff) return cudaSuccess;
-    const uint64_t cap = std::max<uint64_t>(n, 1u << 20);
-    void *ps[] = {v->rk, v->rk2, v->rv, v->rv2, v->rids, v->rs_tmp, v->rscan};
-    for (void *p : ps)
-        if (p) cudaFree(p);
-    v->rk = v->rk2 = nullptr;
-    v->rv = v->rv2 = v->rids = nullptr;
-    v->rs_tmp = v->rscan = nullptr;
-    v->r_cap = 0;
-    cudaError_t e = cudaMalloc((void **)&v->rk, sizeof(unsigned long long) * cap);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&v->rk2, sizeof(unsigned long long) * cap);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&v->rv, sizeof(uint32_t) * cap);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&v->rv2, sizeof(uint32_t) * cap);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&v->rids, sizeof(uint32_t) * cap);
-    if (e == cudaSuccess) e = cudaMalloc(&v->rs_tmp, radix_tmp_bytes(cap));
-    const size_t scan_bytes = scan_tmp_bytes(256 * ((cap + 1023) / 1024) + 1);
-    if (e == cudaSuccess) e = cudaMalloc(&v->rscan, scan_bytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(v->rscan, 0, scan_bytes, v->ctx->stream);
-    if (e == cudaSuccess && !v->roff) e = cudaMalloc((void **)&v->roff, sizeof(unsigned long long) * (v->slots + 1));
-    if (e == cudaSuccess) v->r_cap = cap;
-    (void)act;
-    return e;
-}
+/* a round's control arrays, laid out one after the other in page-locked
+ * memory and copied to the device at once */
+class Control {
+public:
+    template <class T>
+    size_t add(const T *p, size_t n) {
+        const size_t at = (bytes_.size() + 15) & ~(size_t)15;
+        bytes_.resize(at + sizeof(T) * std::max<size_t>(n, 1));
+        if (n) std::memcpy(bytes_.data() + at, p, sizeof(T) * n);
+        return at;
+    }
+    template <class T>
+    size_t add(const std::vector<T> &v) {
+        return add(v.data(), v.size());
+    }
+    /* room for n bytes in v's buffers (grown by half again, kept) */
+    static cudaError_t room(glint_server *v, size_t n) {
+        if (v->ctl_cap >= n) return cudaSuccess;
+        if (v->ctl) cudaFree(v->ctl);
+        if (v->h_ctl) cudaFreeHost(v->h_ctl);
+        v->ctl = v->h_ctl = nullptr;
+        v->ctl_cap = 0;
+        const size_t cap = std::max<size_t>(n + n / 2, 1u << 16);
+        cudaError_t e = cudaMalloc((void **)&v->ctl, cap);
+        if (e == cudaSuccess) e = cudaMallocHost((void **)&v->h_ctl, cap);
+        if (e == cudaSuccess) v->ctl_cap = cap;
+        return e;
+    }
+    size_t size() const { return bytes_.size(); }
+    uint8_t *data() { return bytes_.data(); }
+
+private:
+    std::vector<uint8_t> bytes_;
+};
 
 extern "C" glint_status glint_server_create(glint_ctx *c, uint32_t max_slots, glint_server **out) {
     if (!c || !out || max_slots == 0) return GLINT_ERR_INVALID_ARGUMENT;
@@ -548,30 +540,33 @@ extern "C" glint_status glint_server_create(glint_ctx *c, uint32_t max_slots, gl
     cudaSetDevice(c->device);
     glint_server *v = new glint_server();
     v->ctx = c;
-    v->words = ((uint64_t)c->N + 31) / 32;
-    /* admission by memory: a slot costs its bitmap and two lists */
-    const size_t slot_bytes = sizeof(uint32_t) * (v->words + 2 * (size_t)c->N) + 64;
+    /* whole scan threads per slot */
+    v->words = (uint32_t)((((uint64_t)c->N + 31) / 32 + kScanItems - 1) / kScanItems * kScanItems);
+    /* admission by memory: a slot costs its two bitmaps and its part of the
+     * two result lists */
+    const size_t slot_bytes = sizeof(uint32_t) * (2 * (size_t)v->words + 2 * (size_t)c->N) + 64;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     const size_t fit = (free_b / 2) / slot_bytes;
-    v->slots = (uint32_t)std::min<size_t>(max_slots, std::max<size_t>(fit, 1));
+    /* the marks of all slots are one scan of 32-bit length */
+    const size_t most = std::max<size_t>(1, 0xf0000000ull / v->words);
+    v->slots = (uint32_t)std::min<size_t>(std::min<size_t>(max_slots, most), std::max<size_t>(fit, 1));
     const uint32_t S = v->slots;
     cudaError_t e = cudaSuccess;
     auto A = [&](void **p, size_t n) {
         if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1);
     };
-    A((void **)&v->visited, sizeof(uint32_t) * v->words * S);
-    A((void **)&v->lists, sizeof(uint32_t) * 2 * (size_t)c->N * S);
-    A((void **)&v->counts, sizeof(uint32_t) * S);
-    A((void **)&v->active, sizeof(uint32_t) * S);
-    A((void **)&v->seed_slots, sizeof(uint32_t) * S);
-    A((void **)&v->param, sizeof(SlotParam) * S);
-    A((void **)&v->scanned, sizeof(unsigned long long) * S);
-    A((void **)&v->prefix, sizeof(unsigned long long) * (S + 1));
-    A((void **)&v->front, sizeof(uint32_t) * S);
-    A((void **)&v->pprefix, sizeof(unsigned long long) * (S + 1));
-    A((void **)&v->ucount, sizeof(unsigned int) * S);
-    A((void **)&v->sprefix, sizeof(unsigned long long) * (S + 1));
+    const size_t scan_bytes = scan_tmp_bytes((size_t)v->words * S);
+    A((void **)&v->visited, sizeof(uint32_t) * (size_t)v->words * S);
+    A((void **)&v->fresh, sizeof(uint32_t) * (size_t)v->words * S);
+    A((void **)&v->ids[0], sizeof(uint32_t) * (size_t)c->N * S);
+    A((void **)&v->ids[1], sizeof(uint32_t) * (size_t)c->N * S);
+    A((void **)&v->out, sizeof(unsigned long long) * (2 * (size_t)S + 1));
+    A(&v->scan_tmp, scan_bytes);
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&v->h_out, sizeof(unsigned long long) * (2 * (size_t)S + 1));
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&v->h_ids, sizeof(uint32_t) * kIdsStage);
+    if (e == cudaSuccess) e = Control::room(v, 1u << 16);
+    if (e == cudaSuccess) e = cudaMemsetAsync(v->scan_tmp, 0, scan_bytes, c->stream);
     if (e != cudaSuccess) {
         server_release(v);
         delete v;
@@ -622,24 +617,15 @@ static glint_status server_fail(glint_server *v, cudaError_t e, const char *wher
     return e == cudaErrorMemoryAllocation ? GLINT_ERR_OUT_OF_MEMORY : GLINT_ERR_CUDA;
 }
 
-static HopArgs server_args(glint_server *v, uint32_t nb) {
-    HopArgs a;
-    a.blocks = v->blocks;
-    a.nblocks = nb;
-    a.N = v->ctx->N;
-    a.words = v->words;
-    a.visited = v->visited;
-    a.lists = v->lists;
-    a.param = v->param;
-    a.counts = v->counts;
-    a.scanned = v->scanned;
-    a.active = v->active;
-    a.prefix = v->prefix;
-    a.front = v->front;
-    a.rel = v->rel;
-    a.rel_off = v->rel_off;
-    a.A = 0;
-    return a;
+/* the slot's query is done */
+static void server_finish(glint_server *v, SlotState &st, uint64_t keys_scanned) {
+    for (uint32_t h = st.hop; h < kMaxHops; ++h) st.hop_end[h] = st.ids.size();
+    FinishedQuery f;
+    f.ids = std::move(st.ids);
+    std::memcpy(f.hop_end, st.hop_end, sizeof(f.hop_end));
+    f.keys_scanned = keys_scanned;
+    v->done[st.ticket] = std::move(f);
+    st = SlotState();
 }
 
 extern "C" glint_status glint_server_step(glint_server *v, uint32_t *n_active, uint32_t *n_queued) {
@@ -650,222 +636,162 @@ extern "C" glint_status glint_server_step(glint_server *v, uint32_t *n_active, u
     cudaStream_t s = c->stream;
     const uint32_t N = c->N;
     cudaError_t e;
+    Control ctl;
     /* the kept blocks, as device descriptors */
     const uint32_t nb = (uint32_t)c->ctbs.size();
-    if (v->blocks_cap < nb) {
-        if (v->blocks) cudaFree(v->blocks);
-        v->blocks = nullptr;
-        v->blocks_cap = 0;
-        if ((e = cudaMalloc((void **)&v->blocks, sizeof(StoreBlockDev) * nb)) != cudaSuccess)
-            return server_fail(v, e, "blocks");
-        v->blocks_cap = nb;
-    }
     std::vector<StoreBlockDev> bd(nb);
     for (uint32_t i = 0; i < nb; ++i) {
         const StoreBlock &b = c->ctbs[i];
         bd[i] = StoreBlockDev{b.keys, b.key_bytes, b.ctfs, b.key_index, b.byte_index, b.sids, b.first, b.count,
                               b.okeys, b.end_time_min, b.C};
     }
-    if (nb) cudaMemcpyAsync(v->blocks, bd.data(), sizeof(StoreBlockDev) * nb, cudaMemcpyHostToDevice, s);
-    HopArgs a = server_args(v, nb);
+    const size_t at_blocks = ctl.add(bd);
 
-    /* admission: queued queries into free slots */
-    std::vector<uint32_t> admitted;
-    std::vector<uint32_t> seeds;
-    std::vector<unsigned long long> sprefix(1, 0);
+    /* admission: queued queries into free slots; their seeds, each once, are
+     * their first frontier */
+    std::vector<uint32_t> admitted, seeds, sprefix(1, 0);
     for (uint32_t k = 0; k < v->slots && !v->queue.empty(); ++k) {
         SlotState &st = v->state[k];
         if (st.busy) continue;
         PendingQuery q = std::move(v->queue.front());
         v->queue.pop_front();
+        std::sort(q.seeds.begin(), q.seeds.end());
+        q.seeds.erase(std::unique(q.seeds.begin(), q.seeds.end()), q.seeds.end());
+        while (!q.seeds.empty() && q.seeds.back() >= N) q.seeds.pop_back();
         st = SlotState();
         st.busy = true;
         st.ticket = q.ticket;
         st.hops = q.hops;
+        st.frontier = (uint32_t)q.seeds.size();
+        st.reached = st.frontier;
         v->hparam[k] = SlotParam{q.t_start, q.t_end, (q.t_start == 0 && q.t_end == 0) ? 0u : 1u, 0u};
         admitted.push_back(k);
         seeds.insert(seeds.end(), q.seeds.begin(), q.seeds.end());
-        sprefix.push_back(seeds.size());
+        sprefix.push_back((uint32_t)seeds.size());
     }
-    if (!admitted.empty()) {
-        if (v->seeds_cap < seeds.size()) {
-            if (v->seeds) cudaFree(v->seeds);
-            v->seeds = nullptr;
-            v->seeds_cap = 0;
-            if ((e = cudaMalloc((void **)&v->seeds, sizeof(uint32_t) * seeds.size())) != cudaSuccess)
-                return server_fail(v, e, "seeds");
-            v->seeds_cap = seeds.size();
-        }
-        for (uint32_t k : admitted) {
-            cudaMemsetAsync(v->visited + (size_t)k * v->words, 0, sizeof(uint32_t) * v->words, s);
-            cudaMemsetAsync(v->counts + k, 0, sizeof(uint32_t), s);
-            cudaMemsetAsync(v->scanned + k, 0, sizeof(unsigned long long), s);
-        }
-        cudaMemcpyAsync(v->param, v->hparam.data(), sizeof(SlotParam) * v->slots, cudaMemcpyHostToDevice, s);
-        if (!seeds.empty())
-            cudaMemcpyAsync(v->seeds, seeds.data(), sizeof(uint32_t) * seeds.size(), cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(v->sprefix, sprefix.data(), sizeof(unsigned long long) * sprefix.size(),
-                        cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(v->seed_slots, admitted.data(), sizeof(uint32_t) * admitted.size(), cudaMemcpyHostToDevice,
-                        s);
-        if (!seeds.empty())
-            k_serve_seed<<<grid_for(seeds.size(), 256), 256, 0, s>>>(v->seeds, v->sprefix, v->seed_slots,
-                                                                      (uint32_t)admitted.size(), a);
-        std::vector<uint32_t> cnt(v->slots);
-        cudaMemcpyAsync(cnt.data(), v->counts, sizeof(uint32_t) * v->slots, cudaMemcpyDeviceToHost, s);
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return server_fail(v, e, "seed");
-        for (uint32_t k : admitted) v->state[k].frontier = v->state[k].reached = cnt[k];
-    }
+    const size_t at_seeds = ctl.add(seeds), at_sprefix = ctl.add(sprefix), at_admitted = ctl.add(admitted);
 
     /* one hop for every active slot, over the kept blocks that can hold a
      * key inside its window: a key of a block ends at most at end_time_max
      * and starts no earlier than start_min, and it counts when
-     * start < t_end and t_start < end */
-    std::vector<uint32_t> act, rel, front;
-    std::vector<uint32_t> rel_off(1, 0);
-    std::vector<unsigned long long> prefix(1, 0), pprefix(1, 0);
-    /* frontier walks first, then the pull slots (their frontier reaches at
-     * least as many objects as are left) */
-    std::vector<uint32_t> order;
+     * start < t_end and t_start < end.  Frontier walks first, then the pull
+     * slots (their frontier reaches at least as many objects as are left). */
+    std::vector<uint32_t> act, rel, front, rel_off(1, 0);
+    std::vector<unsigned long long> prefix(1, 0);
+    uint32_t n_push = 0;
     for (int pass = 0; pass < 2; ++pass)
         for (uint32_t k = 0; k < v->slots; ++k) {
             const SlotState &st = v->state[k];
             if (!st.busy || st.hop >= st.hops) continue;
             const bool pull = (uint64_t)st.frontier >= (uint64_t)N - st.reached;
-            if (pull == (pass == 1)) order.push_back(k);
+            if (pull != (pass == 1)) continue;
+            act.push_back(k);
+            front.push_back(st.frontier);
+            const SlotParam &sp = v->hparam[k];
+            uint32_t nrel = 0;
+            for (uint32_t i = 0; i < nb; ++i) {
+                const StoreBlock &b = c->ctbs[i];
+                if (sp.window && b.spans_known && !(b.start_min < sp.t_end && sp.t_start < b.end_time_max)) continue;
+                rel.push_back(i);
+                ++nrel;
+            }
+            rel_off.push_back((uint32_t)rel.size());
+            if (!pull) {
+                prefix.push_back(prefix.back() + (unsigned long long)st.frontier * nrel);
+                ++n_push;
+            }
         }
-    uint32_t n_push = 0;
-    for (uint32_t k : order) {
-        const SlotState &st = v->state[k];
-        const bool pull = (uint64_t)st.frontier >= (uint64_t)N - st.reached;
-        act.push_back(k);
-        front.push_back(st.frontier);
-        const SlotParam &sp = v->hparam[k];
-        uint32_t nrel = 0;
-        for (uint32_t i = 0; i < nb; ++i) {
-            const StoreBlock &b = c->ctbs[i];
-            if (sp.window && b.spans_known && !(b.start_min < sp.t_end && sp.t_start < b.end_time_max)) continue;
-            rel.push_back(i);
-            ++nrel;
-        }
-        rel_off.push_back((uint32_t)rel.size());
-        if (pull) {
-            pprefix.push_back(pprefix.back() + ((uint64_t)N - st.reached));
-        } else {
-            prefix.push_back(prefix.back() + (unsigned long long)st.frontier * nrel);
-            ++n_push;
-        }
-    }
     if (!act.empty()) {
-        if (v->rel_cap < rel.size() + 1) {
-            if (v->rel) cudaFree(v->rel);
-            v->rel = nullptr;
-            v->rel_cap = 0;
-            if ((e = cudaMalloc((void **)&v->rel, sizeof(uint32_t) * (rel.size() + 1))) != cudaSuccess)
-                return server_fail(v, e, "blocks of the windows");
-            v->rel_cap = rel.size() + 1;
-        }
-        if (v->rel_off_cap < rel_off.size()) {
-            if (v->rel_off) cudaFree(v->rel_off);
-            v->rel_off = nullptr;
-            v->rel_off_cap = 0;
-            if ((e = cudaMalloc((void **)&v->rel_off, sizeof(uint32_t) * rel_off.size())) != cudaSuccess)
-                return server_fail(v, e, "blocks of the windows");
-            v->rel_off_cap = rel_off.size();
-        }
-        a.rel = v->rel;
-        a.rel_off = v->rel_off;
-        cudaMemcpyAsync(v->param, v->hparam.data(), sizeof(SlotParam) * v->slots, cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(v->active, act.data(), sizeof(uint32_t) * act.size(), cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(v->front, front.data(), sizeof(uint32_t) * front.size(), cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(v->prefix, prefix.data(), sizeof(unsigned long long) * prefix.size(), cudaMemcpyHostToDevice,
-                        s);
-        cudaMemcpyAsync(v->pprefix, pprefix.data(), sizeof(unsigned long long) * pprefix.size(),
-                        cudaMemcpyHostToDevice, s);
-        if (!rel.empty())
-            cudaMemcpyAsync(v->rel, rel.data(), sizeof(uint32_t) * rel.size(), cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(v->rel_off, rel_off.data(), sizeof(uint32_t) * rel_off.size(), cudaMemcpyHostToDevice, s);
-        for (uint32_t k : act) cudaMemsetAsync(v->counts + k, 0, sizeof(uint32_t), s);
-        a.A = n_push;
+        const uint32_t A = (uint32_t)act.size();
+        const size_t at_param = ctl.add(v->hparam), at_act = ctl.add(act), at_front = ctl.add(front),
+                     at_prefix = ctl.add(prefix), at_rel = ctl.add(rel), at_rel_off = ctl.add(rel_off);
+        std::vector<const uint32_t *> fids(A, nullptr);
+        const size_t at_fids = ctl.add(fids);
+        if ((e = Control::room(v, ctl.size())) != cudaSuccess) return server_fail(v, e, "control arrays");
+        for (uint32_t i = 0; i < admitted.size(); ++i)
+            v->state[admitted[i]].front_ids = reinterpret_cast<const uint32_t *>(v->ctl + at_seeds) + sprefix[i];
+        for (uint32_t i = 0; i < A; ++i) fids[i] = v->state[act[i]].front_ids;
+        std::memcpy(ctl.data() + at_fids, fids.data(), sizeof(uint32_t *) * A);
+        std::memcpy(v->h_ctl, ctl.data(), ctl.size());
+        cudaMemcpyAsync(v->ctl, v->h_ctl, ctl.size(), cudaMemcpyHostToDevice, s);
+        auto dev = [&](auto *type, size_t at) { return reinterpret_cast<decltype(type)>(v->ctl + at); };
+        HopArgs a;
+        a.blocks = dev((const StoreBlockDev *)nullptr, at_blocks);
+        a.N = N;
+        a.words = v->words;
+        a.visited = v->visited;
+        a.fresh = v->fresh;
+        a.param = dev((const SlotParam *)nullptr, at_param);
+        a.scanned = v->out;
+        a.active = dev((const uint32_t *)nullptr, at_act);
+        a.front = dev((const uint32_t *)nullptr, at_front);
+        a.front_ids = dev((const uint32_t *const *)nullptr, at_fids);
+        a.prefix = dev((const unsigned long long *)nullptr, at_prefix);
+        a.rel = dev((const uint32_t *)nullptr, at_rel);
+        a.rel_off = dev((const uint32_t *)nullptr, at_rel_off);
+        a.A = A;
+        const uint32_t n_adm = (uint32_t)admitted.size();
+        const uint32_t *d_adm = dev((const uint32_t *)nullptr, at_admitted);
+        k_serve_begin<<<grid_for((uint64_t)(v->words / 4) * (A + n_adm), 256, 152u * 8u), 256, 0, s>>>(a, d_adm, n_adm);
+        if (!seeds.empty())
+            k_serve_seed<<<grid_for(seeds.size(), 256), 256, 0, s>>>(dev((const uint32_t *)nullptr, at_seeds),
+                                                                     dev((const uint32_t *)nullptr, at_sprefix), d_adm,
+                                                                     n_adm, a);
         const unsigned long long items = prefix.back();
-        if (items) k_serve_hop<<<grid_for((items + 31) / 32, kHopThreads / 32, 152u * 8u), kHopThreads, 0, s>>>(a);
-        const uint32_t n_pull = (uint32_t)act.size() - n_push;
-        if (n_pull) {
+        if (items) {
+            a.A = n_push;
+            k_serve_hop<<<grid_for((items + 31) / 32, kHopThreads / 32, 152u * 8u), kHopThreads, 0, s>>>(a);
+        }
+        if (A > n_push) {
             HopArgs b = a;
-            b.active = v->active + n_push;
-            b.rel_off = v->rel_off + n_push;
-            b.prefix = v->pprefix;
-            b.A = n_pull;
-            for (uint32_t i = n_push; i < act.size(); ++i) cudaMemsetAsync(v->ucount + act[i], 0, sizeof(unsigned), s);
-            const uint32_t nw = (N + 31) / 32;
-            k_serve_unvisited<<<dim3(std::min<uint32_t>((nw + 255) / 256, 1024u), n_pull), 256, 0, s>>>(b, v->ucount);
-            const unsigned long long objs = pprefix.back();
-            if (objs) k_serve_pull<<<grid_for(objs, 8, 152u * 16u), 256, 0, s>>>(b);
-            k_serve_mark<<<dim3(64, n_pull), 256, 0, s>>>(b);
+            b.active = a.active + n_push;
+            b.rel_off = a.rel_off + n_push;
+            b.A = A - n_push;
+            k_serve_pull<<<grid_for((uint64_t)b.A * ((N + 31) / 32), 8, 152u * 16u), 256, 0, s>>>(b);
         }
-        std::vector<uint32_t> cnt(v->slots);
-        std::vector<unsigned long long> scanned(v->slots);
-        cudaMemcpyAsync(cnt.data(), v->counts, sizeof(uint32_t) * v->slots, cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(scanned.data(), v->scanned, sizeof(unsigned long long) * v->slots, cudaMemcpyDeviceToHost, s);
+        MarkOut mo;
+        mo.in = MarkIn{v->fresh, a.active, v->words};
+        mo.visited = v->visited;
+        mo.ids = v->ids[v->side];
+        mo.off = v->out + v->slots;
+        mo.A = A;
+        scan_launch(mo.in, mo, v->words * A, nullptr, v->scan_tmp, s);
+        cudaMemcpyAsync(v->h_out, v->out, sizeof(unsigned long long) * (v->slots + (size_t)A + 1),
+                        cudaMemcpyDeviceToHost, s);
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return server_fail(v, e, "hop");
-        /* the hop's new ids of every active slot, in (slot, id) order: one
-         * sort and one copy for all of them */
-        std::vector<unsigned long long> roff(act.size() + 1, 0);
-        for (size_t i = 0; i < act.size(); ++i) roff[i + 1] = roff[i] + std::min(cnt[act[i]], N);
-        const uint64_t total = roff.back();
-        if (total) {
-            if ((e = server_result_space(v, total, (uint32_t)act.size())) != cudaSuccess)
-                return server_fail(v, e, "results");
-            for (uint32_t k : act) v->hparam[k].cur ^= 1u; /* the lists the hop wrote */
-            cudaMemcpyAsync(v->param, v->hparam.data(), sizeof(SlotParam) * v->slots, cudaMemcpyHostToDevice, s);
-            cudaMemcpyAsync(v->roff, roff.data(), sizeof(unsigned long long) * roff.size(), cudaMemcpyHostToDevice,
-                            s);
-            k_serve_collect<<<grid_for(total, 256), 256, 0, s>>>(v->lists, N, v->active, v->param, v->roff,
-                                                                 (uint32_t)act.size(), v->rk, v->rv);
-            for (uint32_t k : act) v->hparam[k].cur ^= 1u;
-            const int bits = 32 + std::max(1, radix_bits_for(act.size() - 1));
-            if ((e = radix_sort_u64(v->rk, v->rv, v->rk2, v->rv2, total, bits, v->rs_tmp, v->rscan, s)) !=
-                cudaSuccess)
-                return server_fail(v, e, "results sort");
-            k_serve_ids<<<grid_for(total, 256), 256, 0, s>>>(v->rk, total, v->rids);
-            v->buf.resize(total);
-            cudaMemcpyAsync(v->buf.data(), v->rids, sizeof(uint32_t) * total, cudaMemcpyDeviceToHost, s);
+        const unsigned long long *off = v->h_out + v->slots;
+        /* the new ids, in stages, to their queries */
+        for (uint32_t i = 0; i < A; ++i)
+            v->state[act[i]].ids.reserve(v->state[act[i]].ids.size() + (off[i + 1] - off[i]));
+        uint32_t i = 0;
+        for (unsigned long long at = 0; at < off[A]; at += kIdsStage) {
+            const unsigned long long end = std::min<unsigned long long>(at + kIdsStage, off[A]);
+            cudaMemcpyAsync(v->h_ids, mo.ids + at, sizeof(uint32_t) * (end - at), cudaMemcpyDeviceToHost, s);
             if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return server_fail(v, e, "results");
+            for (unsigned long long p = at; p < end;) {
+                while (off[i + 1] <= p) ++i;
+                const unsigned long long q = std::min(off[i + 1], end);
+                std::vector<uint32_t> &ids = v->state[act[i]].ids;
+                ids.insert(ids.end(), v->h_ids + (p - at), v->h_ids + (q - at));
+                p = q;
+            }
         }
-        for (size_t ai = 0; ai < act.size(); ++ai) {
-            const uint32_t k = act[ai];
-            SlotState &st = v->state[k];
-            const uint32_t got = std::min(cnt[k], N);
-            const uint32_t nl = v->hparam[k].cur ^ 1u;
-            if (got) st.ids.insert(st.ids.end(), v->buf.begin() + roff[ai], v->buf.begin() + roff[ai + 1]);
+        for (uint32_t ai = 0; ai < A; ++ai) {
+            SlotState &st = v->state[act[ai]];
+            const uint32_t got = (uint32_t)(off[ai + 1] - off[ai]);
             st.hop_end[st.hop] = st.ids.size();
             ++st.hop;
             st.frontier = got;
+            st.front_ids = mo.ids + off[ai];
             st.reached += got;
-            v->hparam[k].cur = nl;
-            if (st.hop >= st.hops || got == 0) {
-                for (uint32_t h = st.hop; h < kMaxHops; ++h) st.hop_end[h] = st.ids.size();
-                FinishedQuery f;
-                f.ids = std::move(st.ids);
-                std::memcpy(f.hop_end, st.hop_end, sizeof(f.hop_end));
-                f.keys_scanned = scanned[k];
-                v->done[st.ticket] = std::move(f);
-                st = SlotState();
-            }
+            if (st.hop >= st.hops || got == 0) server_finish(v, st, v->h_out[act[ai]]);
         }
+        v->side ^= 1u;
     }
     /* queries admitted with an empty frontier or zero kept blocks finish here */
     for (uint32_t k = 0; k < v->slots; ++k) {
         SlotState &st = v->state[k];
-        if (st.busy && st.frontier == 0 && st.hop < st.hops) {
-            for (uint32_t h = st.hop; h < kMaxHops; ++h) st.hop_end[h] = st.ids.size();
-            FinishedQuery f;
-            f.ids = std::move(st.ids);
-            std::memcpy(f.hop_end, st.hop_end, sizeof(f.hop_end));
-            f.keys_scanned = 0;
-            v->done[st.ticket] = std::move(f);
-            st = SlotState();
-        }
+        if (st.busy && st.frontier == 0 && st.hop < st.hops) server_finish(v, st, 0);
     }
     if (n_active) {
         uint32_t n = 0;
@@ -904,13 +830,6 @@ void server_free_default(glint_ctx *c) {
 void servers_detach(glint_ctx *c) {
     for (glint_server *v : c->servers) {
         server_release(v);
-        v->visited = v->lists = v->counts = v->active = v->seed_slots = v->seeds = nullptr;
-        v->param = nullptr;
-        v->scanned = v->prefix = v->sprefix = nullptr;
-        v->blocks = nullptr;
-        v->rel = v->rel_off = v->front = nullptr;
-        v->pprefix = nullptr;
-        v->ucount = nullptr;
         v->ctx = nullptr;
     }
     c->servers.clear();

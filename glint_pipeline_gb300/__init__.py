@@ -162,19 +162,18 @@ class DeviceBench:
         (search_multi, cuda/geometry.cu:605-663), in bucket order."""
         p = np.ascontiguousarray(pids, dtype=np.uint32)
         n = ctypes.c_uint64()
-        if cap is None:
-            st = self.lib.glint_active_search(self.h, p.ctypes.data_as(ctypes.c_void_p), p.shape[0], None, 0,
+        # without a cap: room for a first guess, and once more where it is short
+        room = max(4096, 32 * p.shape[0]) if cap is None else int(cap)
+        while True:
+            out = np.empty(room, dtype=SEARCH_DTYPE)
+            st = self.lib.glint_active_search(self.h, p.ctypes.data_as(ctypes.c_void_p), p.shape[0],
+                                              out.ctypes.data_as(ctypes.c_void_p) if room else None, room,
                                               ctypes.byref(n))
             if st != 0:
                 raise GlintError(st, self.last_error())
-            cap = n.value
-        out = np.zeros(int(cap), dtype=SEARCH_DTYPE)
-        st = self.lib.glint_active_search(self.h, p.ctypes.data_as(ctypes.c_void_p), p.shape[0],
-                                          out.ctypes.data_as(ctypes.c_void_p) if cap else None, int(cap),
-                                          ctypes.byref(n))
-        if st != 0:
-            raise GlintError(st, self.last_error())
-        return out[: min(int(n.value), int(cap))]
+            if cap is not None or n.value <= room:
+                return out[: min(int(n.value), room)]
+            room = int(n.value)
 
     def precision_probe(self, stride: int = 256) -> dict:
         """The FP32 screen of the precision form against the reference's FP64

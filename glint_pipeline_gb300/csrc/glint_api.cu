@@ -187,7 +187,7 @@ void free_all(glint_ctx *c) {
                     c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
                     c->d_qstart, c->d_qlist, c->d_qslot, c->d_tcount, c->d_tstart, c->d_tlist, c->d_tab,
                     c->d_stamp, c->d_newline, c->d_new, c->d_rextra, c->d_tile_cnt, c->d_tile_off, c->d_log, c->d_cnt, c->d_coef,
-                    c->d_scan_tmp, c->d_scan_tmp_side, c->d_qbits, c->d_qpids, c->d_qout, c->d_qn};
+                    c->d_scan_tmp, c->d_scan_tmp_side, c->d_qbits, c->d_qpids, c->d_qout, c->d_qn, c->d_qfound};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     flush_free(c);
@@ -566,6 +566,7 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
         if (gstack[i] != i) gu = std::max({gu, i + 1, gstack[i] < G ? gstack[i] + 1 : G});
     hc.slots_used = su;
     hc.grids_used = gu;
+    hc.probe_span = 1;
     cudaMemcpy(c->d_cnt, &hc, sizeof(hc), cudaMemcpyHostToDevice);
     SinCoef coef;
     init_sin_coef(&coef);
@@ -683,6 +684,7 @@ static void launch_step(glint_ctx *c, const double *points, bool host) {
  * parameters the captured memcpy reads when the step runs */
 void begin_step(glint_ctx *c, uint32_t cur_time) {
     c->step_index++;
+    c->step_lists = true;
     c->last_time = cur_time;
     c->h_params->step_time = cur_time;
     c->h_params->step_tag = stamp_of(c->step_index);

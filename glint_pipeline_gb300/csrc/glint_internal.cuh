@@ -69,7 +69,8 @@ struct DevCounters {
      * were anything else (0: not known, the whole arrays are in use) */
     unsigned int slots_used;
     unsigned int grids_used;
-    unsigned int pad2;
+    unsigned int probe_span;               /* no entry of the table was ever placed this far past its home
+                                              slot (0: not known) */
     /* this step's parameters, copied in at the start of the step so that a
      * captured step graph reads them from here */
     unsigned int step_time;                /* cur_time */
@@ -263,6 +264,7 @@ struct glint_ctx {
     uint32_t *d_qpids = nullptr;
     glint_search_info *d_qout = nullptr;
     unsigned long long *d_qn = nullptr;
+    unsigned long long *d_qfound = nullptr;
     uint64_t qbits_cap = 0, qpids_cap = 0, qout_cap = 0;
 
     /* misc */
@@ -280,6 +282,7 @@ struct glint_ctx {
     glint::StepTimers timers;
     glint_step_stats last_stats;
     bool stats_valid = false;
+    bool step_lists = false;    /* the leaf and check lists are of the last step (not after a resume) */
 };
 
 namespace glint {

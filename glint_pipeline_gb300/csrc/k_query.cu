@@ -8,19 +8,33 @@
  * records (search_info_unit, tracing/workbench.h:85-88) with an atomic
  * counter; tracing/process.cpp:465-475 prints them after the step.
  *
- * Device form, run after a step against the table it left: the listed ids
+ * Device form, run after a step against the table it left, in bucket order,
+ * in two ways.
+ *
+ * By object (k_search_objects, k_search_sort), for lists that are short beside
+ * the table: an entry is active exactly when its pair was a contact of the
+ * last step, so the contacts of the listed objects are found again from the
+ * step's leaf and check lists, one warp per object, and their entries looked up
+ * (past slots that emptied since, as far as any entry was ever placed from
+ * its home slot); the entries found, at most kFoundMax, are put in bucket order
+ * by one block.
+ *
+ * By bucket (k_search_count, k_search_emit), for the rest: the listed ids
  * become a bitmap of N bits; pass 1 reads the stamp byte of every bucket and
  * the record of occupied buckets (its tag says whether the last step touched
- * it), and counts matching
- * sides per 8192-bucket tile; an exclusive scan gives each tile its offset;
- * pass 2 writes the records in bucket order.  The output order is therefore
- * deterministic.
+ * it), and counts matching sides per 8192-bucket tile; an exclusive scan gives
+ * each tile its offset; pass 2 writes the records of tiles that have any.  A
+ * warp lists the occupied buckets of its span first, so that its lanes all
+ * have a record to read.
+ *
+ * 256 objects of 2M, 2^27 buckets 6% full: a call took 423 us by bucket, each
+ * thread reading the records of 16 consecutive ones, and takes 64 us by object.
  */
 #include <algorithm>
 #include <cstring>
 #include <mutex>
 
-#include "glint_internal.cuh"
+#include "refine_common.cuh"
 
 namespace glint {
 
@@ -53,95 +67,251 @@ __device__ inline bool listed(const SearchArgs &a, uint32_t p) {
     return p < a.N && ((a.bits[p >> 5] >> (p & 31)) & 1u);
 }
 
-/* matching sides of bucket `slot` touched at the last step: bit 0 the lower
- * id, bit 1 the higher id */
-__device__ inline uint32_t search_sides(const SearchArgs &a, uint64_t slot, TRec &r) {
-    r = a.tab[slot];
-    if (r.w0 == kEmptyW0 || (r.w0 & kNewFlag) || rec_tag(r) != a.st) return 0;
-    if (a.cur_time - (uint32_t)r.w1 < a.min_plus1) return 0;
-    return (listed(a, pair_a(r.w0)) ? 1u : 0u) | (listed(a, pair_b(r.w0)) ? 2u : 0u);
+/* matching sides of a record (its words w0, w1) touched at the last step: bit
+ * 0 the lower id, bit 1 the higher id */
+__device__ inline uint32_t search_sides(const SearchArgs &a, const ulonglong2 &r) {
+    if (r.x == kEmptyW0 || (r.x & kNewFlag) || (uint32_t)(r.y >> 32) != a.st) return 0;
+    if (a.cur_time - (uint32_t)r.y < a.min_plus1) return 0;
+    return (listed(a, pair_a(r.x)) ? 1u : 0u) | (listed(a, pair_b(r.x)) ? 2u : 0u);
 }
 
-/* per thread: the sides mask of its 16 buckets, 2 bits each */
-__device__ inline uint32_t search_thread_masks(const SearchArgs &a, uint64_t base) {
-    uint32_t masks = 0;
-    if (base >= a.B) return 0;
-    const uint4 s4 = *reinterpret_cast<const uint4 *>(a.stamp + base); /* stamps padded to 16 */
-    const uint32_t w[4] = {s4.x, s4.y, s4.z, s4.w};
+constexpr int kSearchWarps = kSearchThreads / 32;
+constexpr uint32_t kSearchSpan = kSearchTile / kSearchWarps;
+constexpr int kSearchIlp = 4;
+
+/* warp-collective: the occupied buckets of the span from wbase on, in order,
+ * into list; returns their number */
+__device__ inline uint32_t list_occupied(const SearchArgs &a, uint64_t wbase, uint16_t *list) {
+    const int lane = threadIdx.x & 31;
+    uint32_t n = 0;
 #pragma unroll
-    for (int k = 0; k < kSearchItems; ++k) {
-        if ((uint8_t)(w[k >> 2] >> (8 * (k & 3))) != kStampOld || base + k >= a.B) continue;
-        TRec r;
-        masks |= search_sides(a, base + k, r) << (2 * k);
+    for (uint32_t i = 0; i < kSearchSpan / 512; ++i) {
+        /* 16 stamps per lane (the array is padded to whole tiles) */
+        const uint32_t off = i * 512 + lane * 16;
+        const uint4 v = *reinterpret_cast<const uint4 *>(a.stamp + wbase + off);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        uint32_t bits = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t m = __vcmpeq4(w[k], kStampOld * 0x01010101u) & 0x08040201u;
+            bits |= ((m | (m >> 8) | (m >> 16) | (m >> 24)) & 0xfu) << (4 * k);
+        }
+        uint32_t incl = __popc(bits);
+        const uint32_t mine = incl;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        uint32_t at = n + incl - mine;
+        n += __shfl_sync(0xffffffffu, incl, 31);
+        for (; bits; bits &= bits - 1) list[at++] = (uint16_t)(off + __ffs(bits) - 1);
     }
-    return masks;
+    __syncwarp();
+    return n;
 }
 
 __global__ void __launch_bounds__(kSearchThreads) k_search_count(SearchArgs a, uint32_t *__restrict__ tile_cnt) {
-    __shared__ uint32_t red[kSearchThreads / 32];
-    const uint64_t base = (uint64_t)blockIdx.x * kSearchTile + (uint64_t)threadIdx.x * kSearchItems;
-    uint32_t v = (uint32_t)__popc(search_thread_masks(a, base));
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    __shared__ uint32_t red[kSearchWarps];
+    __shared__ uint16_t list[kSearchWarps][kSearchSpan];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint64_t wbase = (uint64_t)blockIdx.x * kSearchTile + (uint64_t)wid * kSearchSpan;
+    const uint32_t n = list_occupied(a, wbase, list[wid]);
+    uint32_t v = 0;
+    for (uint32_t r0 = 0; r0 < n; r0 += 32 * kSearchIlp) {
+        ulonglong2 rec[kSearchIlp];
+#pragma unroll
+        for (int u = 0; u < kSearchIlp; ++u) {
+            const uint32_t i = r0 + u * 32 + lane;
+            rec[u] = make_ulonglong2(kEmptyW0, 0ull);
+            if (i < n) rec[u] = *reinterpret_cast<const ulonglong2 *>(&a.tab[wbase + list[wid][i]]);
+        }
+#pragma unroll
+        for (int u = 0; u < kSearchIlp; ++u) v += __popc(search_sides(a, rec[u]));
+    }
+    v = __reduce_add_sync(0xffffffffu, v);
     if (lane == 0) red[wid] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t t = 0;
-        for (int i = 0; i < kSearchThreads / 32; ++i) t += red[i];
+        for (int i = 0; i < kSearchWarps; ++i) t += red[i];
         tile_cnt[blockIdx.x] = t;
     }
+}
+
+/* the record of one side of an entry */
+__device__ inline glint_search_info search_record(const TRec &r, uint32_t side, uint32_t cur_time) {
+    const uint32_t pa = pair_a(r.w0), pb = pair_b(r.w0);
+    glint_search_info o;
+    o.pid = side ? pb : pa;
+    o.target = side ? pa : pb;
+    o.start = (uint32_t)r.w1;
+    o.end = cur_time;
+    for (int k = 0; k < 4; ++k) o.mbr[k] = fdec(r.mbr[k]);
+    return o;
 }
 
 __global__ void __launch_bounds__(kSearchThreads) k_search_emit(SearchArgs a, const uint32_t *__restrict__ tile_cnt,
                                                                 const uint32_t *__restrict__ tile_off,
                                                                 glint_search_info *__restrict__ out, uint64_t cap) {
     if (tile_cnt[blockIdx.x] == 0) return; /* uniform per block */
-    __shared__ uint32_t ws[kSearchThreads / 32];
-    const uint64_t base = (uint64_t)blockIdx.x * kSearchTile + (uint64_t)threadIdx.x * kSearchItems;
-    const uint32_t masks = search_thread_masks(a, base);
+    __shared__ uint32_t ws[kSearchWarps];
+    __shared__ uint16_t list[kSearchWarps][kSearchSpan];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t v = (uint32_t)__popc(masks);
-    uint32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) ws[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        uint32_t s = lane < kSearchThreads / 32 ? ws[lane] : 0u;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += y;
-        }
-        if (lane < kSearchThreads / 32) ws[lane] = s;
-    }
-    __syncthreads();
-    if (!masks) return;
-    uint64_t pos = (uint64_t)tile_off[blockIdx.x] + (wid ? ws[wid - 1] : 0u) + x - v;
-    for (int k = 0; k < kSearchItems; ++k) {
-        const uint32_t m = (masks >> (2 * k)) & 3u;
-        if (!m) continue;
-        const TRec r = a.tab[base + k];
-        const uint32_t pa = pair_a(r.w0), pb = pair_b(r.w0);
-        const uint4 mb = *reinterpret_cast<const uint4 *>(r.mbr);
-        for (int side = 0; side < 2; ++side) {
-            if (!(m & (1u << side))) continue;
-            if (pos < cap) {
-                glint_search_info o;
-                o.pid = side ? pb : pa;
-                o.target = side ? pa : pb;
-                o.start = (uint32_t)r.w1;
-                o.end = a.cur_time;
-                o.mbr[0] = fdec(mb.x);
-                o.mbr[1] = fdec(mb.y);
-                o.mbr[2] = fdec(mb.z);
-                o.mbr[3] = fdec(mb.w);
-                out[pos] = o;
+    const uint64_t wbase = (uint64_t)blockIdx.x * kSearchTile + (uint64_t)wid * kSearchSpan;
+    const uint32_t n = list_occupied(a, wbase, list[wid]);
+    uint64_t pos = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        uint32_t v = 0;
+        for (uint32_t r0 = 0; r0 < n; r0 += 32) {
+            const uint32_t i = r0 + lane;
+            ulonglong2 rec = make_ulonglong2(kEmptyW0, 0ull);
+            if (i < n) rec = *reinterpret_cast<const ulonglong2 *>(&a.tab[wbase + list[wid][i]]);
+            const uint32_t m = search_sides(a, rec);
+            if (pass == 0) {
+                v += __popc(m);
+                continue;
             }
-            ++pos;
+            uint32_t incl = __popc(m);
+            const uint32_t mine = incl;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            uint64_t at = pos + incl - mine;
+            pos += __shfl_sync(0xffffffffu, incl, 31);
+            if (!m) continue;
+            const TRec r = a.tab[wbase + list[wid][i]];
+            for (uint32_t side = 0; side < 2; ++side) {
+                if (!(m & (1u << side))) continue;
+                if (at < cap) out[at] = search_record(r, side, a.cur_time);
+                ++at;
+            }
+        }
+        if (pass == 1) break;
+        v = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0) ws[wid] = v;
+        __syncthreads();
+        pos = tile_off[blockIdx.x];
+        for (int w = 0; w < wid; ++w) pos += ws[w];
+    }
+}
+
+/* ---- by object ------------------------------------------------------------ */
+constexpr uint32_t kFoundMax = 4096;
+
+struct ObjectSearch {
+    RefineArgs r;              /* the step's lists and the table (leaf counts from the segment starts: the
+                                  schema update clears those of grids it frees) */
+    SearchArgs s;
+    unsigned long long *found; /* [kFoundMax] bucket * 2 + side */
+    unsigned int *n_found;
+};
+
+/* p1 the checking object, p2 the member, as leaf-major ranks */
+__device__ inline bool within_reach(const RefineArgs &a, uint32_t r1, uint32_t r2) {
+    const longlong2 A = a.sipos[r1], B = a.sipos[r2];
+    const Screen sc = make_screen(__fmaf_rn(0.0f, a.sc[r2], a.sc[r1]), a.f);
+    const int in = fx_screen(A.x - B.x, A.y - B.y, sc, a.f.cy);
+    return in < 0 ? pair_exact(a.sxy, r1, r2, a.ex) : in != 0;
+}
+
+/* the listed object p meets m: its entry, if it has lasted long enough */
+__device__ inline void found_contact(const ObjectSearch &o, uint32_t p, uint32_t m) {
+    const unsigned long long pw = pw_of(p, m);
+    uint64_t slot = home_slot(o.r, pw);
+    const uint32_t span = o.r.cnt->probe_span;
+    for (uint32_t d = 0; d < span; ++d) {
+        const ulonglong2 k = *reinterpret_cast<const ulonglong2 *>(&o.r.tab[slot]);
+        if (k.x == pw) {
+            if ((uint32_t)(k.y >> 32) != o.s.st || o.s.cur_time - (uint32_t)k.y < o.s.min_plus1) return;
+            const uint32_t i = atomicAdd(o.n_found, 1u);
+            if (i < kFoundMax) o.found[i] = slot * 2 + (pair_a(pw) == p ? 0u : 1u);
+            return;
+        }
+        slot = slot + 1 == o.r.B ? 0 : slot + 1;
+    }
+}
+
+/* one warp per listed object: its own leaf's members, the members of the
+ * leaves it checks, and the objects that check its leaf (a contact found from
+ * both sides, or an object listed twice, is found twice) */
+__global__ void __launch_bounds__(128) k_search_objects(ObjectSearch o, const uint32_t *__restrict__ pids,
+                                                        uint32_t npids) {
+    const RefineArgs &a = o.r;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 32; i < npids; i += gridDim.x * blockDim.x / 32) {
+        const uint32_t p = pids[i];
+        if (p >= o.s.N) continue;
+        const uint32_t r = a.rank_of[p], g = a.obj_gid[p];
+        const uint32_t s0 = a.grid_start[g], k = min(a.grid_start[g + 1] - s0, a.cap);
+        const bool stored = r - s0 < k;
+        for (uint32_t j = lane; stored && j < k; j += 32) {
+            const uint32_t m = s0 + j;
+            if (m != r && within_reach(a, min(r, m), max(r, m))) found_contact(o, p, a.sorted[m]);
+        }
+        const uint32_t nq = a.qcount[p], q0 = a.qstart[p];
+        for (uint32_t q = 0; q < nq; ++q) {
+            const uint32_t h = a.qlist[q0 + q];
+            const uint32_t h0 = a.grid_start[h], hk = min(a.grid_start[h + 1] - h0, a.cap);
+            for (uint32_t j = lane; j < hk; j += 32)
+                if (within_reach(a, r, h0 + j)) found_contact(o, p, a.sorted[h0 + j]);
+        }
+        const uint32_t tb = a.tstart[g], te = a.tstart[g + 1];
+        for (uint32_t t = tb + lane; stored && t < te; t += 32) {
+            const uint32_t q = a.tlist[t].x;
+            if (within_reach(a, a.rank_of[q], r)) found_contact(o, p, q);
         }
     }
+}
+
+/* one block: the entries found, in bucket order and each once; n = their
+ * number, or all ones when there were more than kFoundMax */
+__global__ void __launch_bounds__(1024) k_search_sort(ObjectSearch o, glint_search_info *__restrict__ out,
+                                                      uint64_t cap, unsigned long long *n) {
+    __shared__ unsigned long long key[kFoundMax];
+    __shared__ uint32_t ws[32];
+    const uint32_t found = *o.n_found;
+    if (found > kFoundMax) {
+        if (threadIdx.x == 0) *n = ~0ull;
+        return;
+    }
+    uint32_t P = 32;
+    while (P < found) P <<= 1;
+    for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) key[i] = i < found ? o.found[i] : ~0ull;
+    __syncthreads();
+    for (uint32_t k = 2; k <= P; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
+                const uint32_t l = i ^ j;
+                if (l > i) {
+                    const unsigned long long x = key[i], y = key[l];
+                    if ((x > y) == ((i & k) == 0)) {
+                        key[i] = y;
+                        key[l] = x;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t before = 0;
+    for (uint32_t base = 0; base < found; base += blockDim.x) {
+        const uint32_t i = base + threadIdx.x;
+        const bool mine = i < found && (i == 0 || key[i] != key[i - 1]);
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+        if (lane == 0) ws[wid] = __popc(m);
+        __syncthreads();
+        uint32_t at = before, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w < wid) at += ws[w];
+            all += ws[w];
+        }
+        at += __popc(m & ((1u << lane) - 1u));
+        if (mine && at < cap) out[at] = search_record(o.r.tab[key[i] >> 1], (uint32_t)(key[i] & 1), o.s.cur_time);
+        before += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *n = before;
 }
 
 __global__ void k_search_total(const uint32_t *__restrict__ tile_off, uint64_t tiles, unsigned long long *n) {
@@ -176,7 +346,7 @@ cudaError_t launch_active_search(const glint_ctx *c, uint32_t *bits, uint32_t *t
     const SearchArgs a = search_args(c, bits);
     k_search_count<<<(unsigned)tiles, kSearchThreads, 0, s>>>(a, tile_cnt);
     if ((e = scan(tile_cnt, tile_off, tiles, s)) != cudaSuccess) return e;
-    k_search_emit<<<(unsigned)tiles, kSearchThreads, 0, s>>>(a, tile_cnt, tile_off, d_out, cap);
+    if (cap) k_search_emit<<<(unsigned)tiles, kSearchThreads, 0, s>>>(a, tile_cnt, tile_off, d_out, cap);
     k_search_total<<<1, 1, 0, s>>>(tile_off, tiles, d_n);
     return cudaGetLastError();
 }
@@ -198,6 +368,37 @@ cudaError_t grow(T **p, uint64_t &have, uint64_t need) {
     return e;
 }
 
+/* Which way: an object costs its contacts and their entries, a bucket its
+ * stamp and, where occupied, its record.  The two meet at about B / 2000
+ * objects (2^23 buckets, 200k objects: 4000 by object 76 us a call, 8000 by
+ * bucket 71 us), and beyond 2048 objects the entries tend to be more than one
+ * block orders (2^27 buckets, 2M objects: 2000 by object 102 us; 4000, found to
+ * be too many and then read by bucket, 339 us).  Entries far from their home
+ * slots (a table near its capacity) make each look long: past 1024 slots the
+ * buckets are read. */
+bool search_by_object(const glint_ctx *c, uint32_t npids) {
+    const uint32_t span = c->h_cnt->probe_span;
+    return c->step_lists && npids && npids <= 2048 && (uint64_t)npids * 2000 < c->B && span && span <= 1024;
+}
+
+cudaError_t launch_object_search(glint_ctx *c, uint32_t npids, uint64_t cap) {
+    cudaStream_t s = c->stream;
+    cudaError_t e = cudaSuccess;
+    if (!c->d_qfound) e = cudaMalloc((void **)&c->d_qfound, sizeof(unsigned long long) * (kFoundMax + 1));
+    if (e != cudaSuccess) return e;
+    ObjectSearch o;
+    o.r = refine_args(c);
+    o.r.ex.ambiguous = nullptr; /* the step's counters stay the step's */
+    o.r.ex.rechecks = nullptr;
+    o.s = search_args(c, nullptr);
+    o.found = c->d_qfound;
+    o.n_found = reinterpret_cast<unsigned int *>(c->d_qfound + kFoundMax);
+    if ((e = cudaMemsetAsync(o.n_found, 0, sizeof(unsigned int), s)) != cudaSuccess) return e;
+    k_search_objects<<<grid_for(npids, 4, 152u * 16u), 128, 0, s>>>(o, c->d_qpids, npids);
+    k_search_sort<<<1, 1024, 0, s>>>(o, c->d_qout, cap, c->d_qn);
+    return cudaGetLastError();
+}
+
 } // namespace
 
 extern "C" glint_status glint_active_search(glint_ctx *c, const uint32_t *pids, uint32_t npids, glint_search_info *out,
@@ -217,18 +418,26 @@ extern "C" glint_status glint_active_search(glint_ctx *c, const uint32_t *pids, 
     if (e == cudaSuccess && !c->d_qn) e = cudaMalloc((void **)&c->d_qn, sizeof(unsigned long long));
     if (e == cudaSuccess && npids)
         e = cudaMemcpyAsync(c->d_qpids, pids, sizeof(uint32_t) * npids, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) {
+    unsigned long long found = ~0ull;
+    auto fetch = [&]() {
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&found, c->d_qn, sizeof(found), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    };
+    if (e == cudaSuccess && search_by_object(c, npids)) {
+        e = launch_object_search(c, npids, cap);
+        fetch();
+    }
+    /* by bucket, also when more entries were found than one block orders */
+    if (e == cudaSuccess && found == ~0ull) {
         void *tmp = c->d_scan_tmp;
         auto scan = [tmp](const uint32_t *in, uint32_t *o, uint64_t m, cudaStream_t s) {
             return scan_u32(in, o, m, tmp, s);
         };
         e = launch_active_search(c, c->d_qbits, c->d_tile_cnt, c->d_tile_off, scan, c->d_qpids, npids, c->d_qout, cap,
                                  c->d_qn);
+        fetch();
     }
-    unsigned long long found = 0;
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&found, c->d_qn, sizeof(found), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e == cudaSuccess && found && cap)
         e = cudaMemcpy(out, c->d_qout, sizeof(glint_search_info) * std::min<uint64_t>(found, cap),
                        cudaMemcpyDeviceToHost);

@@ -159,10 +159,15 @@ __global__ void __launch_bounds__(256) k_insert(const NewEntry *__restrict__ lis
     const unsigned long long n0 = cnt->new_keys;
     const unsigned long long n = n0 < new_cap ? n0 : new_cap;
     const uint8_t st = (uint8_t)cnt->step_tag;
+    uint64_t span = 0; /* the farthest placement from a home slot, + 1 */
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         ulonglong2 cur = make_ulonglong2(list[i].key | kNewFlag, list[i].prio);
-        uint64_t slot = fastmod(cantor(pair_a(cur.x), pair_b(cur.x)), B, Bm);
+        uint64_t slot = fastmod(cantor(pair_a(cur.x), pair_b(cur.x)), B, Bm), home = slot;
+        auto placed = [&]() {
+            const uint64_t d = (slot >= home ? slot - home : slot + B - home) + 1;
+            span = d > span ? d : span;
+        };
         bool done = false;
         /* empty records hold (kEmptyW0, 0), so the first compare-and-swap at a
          * bucket doubles as its read */
@@ -179,6 +184,7 @@ __global__ void __launch_bounds__(256) k_insert(const NewEntry *__restrict__ lis
                 if (seen.x == kEmptyW0) {
                     ulonglong2 prev = cas128(&tab[slot], seen, cur);
                     if (u128_eq(prev, seen)) {
+                        placed();
                         atomicOr(&newline[slot >> 7], 1u << ((slot >> 2) & 31));
                         done = true;
                         break;
@@ -202,7 +208,9 @@ __global__ void __launch_bounds__(256) k_insert(const NewEntry *__restrict__ lis
                 if ((seen.x & kNewFlag) && seen.y > cur.y) {
                     ulonglong2 prev = cas128(&tab[slot], seen, cur);
                     if (u128_eq(prev, seen)) {
+                        placed();
                         cur = seen; /* the displaced pair walks on */
+                        home = fastmod(cantor(pair_a(cur.x), pair_b(cur.x)), B, Bm);
                         break;
                     }
                     seen = prev;
@@ -214,6 +222,9 @@ __global__ void __launch_bounds__(256) k_insert(const NewEntry *__restrict__ lis
         }
         if (!done) atomicOr(&cnt->error_flags, GLINT_EF_TABLE_FULL);
     }
+    /* a high-water mark: after the first steps hardly any placement passes it */
+    if (span > cnt->probe_span && cnt->probe_span)
+        atomicMax(&cnt->probe_span, (unsigned int)(span < 0xffffffffull ? span : 0xffffffffull));
 }
 
 cudaError_t launch_insert(glint_ctx *c, uint32_t cur_time) {

@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(64) k_step_tail(uint32_t N, const uint32_t *re
 }
 
 void free_all(glint_ctx *c) {
-    void *ptrs[] = {c->d_pts, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj_gid, c->d_obj_lv, c->d_obj_leaf, c->d_obj_pos, c->d_grid_count,
-                    c->d_grid_start, c->d_sorted, c->d_rank_of, c->d_sxy, c->d_sm, c->d_leaf_work,
+    void *ptrs[] = {c->d_pts, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj, c->d_grid_count,
+                    c->d_grid_start, c->d_sorted, c->d_rank, c->d_sxy, c->d_sm, c->d_leaf_work,
                     c->d_nodes, c->d_low, c->d_sstack, c->d_gstack, c->d_split, c->d_evscan, c->d_cand, c->d_newgid,
                     c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
                     c->d_qstart, c->d_qlist, c->d_qslot, c->d_tcount, c->d_tstart, c->d_tlist, c->d_tab,
@@ -414,14 +414,11 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     ALLOC(c->d_sfpos, N);
     ALLOC(c->d_sc, N);
     ALLOC(c->d_fpos, N);
-    ALLOC(c->d_obj_gid, N);
-    ALLOC(c->d_obj_lv, N);
-    ALLOC(c->d_obj_leaf, N);
-    ALLOC(c->d_obj_pos, N);
+    ALLOC(c->d_obj, N);
     ALLOC(c->d_grid_count, (size_t)G + 1);
     ALLOC(c->d_grid_start, (size_t)G + 1);
     ALLOC(c->d_sorted, N);
-    ALLOC(c->d_rank_of, N);
+    ALLOC(c->d_rank, N);
     ALLOC(c->d_sxy, N);
     ALLOC(c->d_sm, N);
     ALLOC(c->d_leaf_work, G);
@@ -637,13 +634,18 @@ void launch_step_front(glint_ctx *c, const double *points, bool host) {
     const bool tm = c->cfg.timing != 0 && !c->cfg.use_graph;
     launch_step_begin(c);
     if (tm) cudaEventRecord(c->timers.ev[0], s);
+    /* points in device memory on a 16-byte boundary are read in place (a copy
+     * of theirs was 10 us of a 1M-object step's 700) */
+    const double2 *pts = c->d_pts;
     if (host) {
         cudaMemcpyAsync(c->d_pts, points, sizeof(double2) * c->N, cudaMemcpyHostToDevice, s);
-    } else if ((const void *)points != (const void *)c->d_pts) {
+    } else if (c->input_device && ((uintptr_t)points & 15) == 0) {
+        pts = reinterpret_cast<const double2 *>(points);
+    } else {
         cudaMemcpyAsync(c->d_pts, points, sizeof(double2) * c->N, cudaMemcpyDeviceToDevice, s);
     }
     if (tm) cudaEventRecord(c->timers.ev[1], s);
-    launch_partition(c, 0);
+    launch_partition(c, pts);
     if (tm) cudaEventRecord(c->timers.ev[2], s);
     launch_filter(c);
     if (tm) cudaEventRecord(c->timers.ev[3], s);
@@ -705,6 +707,7 @@ bool device_points(glint_ctx *c, const void *p) {
         c->last_error = "step input: not device memory";
         return false;
     }
+    c->input_device = at.type == cudaMemoryTypeDevice;
     return true;
 }
 
@@ -769,7 +772,7 @@ static void fill_stats(glint_ctx *c, glint_step_stats *st) {
     st->box_band = h.box_band;
     st->error_flags = h.error_flags;
     /* kernels per step: begin 1, partition 5, filter 3, refine 1, insert 1,
-     * identify 3 + keys 1, schema update 4, tail 1 */
+     * identify 3 (2 for small tables) + keys 1, schema update 4, tail 1 */
     st->launches = 1 + 5 + 3 + 1 + 1 + 4 + (c->cfg.dynamic_schema ? 4 : 0) + 1;
     st->meeting_log_size = h.log_head;
     st->kv_count = h.kv_count;
@@ -937,6 +940,7 @@ namespace glint {
 /* the step on device points, never through the captured graph (whose input
  * buffer is fixed) */
 glint_status enqueue_device_step_plain(glint_ctx *c, const double *d_points, uint32_t cur_time) {
+    c->input_device = true; /* the pipe's own buffers */
     return enqueue_step(c, d_points, false, cur_time, false);
 }
 } // namespace glint

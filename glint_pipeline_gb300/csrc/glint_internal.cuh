@@ -4,7 +4,7 @@
  *
  * HBM layout (N objects, G grid slots, S schema slots, B buckets):
  *   points      double2[N]   lon/lat as given, AoS 16 B per object
- *   obj_*       u32[N]       leaf grid id, last_valid node, leaf node per object
+ *   obj         uint4[N]     leaf grid id, last_valid node, leaf node, place in the leaf, per object
  *   sorted      u32[N]       object ids sorted by (grid id, object id): leaf member lists
  *   sxy         double2[N]   coordinates gathered in that order (leaf tiles)
  *   sipos, sc   [N]          fixed-point coordinates (i64 pair) and screening scale, same order
@@ -83,6 +83,9 @@ struct StepParams {
 };
 /* bytes cleared at the start of every step */
 constexpr size_t kStepCounterBytes = offsetof(DevCounters, ssi);
+
+/* a rank's mark: the object is past its leaf's buffer, which drops it */
+constexpr uint32_t kDropped = 0x80000000u;
 
 /* cross-leaf checks per refine work item (refine_common.cuh) */
 constexpr uint32_t kCrossChunk = 64;       /* default cross-leaf checks per refine work item */
@@ -174,13 +177,15 @@ struct glint_ctx {
     uint32_t last_time = 0;
 
     /* objects */
-    double2 *d_pts = nullptr;
-    uint32_t *d_obj_gid = nullptr, *d_obj_lv = nullptr, *d_obj_leaf = nullptr;
+    double2 *d_pts = nullptr;              /* [N] the step's points, where they are not read in place */
+    uint4 *d_obj = nullptr;                /* [N] each object's leaf grid, last_valid node, leaf node and place in
+                                              its leaf's segment */
+    bool input_device = false;             /* the step's input is device (not managed) memory */
     uint32_t *d_grid_count = nullptr;      /* [G+1] */
     uint32_t *d_grid_start = nullptr;      /* [G+1] */
-    uint32_t *d_obj_pos = nullptr;         /* [N] each object's place in its leaf's segment */
     uint32_t *d_sorted = nullptr;          /* [N] leaf-major order; the next descent's processing order */
-    uint32_t *d_rank_of = nullptr;         /* [N] sorted position of each object */
+    uint2 *d_rank = nullptr;               /* [N] sorted position of each object (kDropped: past its leaf's
+                                              buffer), its leaf node */
     double2 *d_sxy = nullptr;
     double *d_sm = nullptr;                /* [N] sorted metres per degree of longitude (plain form only) */
     longlong2 *d_sipos = nullptr;          /* [N] sorted fixed-point coordinates */
@@ -297,7 +302,7 @@ void init_sin_coef(SinCoef *host);
 
 /* ---- stages ---- */
 cudaError_t launch_step_begin(glint_ctx *c);
-cudaError_t launch_partition(glint_ctx *c, uint32_t cur_time);
+cudaError_t launch_partition(glint_ctx *c, const double2 *pts);
 cudaError_t launch_filter(glint_ctx *c);
 cudaError_t launch_refine_pairs(glint_ctx *c);
 struct RefineArgs;

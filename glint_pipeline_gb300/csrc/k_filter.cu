@@ -41,7 +41,6 @@ constexpr uint32_t kKeptLeaf = 0x80000000u;
  * exact fallback), fixed-point coordinates and screening limits */
 struct WalkPoint {
     double px, py;
-    uint64_t kx, ky;     /* dkey(px), dkey(py) */
     long long X, Y;
     Screen sc;
 };
@@ -50,8 +49,6 @@ __device__ inline WalkPoint walk_point(const double2 p, const longlong2 ip, floa
     WalkPoint w;
     w.px = p.x;
     w.py = p.y;
-    w.kx = dkey(p.x);
-    w.ky = dkey(p.y);
     w.X = ip.x;
     w.Y = ip.y;
     w.sc = make_screen(c, f);
@@ -65,78 +62,20 @@ __device__ __noinline__ bool box_exact(double lx, double ly, double hx, double h
     return box_le_exact(lx, ly, hx, hy, px, py, dpm_lon_fast(py), ex);
 }
 
-/* lookup_rec from node `start`; calls emit(gid, ordinal) in walk order;
- * returns the number of leaves kept.  The box test is screened on the
- * fixed-point boxes; only a box within the guard band of the reach takes the
- * reference's FP64 box distance.  The top/right rule is decided on the
- * fixed-point coordinates where they are more than a unit apart, else on the
- * doubles' keys. */
-template <class Emit>
-__device__ inline uint32_t lookup_walk(const DNode *__restrict__ nodes, const double2 *__restrict__ low,
-                                       const IBox *__restrict__ ibox, uint32_t start, const WalkPoint &w,
-                                       const Frame &f, const ExactCtx &ex, DevCounters *cnt, Emit emit) {
+/* lookup_rec's walk of one object: the nodes and kept leaves still to visit,
+ * in reverse order of the reference's depth-first walk */
+struct Walk {
     uint32_t stack[kStackMax];
-    int sp = 1;
-    stack[0] = start;
-    uint32_t kept = 0;
-    while (sp > 0) {
-        const uint32_t top = stack[--sp];
-        if (top & kKeptLeaf) {
-            emit(top & ~kKeptLeaf, kept);
-            ++kept;
-            continue;
-        }
-        const uint4 chv = *reinterpret_cast<const uint4 *>(nodes[top].child);
-        const uint32_t ch[4] = {chv.x, chv.y, chv.z, chv.w};
-        IBox box[4];
-        uint2 tail[4]; /* gid; type, level */
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            box[i] = ibox[ch[i]];
-            tail[i] = *reinterpret_cast<const uint2 *>(&nodes[ch[i]].gid);
-        }
-#pragma unroll
-        for (int i = 3; i >= 0; --i) {
-            const uint32_t type = tail[i].y & 0xffu;
-            /* nothing at or above the object's latitude */
-            if (box[i].w < w.Y - 1 && (type == kLeaf || type == kBranch)) continue;
-            int in = fx_box_screen(box[i], w.X, w.Y, w.sc, f.cy);
-            if (in < 0) {
-                atomicAdd(&cnt->box_band, 1u);
-                const double2 lo = low[ch[i]];
-                in = box_exact(lo.x, lo.y, kdbl(nodes[ch[i]].khx), kdbl(nodes[ch[i]].khy), w.px, w.py, ex) ? 1 : 0;
-            }
-            if (!in) continue;
-            if (type == kLeaf) {
-                bool keep;
-                if (w.Y < box[i].y - 1) {
-                    keep = true;
-                } else if (w.Y > box[i].y + 1 && w.Y < box[i].w - 1 && (w.X < box[i].x - 1 || w.X > box[i].x + 1)) {
-                    keep = w.X < box[i].x;
-                } else {
-                    const double2 lo = low[ch[i]];
-                    keep = w.ky < dkey(lo.y) || (w.ky < nodes[ch[i]].khy && w.kx < dkey(lo.x));
-                }
-                if (!keep) continue;
-                if (sp < kStackMax) stack[sp++] = tail[i].x | kKeptLeaf;
-                else atomicOr(&cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
-            } else if (type == kBranch && sp < kStackMax) {
-                stack[sp++] = ch[i];
-            } else {
-                atomicOr(&cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
-            }
-        }
-    }
-    return kept;
-}
+    int sp = 0;
+    uint32_t kept = 0; /* leaves kept so far */
+};
 
 struct FilterArgs {
     const uint32_t *sorted;
     const double2 *sxy;
     const longlong2 *sipos;
     const float *sc;
-    const uint32_t *obj_lv;
-    const uint32_t *obj_leaf;
+    const uint4 *obj;
     const DNode *nodes;
     const double2 *low;
     const IBox *ibox;
@@ -146,10 +85,66 @@ struct FilterArgs {
     DevCounters *cnt;
 };
 
+/* One step of a walk: the node on top is opened, or the kept leaf on top is
+ * given to emit(gid, ordinal).  The box test is screened on the fixed-point
+ * boxes; only a box within the guard band of the reach takes the reference's
+ * FP64 box distance.  The top/right rule is decided on the fixed-point
+ * coordinates where they are more than a unit apart, else on the doubles'
+ * keys. */
+template <class Emit>
+__device__ inline void walk_step(const FilterArgs &a, Walk &k, const WalkPoint &w, Emit emit) {
+    const uint32_t top = k.stack[--k.sp];
+    if (top & kKeptLeaf) {
+        emit(top & ~kKeptLeaf, k.kept);
+        ++k.kept;
+        return;
+    }
+    const uint4 chv = *reinterpret_cast<const uint4 *>(a.nodes[top].child);
+    const uint32_t ch[4] = {chv.x, chv.y, chv.z, chv.w};
+    IBox box[4];
+    uint2 tail[4]; /* gid; type, level */
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        box[i] = a.ibox[ch[i]];
+        tail[i] = *reinterpret_cast<const uint2 *>(&a.nodes[ch[i]].gid);
+    }
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+        const uint32_t type = tail[i].y & 0xffu;
+        /* nothing at or above the object's latitude */
+        if (box[i].w < w.Y - 1 && (type == kLeaf || type == kBranch)) continue;
+        int in = fx_box_screen(box[i], w.X, w.Y, w.sc, a.f.cy);
+        if (in < 0) {
+            atomicAdd(&a.cnt->box_band, 1u);
+            const double2 lo = a.low[ch[i]];
+            in = box_exact(lo.x, lo.y, kdbl(a.nodes[ch[i]].khx), kdbl(a.nodes[ch[i]].khy), w.px, w.py, a.ex) ? 1 : 0;
+        }
+        if (!in) continue;
+        if (type == kLeaf) {
+            bool keep;
+            if (w.Y < box[i].y - 1) {
+                keep = true;
+            } else if (w.Y > box[i].y + 1 && w.Y < box[i].w - 1 && (w.X < box[i].x - 1 || w.X > box[i].x + 1)) {
+                keep = w.X < box[i].x;
+            } else {
+                const double2 lo = a.low[ch[i]];
+                keep = dkey(w.py) < dkey(lo.y) || (dkey(w.py) < a.nodes[ch[i]].khy && dkey(w.px) < dkey(lo.x));
+            }
+            if (!keep) continue;
+            if (k.sp < kStackMax) k.stack[k.sp++] = tail[i].x | kKeptLeaf;
+            else atomicOr(&a.cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
+        } else if (type == kBranch && k.sp < kStackMax) {
+            k.stack[k.sp++] = ch[i];
+        } else {
+            atomicOr(&a.cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
+        }
+    }
+}
+
 /* Only border objects (a leaf beside their own in reach) walk the tree:
- * about half of them at 10M objects.  Each warp reads 32 consecutive ranks
- * at a time, queues its border objects in shared memory, and walks them 32 at
- * a time, so that every lane of a walk has an object. */
+ * about half of them at 10M objects, a fifth at 1M.  Each warp reads 32
+ * consecutive ranks at a time, queues its border objects in shared memory and
+ * walks them 32 at a time, so that every lane of a walk has an object. */
 constexpr int kWalkWarps = 4;
 
 struct CheckLists {
@@ -163,73 +158,81 @@ struct CheckLists {
 __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, CheckLists l) {
     __shared__ uint32_t sbuf[kWalkWarps][64];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t below = (1u << lane) - 1u;
     const uint32_t stride = gridDim.x * kWalkWarps * 32;
+    uint32_t base = (blockIdx.x * kWalkWarps + wid) * 32;
     uint32_t nb = 0, nborder = 0;
-    for (uint32_t base = (blockIdx.x * kWalkWarps + wid) * 32;; base += stride) {
-        const bool more = base < a.N;
-        if (more) {
+    for (;;) {
+        while (nb < 32 && base < a.N) {
             const uint32_t i = base + lane;
             bool border = false;
             if (i < a.N) {
-                const uint32_t pid = a.sorted[i];
-                border = a.obj_lv[pid] != a.obj_leaf[pid];
-                if (!border) l.qcount[pid] = 0;
+                const uint32_t p = a.sorted[i];
+                const uint4 o = a.obj[p];
+                border = o.y != o.z;
+                if (!border) l.qcount[p] = 0;
             }
             const unsigned m = __ballot_sync(0xffffffffu, border);
-            if (border) sbuf[wid][nb + __popc(m & ((1u << lane) - 1u))] = i;
+            if (border) sbuf[wid][nb + __popc(m & below)] = i;
             nb += __popc(m);
             nborder += __popc(m);
+            base += stride;
             __syncwarp();
         }
-        if (nb >= 32 || (!more && nb > 0)) {
-            const uint32_t take = nb < 32 ? nb : 32;
-            uint32_t pid = 0, n = 0, lv = 0, row[kQInline];
-            WalkPoint w;
-            if ((uint32_t)lane < take) {
-                const uint32_t i = sbuf[wid][lane];
-                pid = a.sorted[i];
-                lv = a.obj_lv[pid];
-                w = walk_point(a.sxy[i], a.sipos[i], a.sc[i], a.f);
-                n = lookup_walk(a.nodes, a.low, a.ibox, lv, w, a.f, a.ex, a.cnt, [&](uint32_t gid, uint32_t k) {
-                    if (k < kQInline) row[k] = gid;
+        if (nb == 0) break;
+        /* the queue's last objects */
+        const uint32_t take = nb < 32 ? nb : 32;
+        const bool mine = (uint32_t)lane < take;
+        uint32_t pid = 0, lv = 0, row[kQInline];
+        Walk k;
+        WalkPoint w;
+        if (mine) {
+            const uint32_t i = sbuf[wid][nb - take + lane];
+            pid = a.sorted[i];
+            lv = a.obj[pid].y;
+            w = walk_point(a.sxy[i], a.sipos[i], a.sc[i], a.f);
+            k.sp = 1;
+            k.stack[0] = lv;
+            while (k.sp > 0)
+                walk_step(a, k, w, [&](uint32_t gid, uint32_t j) {
+                    if (j < (uint32_t)kQInline) row[j] = gid;
                 });
+        }
+        nb -= take;
+        __syncwarp();
+        /* the warp's checks take one run of the list */
+        uint32_t n = k.kept, incl = n;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        uint32_t at = 0;
+        if (lane == 31 && incl) at = atomicAdd(&a.cnt->cross_checks, incl);
+        at = __shfl_sync(0xffffffffu, at, 31) + incl - n;
+        if (mine) {
+            if ((uint64_t)at + n > l.cap) {
+                atomicOr(&a.cnt->error_flags, GLINT_EF_CHECKS_OVERFLOW);
+                n = 0;
             }
-            __syncwarp();
-            /* the warp's checks take one run of the list */
-            uint32_t incl = n;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            uint32_t at = 0;
-            if (lane == 31 && incl) at = atomicAdd(&a.cnt->cross_checks, incl);
-            at = __shfl_sync(0xffffffffu, at, 31) + incl - n;
-            if ((uint32_t)lane < take) {
-                if ((uint64_t)at + n > l.cap) {
-                    atomicOr(&a.cnt->error_flags, GLINT_EF_CHECKS_OVERFLOW);
-                    n = 0;
-                }
-                l.qstart[pid] = at;
-                l.qcount[pid] = n;
-                auto put = [&](uint32_t gid, uint32_t k) {
-                    l.qlist[at + k] = gid;
-                    l.qslot[at + k] = atomicAdd(&l.tcount[gid], 1u);
-                };
-                for (uint32_t k = 0; k < n && k < (uint32_t)kQInline; ++k) put(row[k], k);
-                if (n > (uint32_t)kQInline)
-                    lookup_walk(a.nodes, a.low, a.ibox, lv, w, a.f, a.ex, a.cnt, [&](uint32_t gid, uint32_t k) {
-                        if (k >= (uint32_t)kQInline && k < n) put(gid, k);
+            l.qstart[pid] = at;
+            l.qcount[pid] = n;
+            auto put = [&](uint32_t gid, uint32_t j) {
+                l.qlist[at + j] = gid;
+                l.qslot[at + j] = atomicAdd(&l.tcount[gid], 1u);
+            };
+            for (uint32_t j = 0; j < n && j < (uint32_t)kQInline; ++j) put(row[j], j);
+            if (n > (uint32_t)kQInline) {
+                /* the rare object with more: walked again for the rest */
+                k.sp = 1;
+                k.kept = 0;
+                k.stack[0] = lv;
+                while (k.sp > 0)
+                    walk_step(a, k, w, [&](uint32_t gid, uint32_t j) {
+                        if (j >= (uint32_t)kQInline && j < n) put(gid, j);
                     });
             }
-            const uint32_t rest = nb - take;
-            __syncwarp();
-            const uint32_t v = (uint32_t)lane < rest ? sbuf[wid][32 + lane] : 0u;
-            __syncwarp();
-            if ((uint32_t)lane < rest) sbuf[wid][lane] = v;
-            __syncwarp();
-            nb = rest;
         }
-        if (!more && nb == 0) break;
+        __syncwarp();
     }
     if (lane == 0 && nborder) atomicAdd(&a.cnt->border_objects, nborder);
 }
@@ -279,8 +282,7 @@ cudaError_t launch_filter(glint_ctx *c) {
     a.sxy = c->d_sxy;
     a.sipos = c->d_sipos;
     a.sc = c->d_sc;
-    a.obj_lv = c->d_obj_lv;
-    a.obj_leaf = c->d_obj_leaf;
+    a.obj = c->d_obj;
     a.nodes = c->d_nodes;
     a.low = c->d_low;
     a.ibox = c->d_ibox;

@@ -49,6 +49,13 @@ uint64_t identify_tiles(uint64_t B) {
     return (B + tile - 1) / tile;
 }
 
+/* the bytes of w equal to v, one bit each */
+__device__ inline uint32_t byte_bits(uint32_t w, uint32_t v) {
+    const uint32_t m = __vcmpeq4(w, v * 0x01010101u) & 0x08040201u; /* bits 0, 9, 18 and 27 */
+    return (m | (m >> 8) | (m >> 16) | (m >> 24)) & 0xfu;
+}
+__device__ inline uint32_t emit_byte_bits(uint32_t w) { return byte_bits(w, kStampEmit); }
+
 /* warp-collective: the span's stamps into shared memory */
 template <uint32_t kSpan>
 __device__ inline void load_stamps(const uint8_t *stamp, uint64_t wbase, uint8_t *sst) {
@@ -80,16 +87,30 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_count(uint8_t *__restrict
         if (v) newline[(wbase >> 7) + lane] = 0;
     }
     load_stamps<kSpan>(stamp, wbase, sst[wid]);
-    /* the span's buckets whose record is needed */
-    const uint32_t below = (1u << lane) - 1u;
+    /* the span's buckets whose record is needed, 16 per lane at a time */
     uint32_t n = 0;
-#pragma unroll 4
-    for (uint32_t off = lane; off < kSpan; off += 32) {
-        const bool need = wbase + off < B &&
-                          (sst[wid][off] != kStampEmpty || ((snl[wid][off >> 7] >> ((off >> 2) & 31)) & 1u));
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (need) slist[wid][n + __popc(m & below)] = (uint16_t)off;
-        n += __popc(m);
+#pragma unroll
+    for (uint32_t i0 = 0; i0 < kSpan; i0 += 512) {
+        const uint32_t off = i0 + lane * 16;
+        uint32_t bits = 0;
+        if (off < kSpan && wbase + off < B) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(&sst[wid][off]);
+            bits = ~(byte_bits(v.x, 0) | (byte_bits(v.y, 0) << 4) | (byte_bits(v.z, 0) << 8) | (byte_bits(v.w, 0) << 12));
+            /* every slot of a line that received a pair */
+            const uint32_t lines = (snl[wid][off >> 7] >> ((off >> 2) & 31)) & 0xfu;
+            bits |= ((lines & 1u) | ((lines & 2u) << 3) | ((lines & 4u) << 6) | ((lines & 8u) << 9)) * 0xfu;
+            const uint64_t left = B - (wbase + off);
+            bits &= left < 16 ? (1u << left) - 1u : 0xffffu;
+        }
+        uint32_t incl = __popc(bits);
+        const uint32_t mine = incl;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        uint32_t at = n + incl - mine;
+        n += __shfl_sync(0xffffffffu, incl, 31);
+        for (; bits; bits &= bits - 1) slist[wid][at++] = (uint16_t)(off + __ffs(bits) - 1);
     }
     __syncwarp();
     uint32_t emit = 0, taken = 0, active = 0;
@@ -190,25 +211,37 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_count(uint8_t *__restrict
     }
 }
 
-/* the bytes of w equal to kStampEmit, one bit each */
-__device__ inline uint32_t emit_bits(uint32_t w) {
-    const uint32_t m = __vcmpeq4(w, kStampEmit * 0x01010101u) & 0x08040201u; /* bits 0, 9, 18 and 27 */
-    return (m | (m >> 8) | (m >> 16) | (m >> 24)) & 0xfu;
-}
-
 /* Pass 2: the reports of tiles that have any, in bucket order, into the
  * meeting log.  A warp reads its stamps 16 at a time, lists the reports of
- * its span in order and writes them with consecutive lanes. */
-template <uint32_t kSpan>
+ * its span in order and writes them with consecutive lanes.  With few tiles
+ * (kOwnScan) a block adds up the counts before its own itself, which costs
+ * less than the scan's launch. */
+template <uint32_t kSpan, bool kOwnScan>
 __global__ void __launch_bounds__(kIdThreads) k_expire_emit(uint8_t *__restrict__ stamp, TRec *__restrict__ tab,
                                                             const uint32_t *__restrict__ tile_cnt,
-                                                            const uint32_t *__restrict__ tile_off,
+                                                            uint32_t *__restrict__ tile_off,
                                                             glint_meeting *__restrict__ log, uint64_t log_cap,
                                                             const DevCounters *cnt) {
-    if (tile_cnt[blockIdx.x] == 0) return; /* uniform per block */
     __shared__ uint32_t ws[kIdWarps];
     __shared__ uint16_t slist[kIdWarps][kSpan];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t before = 0;
+    if (kOwnScan) {
+        /* the last block also leaves the total */
+        const bool last = blockIdx.x == gridDim.x - 1;
+        if (tile_cnt[blockIdx.x] == 0 && !last) return; /* uniform per block */
+        uint32_t v = 0;
+        for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kIdThreads) v += tile_cnt[i];
+        v = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0) ws[wid] = v;
+        __syncthreads();
+        for (int w = 0; w < kIdWarps; ++w) before += ws[w];
+        __syncthreads();
+        if (last && threadIdx.x == 0) tile_off[gridDim.x] = before + tile_cnt[blockIdx.x];
+    } else {
+        if (tile_cnt[blockIdx.x] == 0) return; /* uniform per block */
+        before = tile_off[blockIdx.x];
+    }
     const uint64_t wbase = ((uint64_t)blockIdx.x * kIdWarps + wid) * kSpan;
     uint4 *st = reinterpret_cast<uint4 *>(stamp + wbase);
     uint32_t n = 0;
@@ -217,7 +250,7 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_emit(uint8_t *__restrict_
         const uint32_t i = i0 + lane;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (i < kSpan / 16) v = st[i];
-        uint32_t bits = emit_bits(v.x) | (emit_bits(v.y) << 4) | (emit_bits(v.z) << 8) | (emit_bits(v.w) << 12);
+        uint32_t bits = emit_byte_bits(v.x) | (emit_byte_bits(v.y) << 4) | (emit_byte_bits(v.z) << 8) | (emit_byte_bits(v.w) << 12);
         uint32_t incl = __popc(bits);
         const uint32_t mine = incl;
         for (int o = 1; o < 32; o <<= 1) {
@@ -238,7 +271,7 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_emit(uint8_t *__restrict_
     }
     if (lane == 0) ws[wid] = n;
     __syncthreads();
-    uint64_t pos = cnt->log_head + tile_off[blockIdx.x];
+    uint64_t pos = cnt->log_head + before;
     for (int w = 0; w < wid; ++w) pos += ws[w];
     const uint32_t cur_time = cnt->step_time;
     for (uint32_t i = lane; i < n; i += 32) {
@@ -253,6 +286,9 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_emit(uint8_t *__restrict_
     }
 }
 
+/* up to here a block's own sum is four loads per thread */
+constexpr unsigned kOwnScanTiles = 1024;
+
 template <uint32_t kSpan>
 static void identify_passes(glint_ctx *c) {
     cudaStream_t s = c->stream;
@@ -260,9 +296,14 @@ static void identify_passes(glint_ctx *c) {
     k_expire_count<kSpan><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_newline, c->d_tab, c->B,
                                                        c->cfg.min_meet_time + 1, c->d_tile_cnt, c->d_fpos, c->N,
                                                        c->d_cnt);
+    if (tiles <= kOwnScanTiles) {
+        k_expire_emit<kSpan, true><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_tab, c->d_tile_cnt, c->d_tile_off,
+                                                                c->d_log, c->log_cap, c->d_cnt);
+        return;
+    }
     scan_u32(c->d_tile_cnt, c->d_tile_off, tiles, c->d_scan_tmp, s);
-    k_expire_emit<kSpan><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_tab, c->d_tile_cnt, c->d_tile_off, c->d_log,
-                                                      c->log_cap, c->d_cnt);
+    k_expire_emit<kSpan, false><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_tab, c->d_tile_cnt, c->d_tile_off,
+                                                             c->d_log, c->log_cap, c->d_cnt);
 }
 
 /* The step's reports are counted by tile_off[tiles]; the log's head moves in

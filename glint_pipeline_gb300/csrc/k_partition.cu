@@ -25,9 +25,7 @@ constexpr int kMaxDepth = 64;
 
 __global__ void __launch_bounds__(256) k_descend(const double2 *__restrict__ pts, const uint32_t *__restrict__ order,
                                                  uint32_t N, const DNode *__restrict__ nodes, uint32_t S, uint32_t G,
-                                                 double xb, double yb,
-                                                 uint32_t *__restrict__ obj_gid, uint32_t *__restrict__ obj_lv,
-                                                 uint32_t *__restrict__ obj_leaf, uint32_t *__restrict__ obj_pos,
+                                                 double xb, double yb, uint4 *__restrict__ obj,
                                                  uint32_t *__restrict__ grid_count, DevCounters *cnt) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         const uint32_t pid = order[i];
@@ -59,9 +57,6 @@ __global__ void __launch_bounds__(256) k_descend(const double2 *__restrict__ pts
                 break;
             }
         }
-        obj_gid[pid] = gid;
-        obj_lv[pid] = lv;
-        obj_leaf[pid] = cur;
         /* objects come in the previous step's leaf order, so the lanes of a
          * warp mostly share a leaf: one atomic per leaf and warp, which also
          * gives each object its place in the leaf's segment */
@@ -70,16 +65,19 @@ __global__ void __launch_bounds__(256) k_descend(const double2 *__restrict__ pts
         uint32_t at = 0;
         if ((threadIdx.x & 31) == leader) at = atomicAdd(&grid_count[gid], (uint32_t)__popc(peers));
         at = __shfl_sync(peers, at, leader);
-        obj_pos[pid] = at + __popc(peers & ((1u << (threadIdx.x & 31)) - 1u));
+        /* one 16-byte record: objects come in leaf order, so each write is a
+         * memory transaction of its own */
+        obj[pid] = make_uint4(gid, lv, cur, at + __popc(peers & ((1u << (threadIdx.x & 31)) - 1u)));
     }
 }
 
-__global__ void __launch_bounds__(256) k_scatter(const uint32_t *__restrict__ obj_gid,
-                                                 const uint32_t *__restrict__ obj_pos, uint32_t N,
+__global__ void __launch_bounds__(256) k_scatter(const uint4 *__restrict__ obj, uint32_t N,
                                                  const uint32_t *__restrict__ grid_start,
                                                  uint32_t *__restrict__ sorted) {
-    for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < N; pid += gridDim.x * blockDim.x)
-        sorted[grid_start[obj_gid[pid]] + obj_pos[pid]] = pid;
+    for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < N; pid += gridDim.x * blockDim.x) {
+        const uint4 o = obj[pid];
+        sorted[grid_start[o.x] + o.w] = pid;
+    }
 }
 
 /* the scan of the leaf counts: segment starts, and on the way the leaves that
@@ -130,11 +128,15 @@ struct GatherOut {
     float *sc;
     double *sm;        /* null: not needed */
     float2 *fpos;      /* by object id */
-    uint32_t *rank_of;
+    uint2 *rank;       /* by object id: sorted position and leaf node */
+    const uint4 *obj;
+    uint32_t cap;
 };
 
-__device__ inline void gather_one(const GatherOut &o, const Frame &f, const double2 *__restrict__ pts, uint32_t i,
-                                  uint32_t pid) {
+/* the object pid at place `at` of the segment of a leaf node that starts at s0 */
+__device__ inline void gather_one(const GatherOut &o, const Frame &f, const double2 *__restrict__ pts, uint32_t s0,
+                                  uint32_t at, uint32_t pid, uint32_t leaf) {
+    const uint32_t i = s0 + at;
     const double2 p = pts[pid];
     o.sxy[i] = p;
     bool clamped = false;
@@ -146,7 +148,7 @@ __device__ inline void gather_one(const GatherOut &o, const Frame &f, const doub
     o.sfpos[i] = fp;
     o.fpos[pid] = fp;
     if (o.sm) o.sm[i] = metres_per_degree(p.y, f);
-    o.rank_of[pid] = i;
+    o.rank[pid] = make_uint2(at < o.cap ? i : i | kDropped, leaf);
 }
 
 /* bitonic sort of n (<= 1024) keys in a warp's shared buffer, padded with ~0u */
@@ -193,6 +195,8 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t
         if (n > kWarpSortMax) continue;
         const uint32_t s0 = grid_start[g];
         uint32_t *seg = sorted + s0;
+        const uint32_t leaf = o.obj[seg[0]].z; /* the node of grid g: one for all its objects */
+        __syncwarp();
         if (n <= 32) {
             uint32_t v = lane < (int)n ? seg[lane] : 0xffffffffu;
             /* register bitonic sort across the warp */
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t
             }
             if (lane < (int)n) {
                 seg[lane] = v;
-                gather_one(o, f, pts, s0 + lane, v);
+                gather_one(o, f, pts, s0, lane, v, leaf);
             }
         } else {
             for (uint32_t i = lane; i < n; i += 32) buf[w][i] = seg[i];
@@ -215,7 +219,7 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t
             warp_bitonic(buf[w], n);
             for (uint32_t i = lane; i < n; i += 32) {
                 seg[i] = buf[w][i];
-                gather_one(o, f, pts, s0 + i, buf[w][i]);
+                gather_one(o, f, pts, s0, i, buf[w][i], leaf);
             }
         }
         __syncwarp();
@@ -241,12 +245,15 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
              * follows in this step reads objects */
             if (threadIdx.x == 0) atomicOr(&cnt->error_flags, GLINT_EF_SEGMENT_TOO_LARGE);
             for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-                gather_one(o, f, pts, grid_start[g] + i, sorted[grid_start[g] + i]);
+                gather_one(o, f, pts, grid_start[g], i, sorted[grid_start[g] + i],
+                           o.obj[sorted[grid_start[g]]].z);
             continue;
         }
         uint32_t P = 1024;
         while (P < n) P <<= 1;
         uint32_t *seg = sorted + grid_start[g];
+        const uint32_t leaf = o.obj[seg[0]].z;
+        __syncthreads();
         for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) sbuf[i] = i < n ? seg[i] : 0xffffffffu;
         __syncthreads();
         for (uint32_t k = 2; k <= P; k <<= 1) {
@@ -264,7 +271,7 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
         }
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
             seg[i] = sbuf[i];
-            gather_one(o, f, pts, grid_start[g] + i, sbuf[i]);
+            gather_one(o, f, pts, grid_start[g], i, sbuf[i], leaf);
         }
         __syncthreads();
     }
@@ -293,13 +300,12 @@ cudaError_t launch_step_begin(glint_ctx *c) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_partition(glint_ctx *c, uint32_t /*cur_time*/) {
+cudaError_t launch_partition(glint_ctx *c, const double2 *pts) {
     cudaStream_t s = c->stream;
     const uint32_t N = c->N, G = c->G;
     /* the last step's leaf-major order is the descent's processing order */
-    k_descend<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_pts, c->d_sorted, N, c->d_nodes, c->S, G, c->x_buffer,
-                                                           c->y_buffer, c->d_obj_gid, c->d_obj_lv, c->d_obj_leaf,
-                                                           c->d_obj_pos, c->d_grid_count, c->d_cnt);
+    k_descend<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(pts, c->d_sorted, N, c->d_nodes, c->S, G, c->x_buffer,
+                                                           c->y_buffer, c->d_obj, c->d_grid_count, c->d_cnt);
     LeafScan ls;
     ls.start = ScanStore{c->d_grid_start, true};
     ls.work = c->d_leaf_work;
@@ -308,7 +314,7 @@ cudaError_t launch_partition(glint_ctx *c, uint32_t /*cur_time*/) {
     ls.warp_limit = kWarpSortMax;
     ls.cnt = c->d_cnt;
     scan_launch(ScanWords{c->d_grid_count, true}, ls, G, &c->d_cnt->grids_used, c->d_scan_tmp, s);
-    k_scatter<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_obj_gid, c->d_obj_pos, N, c->d_grid_start, c->d_sorted);
+    k_scatter<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_obj, N, c->d_grid_start, c->d_sorted);
     GatherOut o;
     o.sxy = c->d_sxy;
     o.sipos = c->d_sipos;
@@ -316,11 +322,13 @@ cudaError_t launch_partition(glint_ctx *c, uint32_t /*cur_time*/) {
     o.sc = c->d_sc;
     o.sm = c->cfg.precision_mode == 1 ? nullptr : c->d_sm;
     o.fpos = c->d_fpos;
-    o.rank_of = c->d_rank_of;
+    o.rank = c->d_rank;
+    o.obj = c->d_obj;
+    o.cap = c->cap;
     k_segsort_warp<<<grid_for(N, 16 * kSortWarps, 152u * 8u), 32 * kSortWarps, 0, s>>>(
-        c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_pts, o, c->frame, c->d_cnt);
+        c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted, pts, o, c->frame, c->d_cnt);
     k_segsort_block<<<152, 1024, kBlockSortMax * sizeof(uint32_t), s>>>(
-        c->d_big, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_pts, o, c->frame, c->d_cnt);
+        c->d_big, c->d_grid_start, c->d_grid_count, c->d_sorted, pts, o, c->frame, c->d_cnt);
     return cudaGetLastError();
 }
 

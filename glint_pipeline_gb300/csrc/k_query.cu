@@ -242,9 +242,9 @@ __global__ void __launch_bounds__(128) k_search_objects(ObjectSearch o, const ui
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 32; i < npids; i += gridDim.x * blockDim.x / 32) {
         const uint32_t p = pids[i];
         if (p >= o.s.N) continue;
-        const uint32_t r = a.rank_of[p], g = a.obj_gid[p];
+        const uint32_t rank = a.rank[p].x, r = rank & ~kDropped, g = a.obj[p].x;
         const uint32_t s0 = a.grid_start[g], k = min(a.grid_start[g + 1] - s0, a.cap);
-        const bool stored = r - s0 < k;
+        const bool stored = !(rank & kDropped);
         for (uint32_t j = lane; stored && j < k; j += 32) {
             const uint32_t m = s0 + j;
             if (m != r && within_reach(a, min(r, m), max(r, m))) found_contact(o, p, a.sorted[m]);
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(128) k_search_objects(ObjectSearch o, const ui
         const uint32_t tb = a.tstart[g], te = a.tstart[g + 1];
         for (uint32_t t = tb + lane; stored && t < te; t += 32) {
             const uint32_t q = a.tlist[t].x;
-            if (within_reach(a, a.rank_of[q], r)) found_contact(o, p, q);
+            if (within_reach(a, a.rank[q].x & ~kDropped, r)) found_contact(o, p, q);
         }
     }
 }

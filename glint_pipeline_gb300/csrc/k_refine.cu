@@ -74,7 +74,6 @@ RefineArgs refine_args(glint_ctx *c) {
     a.sorted = c->d_sorted;
     a.sxy = c->d_sxy;
     a.sm = c->d_sm;
-    a.obj_leaf = c->d_obj_leaf;
     a.ibox = c->d_ibox;
     a.tstart = c->d_tstart;
     a.tlist = c->d_tlist;
@@ -82,8 +81,8 @@ RefineArgs refine_args(glint_ctx *c) {
     a.sfpos = c->d_sfpos;
     a.sc = c->d_sc;
     a.f = c->frame;
-    a.obj_gid = c->d_obj_gid;
-    a.rank_of = c->d_rank_of;
+    a.obj = c->d_obj;
+    a.rank = c->d_rank;
     a.qstart = c->d_qstart;
     a.qcount = c->d_qcount;
     a.qlist = c->d_qlist;

@@ -37,11 +37,10 @@ struct RefineArgs {
     const longlong2 *sipos;    /* fixed-point coordinates, leaf-major */
     const float2 *sfpos;       /* FP32 coordinates, leaf-major */
     const float *sc;           /* screening scale cx, leaf-major */
-    const uint32_t *obj_gid;
-    const uint32_t *rank_of;
+    const uint4 *obj;          /* by object id: leaf grid, .. */
+    const uint2 *rank;         /* by object id: leaf-major rank (kDropped: not stored), leaf node */
     const uint32_t *qstart, *qcount;
     const uint32_t *qlist;
-    const uint32_t *obj_leaf;
     const IBox *ibox;
     const uint2 *extra;        /* (leaf, chunk) items beyond each leaf's first chunk */
     TRec *tab;
@@ -168,7 +167,7 @@ __device__ inline bool queued_contact(const RefineArgs &a, QEntry &q, RefineTall
          * order; keep only one event */
         const uint32_t qid = (uint32_t)(q.prio >> 36) & 0x7ffffffu;
         const uint32_t mid = pair_a(q.pw) == qid ? pair_b(q.pw) : pair_a(q.pw);
-        if (has_check(a, mid, a.obj_gid[qid]) && pair_fp64(a, r2, r1)) return false;
+        if (has_check(a, mid, a.obj[qid].x) && pair_fp64(a, r2, r1)) return false;
     }
     const float2 A = a.sfpos[r1], B = a.sfpos[r2];
     q.v = make_uint4(__float_as_uint(A.x), __float_as_uint(A.y), __float_as_uint(B.x), __float_as_uint(B.y));
@@ -444,13 +443,13 @@ __device__ inline void refine_item(const RefineArgs &a, uint32_t g, uint32_t chu
             const uint2 qe = a.tlist[t0 + lane];
             q = qe.x;
             ord = qe.y;
-            qr = a.rank_of[q];
-            const IBox own = a.ibox[a.obj_leaf[q]];
-            const uint32_t qgid = a.obj_gid[q];
+            const uint2 rl = a.rank[q];
+            qstored = !(rl.x & kDropped);
+            qr = rl.x & ~kDropped;
+            const IBox own = a.ibox[rl.y];
             const longlong2 qi = a.sipos[qr];
             cq = a.sc[qr];
             if (!kFp64) qf = a.sfpos[qr];
-            qstored = (qr - a.grid_start[qgid]) < a.cap;
             px = fx_to_f(qi.x - o.X0);
             py = fx_to_f(qi.y - o.Y0);
             bq = pair_band(f, cq, fmaxf(o.Mx, fabsf(px)), fmaxf(o.My, fabsf(py)));
@@ -514,7 +513,7 @@ __device__ inline void refine_item(const RefineArgs &a, uint32_t g, uint32_t chu
                     t.hits += hit ? 1 : 0;
                     /* mm's test comes first in the reference's order when
                      * mm < q; keep only one event */
-                    if (hit && dup && has_check(a, mm, a.obj_gid[Q0])) {
+                    if (hit && dup && has_check(a, mm, a.obj[Q0].x)) {
                         const float cm = m.cb[j].x;
                         const float d2 = screen_q(f, P.x - X, P.y - Y, cm);
                         const float b2 = pair_band(f, cm, fmaxf(o.Mx, fabsf(X)), fmaxf(o.My, fabsf(Y)));

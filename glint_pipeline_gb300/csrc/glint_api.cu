@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(64) k_step_tail(uint32_t N, const uint32_t *re
 }
 
 void free_all(glint_ctx *c) {
-    void *ptrs[] = {c->d_pts, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj, c->d_grid_count,
+    void *ptrs[] = {c->d_pts, c->d_in, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj, c->d_grid_count,
                     c->d_grid_start, c->d_sorted, c->d_rank, c->d_sxy, c->d_sm, c->d_leaf_work,
                     c->d_nodes, c->d_low, c->d_sstack, c->d_gstack, c->d_split, c->d_evscan, c->d_cand, c->d_newgid,
                     c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
@@ -199,7 +199,7 @@ void free_all(glint_ctx *c) {
     server_free_default(c);
     servers_detach(c);
     if (c->h_cnt) cudaFreeHost(c->h_cnt);
-    if (c->h_params) cudaFreeHost(c->h_params);
+    if (c->h_input) cudaFreeHost(c->h_input);
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
     if (c->graph) cudaGraphDestroy(c->graph);
     if (c->timers.created) {
@@ -410,6 +410,7 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
         }                                                                  \
     } while (0)
     ALLOC(c->d_pts, N);
+    ALLOC(c->d_in, 1);
     ALLOC(c->d_sipos, N);
     ALLOC(c->d_sfpos, N);
     ALLOC(c->d_sc, N);
@@ -469,13 +470,13 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
         delete c;
         return st;
     }
-    if ((e = cudaMallocHost((void **)&c->h_params, sizeof(StepParams))) != cudaSuccess) {
+    if ((e = cudaMallocHost((void **)&c->h_input, sizeof(StepInput))) != cudaSuccess) {
         glint_status st = cuda_fail(c, e, "cudaMallocHost");
         free_all(c);
         delete c;
         return st;
     }
-    std::memset(c->h_params, 0, sizeof(StepParams));
+    std::memset((void *)c->h_input, 0, sizeof(StepInput));
     if ((e = cudaMallocHost((void **)&c->h_cnt, sizeof(DevCounters))) != cudaSuccess) {
         glint_status st = cuda_fail(c, e, "cudaMallocHost");
         free_all(c);
@@ -624,28 +625,28 @@ glint_status glint_get_capacities(const glint_ctx *c, uint32_t *sc, uint32_t *gc
 
 namespace glint {
 
-/* The launches of one step, from the counter reset to the copy of the
+/* A step's points: host points are copied into the context's buffer; points
+ * in device memory on a 16-byte boundary are read in place (a copy of theirs
+ * was 10 us of a 1M-object step's 700); others are copied too. */
+cudaError_t step_input(glint_ctx *c, const double *points, bool host) {
+    c->h_input->pts = c->d_pts;
+    if (!host && c->input_device && ((uintptr_t)points & 15) == 0) {
+        c->h_input->pts = reinterpret_cast<const double2 *>(points);
+        return cudaSuccess;
+    }
+    return cudaMemcpyAsync(c->d_pts, points, sizeof(double2) * c->N,
+                           host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, c->stream);
+}
+
+/* The launches of one step after its begin kernel, to the copy of the
  * counters to the host; no host synchronisation, so they can be captured.
  * A step is its front (up to the refine stage's work items), the refine
  * pair tests, and its back: a batch of regions runs every front, then one
  * refine launch over all regions, then every back. */
-void launch_step_front(glint_ctx *c, const double *points, bool host) {
+void launch_step_front(glint_ctx *c) {
     cudaStream_t s = c->stream;
     const bool tm = c->cfg.timing != 0 && !c->cfg.use_graph;
-    launch_step_begin(c);
-    if (tm) cudaEventRecord(c->timers.ev[0], s);
-    /* points in device memory on a 16-byte boundary are read in place (a copy
-     * of theirs was 10 us of a 1M-object step's 700) */
-    const double2 *pts = c->d_pts;
-    if (host) {
-        cudaMemcpyAsync(c->d_pts, points, sizeof(double2) * c->N, cudaMemcpyHostToDevice, s);
-    } else if (c->input_device && ((uintptr_t)points & 15) == 0) {
-        pts = reinterpret_cast<const double2 *>(points);
-    } else {
-        cudaMemcpyAsync(c->d_pts, points, sizeof(double2) * c->N, cudaMemcpyDeviceToDevice, s);
-    }
-    if (tm) cudaEventRecord(c->timers.ev[1], s);
-    launch_partition(c, pts);
+    launch_partition(c);
     if (tm) cudaEventRecord(c->timers.ev[2], s);
     launch_filter(c);
     if (tm) cudaEventRecord(c->timers.ev[3], s);
@@ -676,21 +677,18 @@ void launch_step_back(glint_ctx *c) {
     if (tm) cudaEventRecord(c->timers.ev[7], s);
 }
 
-static void launch_step(glint_ctx *c, const double *points, bool host) {
-    launch_step_front(c, points, host);
+static void launch_step(glint_ctx *c) {
+    launch_step_front(c);
     launch_refine_pairs(c);
     launch_step_back(c);
 }
 
-/* the host side of starting a step: its number, time, tag and the
- * parameters the captured memcpy reads when the step runs */
+/* the host side of starting a step: its number, time, tag and parameters */
 void begin_step(glint_ctx *c, uint32_t cur_time) {
     c->step_index++;
     c->step_lists = true;
     c->last_time = cur_time;
-    c->h_params->step_time = cur_time;
-    c->h_params->step_tag = stamp_of(c->step_index);
-    c->h_params->end_time_min = c->end_time_min;
+    c->h_input->p = StepParams{cur_time, stamp_of(c->step_index), c->end_time_min, 0};
     c->stats_valid = false;
 }
 
@@ -715,35 +713,64 @@ bool device_points(glint_ctx *c, const void *p) {
 
 extern "C" {
 
-static glint_status enqueue_step(glint_ctx *c, const double *points, bool host, uint32_t cur_time,
-                                 bool allow_graph = true) {
-    cudaStream_t s = c->stream;
-    /* a captured step reads its parameters from host memory when it runs:
-     * the previous step must have finished before they are overwritten */
-    if (c->cfg.use_graph && c->step_index > 0) cudaStreamSynchronize(s);
-    begin_step(c, cur_time);
-    if (!c->cfg.use_graph || host || !allow_graph) {
-        launch_step(c, points, host);
-    } else {
-        if (c->graph_exec && c->graph_src != (const void *)points) {
-            cudaGraphExecDestroy(c->graph_exec);
-            cudaGraphDestroy(c->graph);
-            c->graph_exec = nullptr;
-            c->graph = nullptr;
-        }
-        if (!c->graph_exec) {
-            cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-            if (e != cudaSuccess) return cuda_fail(c, e, "step capture");
-            launch_step(c, points, false);
-            e = cudaStreamEndCapture(s, &c->graph);
-            if (e == cudaSuccess) e = cudaGraphInstantiate(&c->graph_exec, c->graph, 0);
-            if (e != cudaSuccess) return cuda_fail(c, e, "step capture");
-            c->graph_src = points;
-        }
-        cudaError_t e = cudaGraphLaunch(c->graph_exec, s);
-        if (e != cudaSuccess) return cuda_fail(c, e, "step graph");
+/* the step's launches after its begin kernel, captured once as a graph: they
+ * read their parameters and where the points lie from the device, so one graph
+ * serves every step.  They append to the pending keys' buffer, which a flush
+ * that was refused leaves exchanged with its sorted one: then it is captured
+ * again. */
+static cudaError_t step_graph(glint_ctx *c) {
+    if (c->graph_exec && c->graph_keys == (const void *)c->d_keys) return cudaSuccess;
+    if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
+    if (c->graph) cudaGraphDestroy(c->graph);
+    c->graph_exec = nullptr;
+    c->graph = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    launch_step(c);
+    e = cudaStreamEndCapture(c->stream, &c->graph);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&c->graph_exec, c->graph, 0);
+    if (e != cudaSuccess) {
+        c->graph_exec = nullptr;
+        return e;
     }
-    cudaError_t e = cudaGetLastError();
+    c->graph_keys = c->d_keys;
+    return cudaSuccess;
+}
+
+/* One launch per step instead of 17 (each about 2.5 us of the host's time,
+ * 0.5 us more between dependent kernels on the device): 20k objects 177 -> 128 us a
+ * step, 100k 205 -> 165 us, 1M 850 -> 824 us.  The first step of
+ * a context is launched kernel by kernel unless glint_config.use_graph asks for
+ * the graph at once, as are timed steps and steps inside a caller's own
+ * capture. */
+static glint_status enqueue_step(glint_ctx *c, const double *points, bool host, uint32_t cur_time) {
+    cudaStream_t s = c->stream;
+    const bool tm = c->cfg.timing != 0 && !c->cfg.use_graph;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(s, &cap);
+    const bool graph = !tm && cap == cudaStreamCaptureStatusNone && !c->graph_off &&
+                       (c->cfg.use_graph || c->step_index > 0);
+    if (graph) {
+        const cudaError_t e = step_graph(c);
+        if (e != cudaSuccess) {
+            if (c->cfg.use_graph) return cuda_fail(c, e, "step capture");
+            cudaGetLastError();
+            c->graph_off = true;
+        }
+    }
+    begin_step(c, cur_time);
+    if (tm) cudaEventRecord(c->timers.ev[0], s);
+    cudaError_t e = step_input(c, points, host);
+    if (e != cudaSuccess) return cuda_fail(c, e, "step input");
+    if (tm) cudaEventRecord(c->timers.ev[1], s);
+    launch_step_begin(c, false);
+    if (graph && !c->graph_off) {
+        e = cudaGraphLaunch(c->graph_exec, s);
+        if (e != cudaSuccess) return cuda_fail(c, e, "step graph");
+    } else {
+        launch_step(c);
+    }
+    e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "step launch");
     return GLINT_OK;
 }
@@ -941,6 +968,6 @@ namespace glint {
  * buffer is fixed) */
 glint_status enqueue_device_step_plain(glint_ctx *c, const double *d_points, uint32_t cur_time) {
     c->input_device = true; /* the pipe's own buffers */
-    return enqueue_step(c, d_points, false, cur_time, false);
+    return enqueue_step(c, d_points, false, cur_time);
 }
 } // namespace glint

@@ -45,7 +45,7 @@ struct glint_batch {
     uint32_t cap_max = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    std::vector<const double *> src;
+    std::vector<const void *> keys; /* the buffers the captured key appends write to */
     bool launched = false;
     int device = 0;
 };
@@ -71,13 +71,14 @@ void batch_release(glint_batch *b) {
 
 /* the launches of one timestep of every region, on the batch stream and the
  * regions' streams; captured into the batch's graph */
-void launch_batch_step(glint_batch *b, const double *const *d_points) {
+void launch_batch_step(glint_batch *b) {
     const size_t R = b->regions.size();
     cudaEventRecord(b->fork_ev, b->stream);
     for (size_t r = 0; r < R; ++r) {
         glint_ctx *c = b->regions[r];
         cudaStreamWaitEvent(c->stream, b->fork_ev, 0);
-        glint::launch_step_front(c, d_points[r], false);
+        glint::launch_step_begin(c, true);
+        glint::launch_step_front(c);
         cudaEventRecord(b->front_ev[r], c->stream);
         cudaStreamWaitEvent(b->stream, b->front_ev[r], 0);
     }
@@ -185,14 +186,22 @@ extern "C" glint_status glint_batch_step(glint_batch *b, const double *const *d_
         const cudaError_t e = cudaStreamSynchronize(b->stream);
         if (e != cudaSuccess) return batch_fail(b, e, "batch step");
     }
+    for (glint_ctx *c : b->regions) glint::begin_step(c, cur_time);
+    for (size_t r = 0; r < R; ++r) {
+        const cudaError_t e = glint::step_input(b->regions[r], d_points[r], false);
+        if (e != cudaSuccess) return batch_fail(b, e, "batch input");
+    }
     /* work a caller queued on a region's own stream (a search, a flush) goes
      * first */
     for (size_t r = 0; r < R; ++r) {
         cudaEventRecord(b->pre_ev[r], b->regions[r]->stream);
         cudaStreamWaitEvent(b->stream, b->pre_ev[r], 0);
     }
-    for (glint_ctx *c : b->regions) glint::begin_step(c, cur_time);
-    const bool same = b->exec && std::equal(b->src.begin(), b->src.end(), d_points);
+    /* the graph takes each region's parameters and points from host memory
+     * when it runs, so it serves every timestep; its key appends write to the
+     * buffers it was captured with, which a refused flush leaves exchanged */
+    bool same = b->exec != nullptr;
+    for (size_t r = 0; r < R && same; ++r) same = b->keys[r] == (const void *)b->regions[r]->d_keys;
     if (!same) {
         if (b->exec) cudaGraphExecDestroy(b->exec);
         if (b->graph) cudaGraphDestroy(b->graph);
@@ -200,11 +209,12 @@ extern "C" glint_status glint_batch_step(glint_batch *b, const double *const *d_
         b->graph = nullptr;
         cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return batch_fail(b, e, "batch capture");
-        launch_batch_step(b, d_points);
+        launch_batch_step(b);
         e = cudaStreamEndCapture(b->stream, &b->graph);
         if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, b->graph, 0);
         if (e != cudaSuccess) return batch_fail(b, e, "batch capture");
-        b->src.assign(d_points, d_points + R);
+        b->keys.clear();
+        for (glint_ctx *c : b->regions) b->keys.push_back(c->d_keys);
     }
     cudaError_t e = cudaGraphLaunch(b->exec, b->stream);
     if (e == cudaSuccess) e = cudaGetLastError();

@@ -81,6 +81,11 @@ struct DevCounters {
 struct StepParams {
     unsigned int step_time, step_tag, end_time_min, pad3;
 };
+/* what a step starts from: its parameters and where its points lie */
+struct StepInput {
+    StepParams p;
+    const double2 *pts;
+};
 /* bytes cleared at the start of every step */
 constexpr size_t kStepCounterBytes = offsetof(DevCounters, ssi);
 
@@ -280,10 +285,12 @@ struct glint_ctx {
     void *d_scan_tmp_side = nullptr;       /* the schema update's, as it runs beside identify */
     size_t scan_tmp_bytes = 0;
     double2 *h_stage = nullptr;            /* pinned staging for host points (optional) */
-    glint::StepParams *h_params = nullptr; /* pinned: the next step's parameters */
-    cudaGraph_t graph = nullptr;           /* the captured step (glint_config.use_graph) */
+    glint::StepInput *h_input = nullptr;   /* pinned: the next step's (a batch's captured steps read it) */
+    const double2 **d_in = nullptr;        /* device: where the running step's points lie */
+    cudaGraph_t graph = nullptr;           /* the captured step, from its begin kernel on */
     cudaGraphExec_t graph_exec = nullptr;
-    const void *graph_src = nullptr;       /* input buffer the graph copies from */
+    const void *graph_keys = nullptr;      /* the pending keys' buffer it appends to */
+    bool graph_off = false;                /* capturing failed: steps are launched one by one */
     glint::StepTimers timers;
     glint_step_stats last_stats;
     bool stats_valid = false;
@@ -301,15 +308,16 @@ cudaError_t scan_u32(const uint32_t *in, uint32_t *out, size_t n, void *tmp, cud
 void init_sin_coef(SinCoef *host);
 
 /* ---- stages ---- */
-cudaError_t launch_step_begin(glint_ctx *c);
-cudaError_t launch_partition(glint_ctx *c, const double2 *pts);
+cudaError_t launch_step_begin(glint_ctx *c, bool from_host);
+cudaError_t launch_partition(glint_ctx *c);
 cudaError_t launch_filter(glint_ctx *c);
 cudaError_t launch_refine_pairs(glint_ctx *c);
 struct RefineArgs;
 RefineArgs refine_args(glint_ctx *c);
 cudaError_t launch_refine_precision_batch(const RefineArgs *d_args, uint32_t R, uint32_t cap_max, uint32_t *ex_off,
                                           uint32_t *wk_off, unsigned int *next, cudaStream_t s);
-void launch_step_front(glint_ctx *c, const double *points, bool host);
+cudaError_t step_input(glint_ctx *c, const double *points, bool host);
+void launch_step_front(glint_ctx *c);
 void launch_step_back(glint_ctx *c);
 void begin_step(glint_ctx *c, uint32_t cur_time);
 bool device_points(glint_ctx *c, const void *p);

@@ -23,10 +23,11 @@ namespace glint {
 
 constexpr int kMaxDepth = 64;
 
-__global__ void __launch_bounds__(256) k_descend(const double2 *__restrict__ pts, const uint32_t *__restrict__ order,
+__global__ void __launch_bounds__(256) k_descend(const double2 *const *in, const uint32_t *__restrict__ order,
                                                  uint32_t N, const DNode *__restrict__ nodes, uint32_t S, uint32_t G,
                                                  double xb, double yb, uint4 *__restrict__ obj,
                                                  uint32_t *__restrict__ grid_count, DevCounters *cnt) {
+    const double2 *__restrict__ pts = *in;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         const uint32_t pid = order[i];
         const double2 p = pts[pid];
@@ -184,9 +185,10 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t
                                                                   const uint32_t *__restrict__ grid_start,
                                                                   const uint32_t *__restrict__ grid_count,
                                                                   uint32_t *__restrict__ sorted,
-                                                                  const double2 *__restrict__ pts, GatherOut o,
+                                                                  const double2 *const *in, GatherOut o,
                                                                   Frame f, const DevCounters *cnt) {
     __shared__ uint32_t buf[kSortWarps][kWarpSortMax];
+    const double2 *__restrict__ pts = *in;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nwork = cnt->n_leaf_work;
     for (uint32_t li = blockIdx.x * kSortWarps + w; li < nwork; li += gridDim.x * kSortWarps) {
@@ -233,9 +235,10 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
                                                         const uint32_t *__restrict__ grid_start,
                                                         const uint32_t *__restrict__ grid_count,
                                                         uint32_t *__restrict__ sorted,
-                                                        const double2 *__restrict__ pts, GatherOut o, Frame f,
+                                                        const double2 *const *in, GatherOut o, Frame f,
                                                         DevCounters *cnt) {
     extern __shared__ uint32_t sbuf[];
+    const double2 *__restrict__ pts = *in;
     const uint32_t nbig = cnt->n_big;
     for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
         const uint32_t g = big[bi];
@@ -277,9 +280,10 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
     }
 }
 
-/* the start of a step: its counters cleared, its parameters (host memory)
- * taken in, and the counts of the leaves in use cleared */
-__global__ void __launch_bounds__(256) k_step_begin(const StepParams *__restrict__ params,
+/* the start of a step: its counters cleared, its parameters taken in (by
+ * value; from host memory in a batch's captured step), and the counts of the
+ * leaves in use cleared */
+__global__ void __launch_bounds__(256) k_step_begin(StepInput input, const StepInput *from, const double2 **in,
                                                     uint32_t *__restrict__ grid_count, uint32_t *__restrict__ tcount,
                                                     uint32_t G, DevCounters *cnt) {
     const uint32_t n = cnt->grids_used && cnt->grids_used < G ? cnt->grids_used : G;
@@ -290,21 +294,25 @@ __global__ void __launch_bounds__(256) k_step_begin(const StepParams *__restrict
     if (blockIdx.x == 0) {
         uint32_t *w = reinterpret_cast<uint32_t *>(cnt);
         for (uint32_t i = threadIdx.x; i < kStepCounterBytes / 4; i += blockDim.x) w[i] = 0;
-        if (threadIdx.x == 0) *reinterpret_cast<StepParams *>(&cnt->step_time) = *params;
+        if (threadIdx.x == 0) {
+            if (from) input = *from;
+            *reinterpret_cast<StepParams *>(&cnt->step_time) = input.p;
+            *in = input.pts;
+        }
     }
 }
 
-cudaError_t launch_step_begin(glint_ctx *c) {
-    k_step_begin<<<grid_for(c->G, 256, 152u * 4u), 256, 0, c->stream>>>(c->h_params, c->d_grid_count, c->d_tcount, c->G,
-                                                                       c->d_cnt);
+cudaError_t launch_step_begin(glint_ctx *c, bool from_host) {
+    k_step_begin<<<grid_for(c->G, 256, 152u * 4u), 256, 0, c->stream>>>(
+        *c->h_input, from_host ? c->h_input : nullptr, c->d_in, c->d_grid_count, c->d_tcount, c->G, c->d_cnt);
     return cudaGetLastError();
 }
 
-cudaError_t launch_partition(glint_ctx *c, const double2 *pts) {
+cudaError_t launch_partition(glint_ctx *c) {
     cudaStream_t s = c->stream;
     const uint32_t N = c->N, G = c->G;
     /* the last step's leaf-major order is the descent's processing order */
-    k_descend<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(pts, c->d_sorted, N, c->d_nodes, c->S, G, c->x_buffer,
+    k_descend<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_in, c->d_sorted, N, c->d_nodes, c->S, G, c->x_buffer,
                                                            c->y_buffer, c->d_obj, c->d_grid_count, c->d_cnt);
     LeafScan ls;
     ls.start = ScanStore{c->d_grid_start, true};
@@ -326,9 +334,9 @@ cudaError_t launch_partition(glint_ctx *c, const double2 *pts) {
     o.obj = c->d_obj;
     o.cap = c->cap;
     k_segsort_warp<<<grid_for(N, 16 * kSortWarps, 152u * 8u), 32 * kSortWarps, 0, s>>>(
-        c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted, pts, o, c->frame, c->d_cnt);
+        c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_in, o, c->frame, c->d_cnt);
     k_segsort_block<<<152, 1024, kBlockSortMax * sizeof(uint32_t), s>>>(
-        c->d_big, c->d_grid_start, c->d_grid_count, c->d_sorted, pts, o, c->frame, c->d_cnt);
+        c->d_big, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_in, o, c->frame, c->d_cnt);
     return cudaGetLastError();
 }
 

@@ -96,8 +96,9 @@ typedef struct glint_config {
     uint64_t kv_restriction;       /* 0 -> G_bytes*2^25 keys (util/config.h:80) */
     uint64_t kv_capacity;          /* key buffer; 0 -> kv_restriction + max(1000000, 4*num_objects)
                                       (util/config.h:81 adds 1000000) */
-    uint32_t use_graph;            /* 1: capture the step once as a CUDA graph and replay it (device
-                                      input buffer only; per-stage timing off) */
+    uint32_t use_graph;            /* 1: the step is captured as a CUDA graph from the first step on and
+                                      capturing must succeed (per-stage timing off); 0: from the second
+                                      untimed step on, launched kernel by kernel where it cannot be */
     uint32_t store_host_keep;      /* further blocks kept in page-locked host memory, which the GPU reads
                                       over the host link: the oldest device-kept block moves there when
                                       a new one arrives beyond store_keep; 0 -> none */
@@ -582,8 +583,8 @@ glint_status glint_precision_probe(glint_ctx *ctx, uint32_t stride, glint_precis
  * as one CUDA graph captured at the first step: every region's stages up to
  * the refine stage, one refine launch over the work items of all regions in
  * precision_mode 1 (regions in mode 0 refine on their own streams), then
- * every region's remaining stages.  Keep the same buffers so the graph is
- * reused; it is captured again when a pointer changes.  The call returns
+ * every region's remaining stages.  The graph takes the points' addresses when
+ * it runs, so they may change from call to call.  The call returns
  * without waiting (after the previous timestep is done); glint_batch_sync
  * waits for it and runs each region's automatic flush, filling stats[r] when
  * stats is not NULL.  glint_batch_region gives a region's context for its

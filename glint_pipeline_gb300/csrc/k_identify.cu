@@ -24,8 +24,8 @@
  * every lane busy and kIdIlp records per lane in flight.  Stamps are changed
  * in shared memory and written back as whole 16-byte words.  Walking in order
  * took 9.0 + 0.85 ms (pass 1 + pass 2) at 10M objects, 2^30 buckets 27% full,
- * 1410 + 227 us at 2M in dense spots, 2^28 buckets; the lists take 7.8 + 0.41
- * ms and 1097 + 109 us.
+ * 1410 + 227 us at 2M in dense spots, 2^28 buckets; the lists take 7.7 + 0.43
+ * ms (6.5 TB/s of DRAM traffic, the copy's rate) and 1016 + 115 us.
  */
 #include "glint_internal.cuh"
 
@@ -34,7 +34,10 @@ namespace glint {
 constexpr int kIdThreads = 256;
 constexpr int kIdWarps = kIdThreads / 32;
 constexpr uint8_t kStampEmit = 4;
-constexpr int kIdIlp = 4;
+/* Records per lane in flight: with full lanes two are enough, and the registers
+ * they save hold 40 warps per SM instead of 32 (four: 171 us at 1M objects, 2^26
+ * buckets; two: 147; one: 145; two and spans of 512 or 2048: 148 and 192) */
+constexpr int kIdIlp = 2;
 
 /* Buckets per warp.  1024 amortises a block's start over many records; a
  * small table (below 2^23 buckets) would then be a handful of blocks, each

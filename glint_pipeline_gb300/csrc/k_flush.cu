@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(256) k_keys_append(const glint_meeting *__rest
         }
         const float4 box = make_float4(m.mbr[0], m.mbr[1], m.mbr[2], m.mbr[3]);
         const uint32_t l0 = f2u_coord(box.x), l1 = f2u_coord(box.y), h0 = f2u_coord(box.z), h1 = f2u_coord(box.w);
+        const uint4 have0 = __ldcg(&a.obox[pid]), have1 = __ldcg(&a.obox[target]);
         for (int k = 0; k < 2; ++k) {
             if (k == 1) {
                 const uint32_t t = pid;
@@ -128,11 +129,15 @@ __global__ void __launch_bounds__(256) k_keys_append(const glint_meeting *__rest
                               (u128)(uint32_t)(m.end - end_time_min);
             a.boxes[idx + k] = box;
             atomicAdd(&a.same[pid], 1u); /* objects with keys are counted at the flush */
+            /* the object's box only grows: a bound that the box as read
+             * already covers needs no atomic (most do once an object has a
+             * few keys in the window) */
             uint32_t *o = reinterpret_cast<uint32_t *>(&a.obox[pid]);
-            atomicMin(&o[0], l0);
-            atomicMin(&o[1], l1);
-            atomicMax(&o[2], h0);
-            atomicMax(&o[3], h1);
+            const uint4 have = k == 0 ? have0 : have1;
+            if (l0 < have.x) atomicMin(&o[0], l0);
+            if (l1 < have.y) atomicMin(&o[1], l1);
+            if (h0 > have.z) atomicMax(&o[2], h0);
+            if (h1 > have.w) atomicMax(&o[3], h1);
         }
     }
 }

@@ -130,7 +130,13 @@ struct StoreBlock {
                                               end_time_max: a query window outside both finds nothing */
     bool spans_known = false;              /* start_min and end_time_max were taken from the keys here
                                               (flushed or merged blocks; not blocks read from files) */
+    void *slab = nullptr;                  /* the one allocation that holds all its arrays (store_block_alloc),
+                                              returned in the order of slab_stream */
+    cudaStream_t slab_stream = nullptr;
 };
+/* b's device arrays for key_bytes of packed keys, C CTFs (C + 1 index entries)
+ * and o_n oversize keys, in one allocation of the context's block pool */
+cudaError_t store_block_alloc(glint_ctx *c, StoreBlock &b, size_t key_bytes, uint32_t C, uint64_t o_n);
 void store_block_release(StoreBlock &b);
 /* the kept blocks after one was added: the oldest device blocks beyond
  * store_keep move to host memory while fewer than store_host_keep are
@@ -263,6 +269,8 @@ struct glint_ctx {
     uint32_t flushes = 0;
     std::vector<glint::StoreBlock> ctbs;   /* flushed blocks kept for queries, oldest first */
     cudaMemPool_t compact_pool = nullptr;  /* compaction scratch; stays mapped between merges */
+    cudaMemPool_t store_pool = nullptr;    /* kept blocks; holds a dropped block's memory for the next */
+    uint64_t store_pool_keep = 0;          /* bytes it may hold between flushes */
     glint_server *server = nullptr;        /* the default server behind glint_query_batch */
     std::vector<glint_server *> servers;   /* every live server on this context */
     cudaEvent_t flush_ev[2];

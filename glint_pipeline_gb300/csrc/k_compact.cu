@@ -42,7 +42,6 @@ namespace {
 
 constexpr int kOidBit = 26;                  /* OID_BIT, util/util.h:49 */
 constexpr uint64_t kBitBytes = 256 * 256 / 8; /* one CTF's bitmap slot */
-constexpr unsigned long long kExtraFlag = 1ull << 52;
 constexpr uint64_t kCellLoopMax = 1ull << 20;
 
 typedef unsigned __int128 u128;
@@ -71,7 +70,8 @@ enum : uint32_t {
     kExtraCount = 3,  /* keys for the extra oversize list */
     kNoSid = 4,       /* source oversize keys without sid bits */
     kExtraOrder = 5,  /* the extra list out of full-key order */
-    kNumCounters = 6
+    kOversizeObjects = 6,
+    kNumCounters = 7
 };
 
 __device__ inline uint32_t last_le(const unsigned long long *a, uint32_t n, unsigned long long v) {
@@ -112,7 +112,10 @@ __global__ void __launch_bounds__(256) k_cmp_parse(const SrcBlock *__restrict__ 
                                                    uint32_t N, const float *__restrict__ tf,
                                                    const double *__restrict__ td, Rec *__restrict__ recs,
                                                    unsigned long long *__restrict__ skey, uint32_t *__restrict__ sval,
-                                                   unsigned long long *__restrict__ counters) {
+                                                   int oid_bits, unsigned long long *__restrict__ counters) {
+    /* sort keys (extra, oid, target), as many bits as N's ids have: 48 at 2M
+     * objects, one radix pass less than the 53 of the largest */
+    const unsigned long long extra_flag = 1ull << (kOidBit + oid_bits);
     for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < R; g += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t i = 0;
         while (i + 1 < nsrc && src[i + 1].base <= g) ++i;
@@ -156,12 +159,12 @@ __global__ void __launch_bounds__(256) k_cmp_parse(const SrcBlock *__restrict__ 
         sval[g] = (uint32_t)g;
         if (r.oid >= N || r.target >= (1u << kOidBit)) {
             atomicAdd(&counters[kErrOid], 1ull);
-            skey[g] = kExtraFlag | ((unsigned long long)((1u << kOidBit) - 1) << kOidBit);
+            skey[g] = extra_flag;
             continue;
         }
         const bool extra = b.sids[r.oid] == 1;
         if (extra) atomicAdd(&counters[kExtraCount], 1ull);
-        skey[g] = (extra ? kExtraFlag : 0ull) | ((unsigned long long)r.oid << kOidBit) | r.target;
+        skey[g] = (extra ? extra_flag : 0ull) | ((unsigned long long)r.oid << kOidBit) | r.target;
     }
 }
 
@@ -567,6 +570,16 @@ __global__ void k_cmp_orun_index(const ulonglong2 *__restrict__ okeys, uint64_t 
     }
 }
 
+/* objects whose keys are in the oversize buffer (sid 1); counting them on the
+ * host cost a copy of the sids and a loop over the objects, 2 ms at 2M */
+__global__ void __launch_bounds__(256) k_cmp_count_oversize(const uint16_t *__restrict__ sids, uint32_t N,
+                                                            unsigned long long *n) {
+    uint32_t v = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) v += sids[i] == 1;
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(n, (unsigned long long)v);
+}
+
 __global__ void k_cmp_obitmap(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kBitBytes / 4; i += gridDim.x * blockDim.x)
         dst[i] |= src[i];
@@ -719,8 +732,9 @@ extern "C" glint_status glint_store_compact(glint_ctx *c, uint32_t first, uint32
     cudaMemsetAsync(rend, 0, sizeof(uint32_t) * N, s);
 
     /* parse and order the keys */
-    if (R) k_cmp_parse<<<grid_for(R, 256), 256, 0, s>>>(d_src, count, R, N, tf, td, recs, skey, sval, d_cnt);
-    if ((e = radix_sort_u64(skey, sval, skey2, sval2, R, 53, rs_tmp, scan_tmp, s)) != cudaSuccess)
+    const int oid_bits = std::max(1, radix_bits_for(N - 1));
+    if (R) k_cmp_parse<<<grid_for(R, 256), 256, 0, s>>>(d_src, count, R, N, tf, td, recs, skey, sval, oid_bits, d_cnt);
+    if ((e = radix_sort_u64(skey, sval, skey2, sval2, R, kOidBit + oid_bits + 1, rs_tmp, scan_tmp, s)) != cudaSuccess)
         return cuda_fail(e, "key sort");
     unsigned long long hc[kNumCounters];
     if ((e = cudaMemcpyAsync(hc, d_cnt, sizeof(hc), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
@@ -848,21 +862,7 @@ extern "C" glint_status glint_store_compact(glint_ctx *c, uint32_t first, uint32
 
     /* the new block */
     StoreBlock nb;
-    cudaError_t ae = cudaSuccess;
-    auto A = [&](void **p, size_t n) {
-        if (ae == cudaSuccess) ae = cudaMalloc(p, n ? n : 1);
-    };
-    A((void **)&nb.keys, KB);
-    A((void **)&nb.ctfs, sizeof(glint_ctf_meta) * S2);
-    A((void **)&nb.key_index, sizeof(unsigned long long) * (S2 + 1));
-    A((void **)&nb.byte_index, sizeof(unsigned long long) * (S2 + 1));
-    A((void **)&nb.sids, sizeof(uint16_t) * N);
-    A((void **)&nb.first, sizeof(uint32_t) * N);
-    A((void **)&nb.count, sizeof(uint32_t) * N);
-    A((void **)&nb.okeys, sizeof(ulonglong2) * O);
-    A((void **)&nb.oboxes, sizeof(float4) * O);
-    A((void **)&nb.bitmaps, (size_t)S2 * kBitBytes);
-    A((void **)&nb.obitmap, kBitBytes);
+    const cudaError_t ae = store_block_alloc(c, nb, KB, S2, O);
     if (ae != cudaSuccess) {
         store_block_release(nb);
         return cuda_fail(ae, "new block");
@@ -992,6 +992,7 @@ extern "C" glint_status glint_store_compact(glint_ctx *c, uint32_t first, uint32
         k_cmp_orun_first<<<grid_for(O, 256), 256, 0, s>>>(nb.okeys, O, N, ofirst);
         k_cmp_orun_index<<<grid_for(N, 256), 256, 0, s>>>(nb.okeys, O, N, nsids, ofirst, nb.first, nb.count);
     }
+    k_cmp_count_oversize<<<grid_for(N, 256, 152u * 4u), 256, 0, s>>>(nsids, N, d_cnt + kOversizeObjects);
     for (uint32_t i = 0; i < count; ++i)
         k_cmp_obitmap<<<2, 1024, 0, s>>>(reinterpret_cast<const uint32_t *>(c->ctbs[first + i].obitmap),
                                          reinterpret_cast<uint32_t *>(nb.obitmap));
@@ -1008,11 +1009,6 @@ extern "C" glint_status glint_store_compact(glint_ctx *c, uint32_t first, uint32
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ev.a, ev.b);
 
-    std::vector<uint16_t> hsids(N);
-    if ((e = cudaMemcpy(hsids.data(), nsids, sizeof(uint16_t) * N, cudaMemcpyDeviceToHost)) != cudaSuccess) {
-        store_block_release(nb);
-        return cuda_fail(e, "sids");
-    }
     nb.kv = KV;
     nb.o_count = O;
     nb.key_bytes = KB;
@@ -1022,7 +1018,7 @@ extern "C" glint_status glint_store_compact(glint_ctx *c, uint32_t first, uint32
     std::memcpy(nb.o_times, ot, sizeof(ot));
     std::memcpy(nb.rec_times, rec, sizeof(rec));
     nb.sid_count = split;
-    for (uint32_t o = 0; o < N; ++o) nb.oversize_oid_count += hsids[o] == 1;
+    nb.oversize_oid_count = (uint32_t)hc[kOversizeObjects];
     nb.start_min = c->ctbs[first].start_min;
     nb.spans_known = true;
     for (uint32_t i = 0; i < count; ++i) {

@@ -53,7 +53,20 @@ constexpr uint32_t kBitEdge = 256;     /* DEFAULT_bitmap_edge, util/util.h:47 */
 constexpr uint64_t kBitCount = (uint64_t)kBitEdge * kBitEdge;
 constexpr uint32_t kSegWarpMax = 256;
 constexpr uint32_t kSegBlockMax = 8192;
-constexpr unsigned long long kGroupNone = 2ull << 40;
+/* the classes that order the objects' key segments: a CTF's objects by its
+ * sid (at most 64^2 + 1), then the oversize part's, then those without keys */
+constexpr unsigned long long kGroupOver = 1ull << 14, kGroupNone = 2ull << 14;
+constexpr int kGroupBits = 16;
+
+/* The STR sorts' keys: an object's mean position as (x << y_bits | y), x and y
+ * counted from just below the map's low corner, so that the keys are as short
+ * as the map allows (34 bits for 40 km instead of the reference's 64): the
+ * order is the reference's.  Only objects whose keys' boxes lie inside the map
+ * have one, and none is 0, which the objects without stand first with. */
+struct MidFrame {
+    uint32_t x0, y0;
+    int x_bits, y_bits;
+};
 
 typedef unsigned __int128 u128;
 
@@ -151,7 +164,7 @@ __global__ void k_init_obox(uint4 *obox, uint32_t N) {
  * the oversize buffer (partition, :1784-1797) */
 __global__ void __launch_bounds__(256) k_set_oid(uint32_t N, const uint32_t *__restrict__ same,
                                                  const uint4 *__restrict__ obox, uint16_t *__restrict__ sids,
-                                                 double dprob, uint32_t *__restrict__ oids,
+                                                 double dprob, MidFrame mf, uint32_t *__restrict__ oids,
                                                  unsigned long long *__restrict__ mid, uint8_t *__restrict__ over,
                                                  DevCounters *cnt) {
     uint32_t with_keys = 0;
@@ -169,7 +182,7 @@ __global__ void __launch_bounds__(256) k_set_oid(uint32_t N, const uint32_t *__r
             } else {
                 const uint32_t ave_mid0 = o.x / 2 + o.z / 2;
                 const uint32_t ave_mid1 = o.w / 2 + o.w / 2; /* high[1] twice, as the reference */
-                m = ((unsigned long long)ave_mid0 << 32) + ave_mid1;
+                m = ((unsigned long long)(ave_mid0 - mf.x0) << mf.y_bits) | (ave_mid1 - mf.y0);
             }
         }
         mid[id] = m;
@@ -188,7 +201,7 @@ __global__ void k_mark_over(uint32_t N, const uint16_t *__restrict__ sids, uint8
 /* narrow_xy_to_y (:771-778) + the per-slice sort keys (:1881-1890): slice
  * index + 1 above the y half, 0 for the objects before the slices */
 __global__ void k_str_slice_keys(unsigned long long *__restrict__ mid, uint32_t N, uint32_t zero_one, uint32_t x_part,
-                                 uint32_t split) {
+                                 uint32_t split, int y_bits) {
     for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
         if (id < zero_one) {
             mid[id] = 0;
@@ -196,7 +209,7 @@ __global__ void k_str_slice_keys(unsigned long long *__restrict__ mid, uint32_t 
         }
         uint32_t part = (id - zero_one) / x_part;
         if (part > split - 1) part = split - 1;
-        mid[id] = ((unsigned long long)(part + 1) << 32) | (mid[id] & 0xffffffffull);
+        mid[id] = ((unsigned long long)(part + 1) << y_bits) | (mid[id] & ((1ull << y_bits) - 1));
     }
 }
 
@@ -219,7 +232,7 @@ __global__ void k_group_keys(uint32_t N, const uint32_t *__restrict__ same, cons
     for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < N; id += gridDim.x * blockDim.x) {
         unsigned long long k = kGroupNone;
         if (same[id]) {
-            k = over[id] ? ((1ull << 40) | id) : (((unsigned long long)sids[id] << kOidBit) | id);
+            k = over[id] ? kGroupOver : sids[id]; /* ids ascend, and the sort is stable */
         }
         gk[id] = k;
         gv[id] = id;
@@ -238,8 +251,8 @@ __global__ void k_group_starts(uint32_t N, const unsigned long long *__restrict_
                                unsigned long long *__restrict__ main_count) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         seg_of[gv[i]] = start[i];
-        const bool is_main = gk[i] < (1ull << 40);
-        const bool next_main = i + 1 < N && gk[i + 1] < (1ull << 40);
+        const bool is_main = gk[i] < kGroupOver;
+        const bool next_main = i + 1 < N && gk[i + 1] < kGroupOver;
         if (is_main && !next_main) *main_count = start[i + 1];
         if (i == 0 && !is_main) *main_count = 0;
     }
@@ -858,6 +871,28 @@ void flush_set_attributes() {
                          (int)(kSegBlockMax * (sizeof(u128) + sizeof(uint32_t))));
 }
 
+/* float_to_uint of a coordinate, on the host (f2u_coord) */
+static uint32_t h_f2u(float xy) {
+    const float t = (xy + 180.0f) * 100000.0f;
+    if (!(t > 0.0f)) return 0;
+    return t >= 4294967296.0f ? 0xffffffffu : (uint32_t)t;
+}
+
+/* The bounds of the mean positions: a key's box is two f32 corners inside the
+ * map, f2u_coord does not decrease, and a mean of halves a / 2 + b / 2 of values
+ * in [lo, hi] is in [lo - 1, hi]. */
+static MidFrame mid_frame(const glint_box &map) {
+    uint32_t base[2];
+    int bits[2];
+    for (int k = 0; k < 2; ++k) {
+        const uint32_t lo = h_f2u(std::nextafterf((float)map.low[k], -INFINITY));
+        const uint32_t hi = h_f2u(std::nextafterf((float)map.high[k], INFINITY));
+        base[k] = lo >= 2 ? lo - 2 : 0;
+        bits[k] = std::max(1, radix_bits_for(hi >= base[k] ? hi - base[k] : 0xffffffffu));
+    }
+    return MidFrame{base[0], base[1], bits[0], bits[1]};
+}
+
 /* the whole flush on the context's stream; host synchronisation where the
  * reference's own flush reads counts back */
 glint_status run_flush(glint_ctx *c, glint_store_info *info, std::string &err) {
@@ -870,8 +905,9 @@ glint_status run_flush(glint_ctx *c, glint_store_info *info, std::string &err) {
         return e == cudaErrorMemoryAllocation ? GLINT_ERR_OUT_OF_MEMORY : GLINT_ERR_CUDA;
     };
     cudaError_t e;
+    const MidFrame mf = mid_frame(c->mbr);
     /* set_oid and the area cut */
-    k_set_oid<<<grid_for(N, 256), 256, 0, s>>>(N, c->d_same, c->d_obox, c->d_sids, c->cfg.dProbFalse, c->d_oids,
+    k_set_oid<<<grid_for(N, 256), 256, 0, s>>>(N, c->d_same, c->d_obox, c->d_sids, c->cfg.dProbFalse, mf, c->d_oids,
                                                 c->d_mid, c->d_over, c->d_cnt);
     k_mark_over<<<grid_for(N, 256), 256, 0, s>>>(N, c->d_sids, c->d_over);
     if ((e = cudaMemcpyAsync(&h, c->d_cnt, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
@@ -894,13 +930,14 @@ glint_status run_flush(glint_ctx *c, glint_store_info *info, std::string &err) {
     /* d_ctf_keys needs no clearing: the packing writes every byte of the
      * key_bytes it holds, and nothing reads past them */
 
-    /* STR: by mean x (full 64-bit key), then by y inside each x-slice */
-    if ((e = radix_sort_u64(c->d_mid, c->d_oids, c->d_mid2, c->d_oids2, N, 64, c->d_rs_tmp, c->d_scan_tmp, s)))
+    /* STR: by mean x (then y), then by y inside each x-slice */
+    if ((e = radix_sort_u64(c->d_mid, c->d_oids, c->d_mid2, c->d_oids2, N, mf.x_bits + mf.y_bits,
+                            c->d_rs_tmp, c->d_scan_tmp, s)))
         return fail(e, "STR x sort");
     if (zero_one < N) {
-        k_str_slice_keys<<<grid_for(N, 256), 256, 0, s>>>(c->d_mid, N, zero_one, x_part, split);
-        int bits = 33;
-        while ((1ull << (bits - 32)) <= split) ++bits;
+        k_str_slice_keys<<<grid_for(N, 256), 256, 0, s>>>(c->d_mid, N, zero_one, x_part, split, mf.y_bits);
+        int bits = mf.y_bits + 1;
+        while ((1ull << (bits - mf.y_bits)) <= split) ++bits;
         if ((e = radix_sort_u64(c->d_mid, c->d_oids, c->d_mid2, c->d_oids2, N, bits, c->d_rs_tmp, c->d_scan_tmp, s)))
             return fail(e, "STR y sort");
         k_make_sid<<<grid_for(N, 256), 256, 0, s>>>(c->d_oids, N, zero_one, x_part, split, c->d_sids);
@@ -910,7 +947,7 @@ glint_status run_flush(glint_ctx *c, glint_store_info *info, std::string &err) {
     unsigned long long *gk = c->d_mid;  /* the STR keys are no longer needed */
     uint32_t *gv = c->d_oids2;
     k_group_keys<<<grid_for(N, 256), 256, 0, s>>>(N, c->d_same, c->d_sids, c->d_over, gk, gv);
-    if ((e = radix_sort_u64(gk, gv, c->d_mid2, c->d_segbig, N, 42, c->d_rs_tmp, c->d_scan_tmp, s)))
+    if ((e = radix_sort_u64(gk, gv, c->d_mid2, c->d_segbig, N, kGroupBits, c->d_rs_tmp, c->d_scan_tmp, s)))
         return fail(e, "object order");
     k_group_counts<<<grid_for(N, 256), 256, 0, s>>>(N, gk, gv, c->d_same, c->d_gcount);
     scan_u32(c->d_gcount, c->d_gstart, N, c->d_scan_tmp, s);
@@ -1034,22 +1071,7 @@ glint_status run_flush(glint_ctx *c, glint_store_info *info, std::string &err) {
     /* keep the block on the device for queries */
     if (c->cfg.store_keep) {
         StoreBlock b;
-        const size_t bytes_keys = bytes ? bytes : 1;
-        cudaError_t ae = cudaSuccess;
-        auto A = [&](void **p, size_t n) {
-            if (ae == cudaSuccess) ae = cudaMalloc(p, n ? n : 1);
-        };
-        A((void **)&b.keys, bytes_keys);
-        A((void **)&b.ctfs, sizeof(glint_ctf_meta) * C);
-        A((void **)&b.key_index, sizeof(unsigned long long) * C);
-        A((void **)&b.byte_index, sizeof(unsigned long long) * C);
-        A((void **)&b.sids, sizeof(uint16_t) * N);
-        A((void **)&b.first, sizeof(uint32_t) * N);
-        A((void **)&b.count, sizeof(uint32_t) * N);
-        A((void **)&b.okeys, sizeof(ulonglong2) * o_n);
-        A((void **)&b.oboxes, sizeof(float4) * o_n);
-        A((void **)&b.bitmaps, (size_t)C * kBitCount / 8);
-        A((void **)&b.obitmap, kBitCount / 8);
+        cudaError_t ae = store_block_alloc(c, b, bytes, C, o_n);
         if (ae != cudaSuccess) {
             store_block_release(b);
             return fail(ae, "keep block");
@@ -1140,6 +1162,7 @@ extern "C" glint_status glint_serve_only(glint_ctx *c, uint64_t reserve, uint32_
             if (*p) cudaFree(*p);
             *p = nullptr;
         }
+        if (c->store_pool) cudaMemPoolTrimTo(c->store_pool, 0);
         c->serve_only = true;
         c->store_valid = false;
         c->stats_valid = false;
@@ -1241,7 +1264,62 @@ extern "C" glint_status glint_store_read(glint_ctx *c, uint8_t *keys, uint16_t *
 }
 
 namespace glint {
+/* A flush allocated eleven arrays and freed eleven of the block it dropped,
+ * each with its own mapping and device-wide wait (2M objects, 7M keys: 2.25 ms a
+ * flush with them, 2.05 without); so did a merge (7.0 ms for 22M keys in three
+ * blocks, 4.9 with one allocation of a pool and the oversize objects counted on
+ * the device).  What the pool keeps of dropped blocks is
+ * bounded by what flushes and merges hold for a moment anyway;
+ * glint_serve_only empties it and it goes with the context. */
+cudaError_t store_block_alloc(glint_ctx *c, StoreBlock &b, size_t key_bytes, uint32_t C, uint64_t o_n) {
+    cudaError_t e = cudaSuccess;
+    if (!c->store_pool) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->device;
+        if ((e = cudaMemPoolCreate(&c->store_pool, &props)) != cudaSuccess) {
+            c->store_pool = nullptr;
+            return e;
+        }
+    }
+    const size_t N = c->N;
+    void **fields[] = {(void **)&b.keys, (void **)&b.ctfs, (void **)&b.key_index, (void **)&b.byte_index,
+                       (void **)&b.sids, (void **)&b.first, (void **)&b.count, (void **)&b.okeys,
+                       (void **)&b.oboxes, (void **)&b.bitmaps, (void **)&b.obitmap};
+    const size_t bytes[] = {key_bytes, sizeof(glint_ctf_meta) * C, sizeof(unsigned long long) * (C + 1),
+                            sizeof(unsigned long long) * (C + 1), sizeof(uint16_t) * N, sizeof(uint32_t) * N,
+                            sizeof(uint32_t) * N, sizeof(ulonglong2) * o_n, sizeof(float4) * o_n,
+                            (size_t)C * kBitCount / 8, kBitCount / 8};
+    constexpr int F = sizeof(bytes) / sizeof(bytes[0]);
+    auto padded = [](size_t n) { return (std::max<size_t>(n, 1) + 255) / 256 * 256; };
+    size_t total = 0;
+    for (size_t n : bytes) total += padded(n);
+    /* what the pool may hold: its blocks, and beyond them twice the largest so
+     * far (the sources of a merge are about its result) */
+    c->store_pool_keep = std::max<uint64_t>(c->store_pool_keep, 2 * total);
+    uint64_t used = 0;
+    cudaMemPoolGetAttribute(c->store_pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    uint64_t keep = used + total + c->store_pool_keep;
+    cudaMemPoolSetAttribute(c->store_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    uint8_t *p = nullptr;
+    if ((e = cudaMallocFromPoolAsync((void **)&p, total, c->store_pool, c->stream)) != cudaSuccess) return e;
+    b.slab = p;
+    b.slab_stream = c->stream;
+    for (int i = 0; i < F; ++i) {
+        *fields[i] = p;
+        p += padded(bytes[i]);
+    }
+    return cudaSuccess;
+}
+
 void store_block_release(StoreBlock &b) {
+    if (b.slab) {
+        cudaFreeAsync(b.slab, b.slab_stream);
+        b = StoreBlock();
+        return;
+    }
     void *ps[] = {b.keys,  b.ctfs,  b.key_index, b.byte_index, b.sids,   b.first,
                   b.count, b.okeys, b.oboxes,    b.bitmaps,    b.obitmap};
     for (void *p : ps)
@@ -1290,9 +1368,11 @@ static cudaError_t block_to_host(glint_ctx *c, StoreBlock &b, bool &moved) {
         return e;
     }
     for (int i = 0; i < F; ++i) {
-        if (*fields[i]) cudaFree(*fields[i]);
+        if (*fields[i] && !b.slab) cudaFree(*fields[i]);
         *fields[i] = host[i];
     }
+    if (b.slab) cudaFreeAsync(b.slab, b.slab_stream);
+    b.slab = nullptr;
     b.on_host = true;
     moved = true;
     return cudaSuccess;

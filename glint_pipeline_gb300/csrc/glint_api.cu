@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(64) k_step_tail(uint32_t N, const uint32_t *re
 }
 
 void free_all(glint_ctx *c) {
-    void *ptrs[] = {c->d_pts, c->d_in, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_obj, c->d_grid_count,
+    void *ptrs[] = {c->d_pts, c->d_in, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_cbox, c->d_obj, c->d_grid_count,
                     c->d_grid_start, c->d_sorted, c->d_rank, c->d_sxy, c->d_sm, c->d_leaf_work,
                     c->d_nodes, c->d_low, c->d_sstack, c->d_gstack, c->d_split, c->d_evscan, c->d_cand, c->d_newgid,
                     c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
@@ -426,6 +426,7 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     ALLOC(c->d_nodes, S);
     ALLOC(c->d_low, S);
     ALLOC(c->d_ibox, S);
+    ALLOC(c->d_cbox, 4 * (size_t)S);
     ALLOC(c->d_sstack, S);
     ALLOC(c->d_gstack, G);
     ALLOC(c->d_split, (size_t)S + 4);
@@ -568,6 +569,7 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     SinCoef coef;
     init_sin_coef(&coef);
     cudaMemcpy(c->d_coef, &coef, sizeof(coef), cudaMemcpyHostToDevice);
+    launch_child_boxes(c);
     k_fill_empty<<<grid_for(c->B, 256, 152u * 16u), 256, 0, c->stream>>>(c->d_tab, c->B);
     cudaMemsetAsync(c->d_scan_tmp, 0, c->scan_tmp_bytes, c->stream);
     cudaMemsetAsync(c->d_scan_tmp_side, 0, c->scan_tmp_bytes, c->stream);

@@ -446,6 +446,12 @@ __host__ __device__ inline IBox fx_box(double lx, double ly, double hx, double h
     return b;
 }
 
+/* a box in FP32 units; a coordinate beyond fx_to_f's range is NaN, which a
+ * comparison leaves undecided */
+__device__ inline float4 f_box(const IBox &b) {
+    return make_float4(fx_to_f(b.x), fx_to_f(b.y), fx_to_f(b.z), fx_to_f(b.w));
+}
+
 /* box distance screening: the gap from the point to the box along each axis */
 __device__ inline int fx_box_screen(const IBox &b, long long px, long long py, const Screen &s, float cy) {
     const long long x1 = b.x - px, x2 = px - b.z, y1 = b.y - py, y2 = py - b.w;

@@ -204,6 +204,7 @@ struct glint_ctx {
     float *d_sc = nullptr;                 /* [N] sorted metres per unit along x */
     float2 *d_fpos = nullptr;              /* [N] f32 coordinates by object id */
     glint::IBox *d_ibox = nullptr;           /* [S] fixed-point node boxes */
+    float4 *d_cbox = nullptr;              /* [4 S] a branch's children's boxes in FP32 units */
     glint::Frame frame;
     uint32_t *d_leaf_work = nullptr;       /* [G] grid ids with objects */
 
@@ -319,6 +320,8 @@ void init_sin_coef(SinCoef *host);
 cudaError_t launch_step_begin(glint_ctx *c, bool from_host);
 cudaError_t launch_partition(glint_ctx *c);
 cudaError_t launch_filter(glint_ctx *c);
+/* the children's boxes of every branch, from the schema as it stands */
+cudaError_t launch_child_boxes(glint_ctx *c);
 cudaError_t launch_refine_pairs(glint_ctx *c);
 struct RefineArgs;
 RefineArgs refine_args(glint_ctx *c);

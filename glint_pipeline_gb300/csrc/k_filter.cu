@@ -12,19 +12,21 @@
  * in object order and, per object, in walk order.
  *
  * Device form: one thread per border object, objects visited in leaf-major
- * order so that neighbouring threads walk the same nodes.  A node is opened
- * once: its four children's boxes are requested together and tested, and the
- * ones to visit go on a stack in reverse order, so that they come off in the
- * reference's.  A branch whose top is below the object is not opened: nothing
- * under it can be kept.  The walk reserves the object's place in the check
- * list and counts its checks by target leaf (which gives each its place there)
- * as it ends; after a scan of those counts the checks are copied, grouped by
- * target leaf, for the refine tiles.  The list by querier stays for the
+ * order so that neighbouring threads walk the same nodes.  A node that comes off
+ * the walk's stack is tested, kept or opened from words that are all requested
+ * at once: its own, and its children's boxes in FP32, which rule out most of
+ * the children; the others go on the stack in reverse order, so that they come
+ * off in the reference's.  A node whose top is below the object is not opened:
+ * nothing under it can be kept.  The walk reserves the object's place in the
+ * check list and counts its checks by target leaf (which gives each its place
+ * there) as it ends; after a scan of those counts the checks are copied, grouped
+ * by target leaf, for the refine tiles.  The list by querier stays for the
  * duplicate rule in refine.
  *
- * Bound: the chain of dependent loads from node to child.  Testing one child
- * at a time took 125 us at 1M objects (29 us at 20k, for 3k border objects);
- * opening nodes takes 113 (17).
+ * Bound: the chain of dependent loads from node to child.  Testing one child at
+ * a time, a load for its id and one for its words, took 125 us at 1M objects (29
+ * us at 20k, for 3k border objects); four children at a time 105 (17.6), a node
+ * in one load 92 (15.1).  10M: 1.72, 1.28 and 1.24 ms.
  */
 #include <cmath>
 
@@ -35,7 +37,7 @@ namespace glint {
 constexpr int kQInline = 8;
 /* 64 levels, each of which leaves at most three children waiting */
 constexpr int kStackMax = 200;
-constexpr uint32_t kKeptLeaf = 0x80000000u;
+constexpr uint32_t kWalkStart = 0x80000000u; /* the node a walk starts from is opened untested */
 
 /* the querier of a walk: exact coordinates (for the top/right rule and the
  * exact fallback), fixed-point coordinates and screening limits */
@@ -43,6 +45,9 @@ struct WalkPoint {
     double px, py;
     long long X, Y;
     Screen sc;
+    float fx, fy;        /* X, Y in FP32 */
+    float rx, ry;        /* farther than this along an axis is out of reach, whatever FP32 rounded away */
+    float top;           /* a box that ends below this ends below the object */
 };
 
 __device__ inline WalkPoint walk_point(const double2 p, const longlong2 ip, float c, const Frame &f) {
@@ -52,6 +57,16 @@ __device__ inline WalkPoint walk_point(const double2 p, const longlong2 ip, floa
     w.X = ip.x;
     w.Y = ip.y;
     w.sc = make_screen(c, f);
+    /* FP32 holds a coordinate to 2^-24 of itself (1.2 mm in a map of 40 km): a
+     * gap of about the reach is off by less than 2^-22 of the coordinate and
+     * two units */
+    w.fx = fx_to_f(ip.x);
+    w.fy = fx_to_f(ip.y);
+    const float r = sqrtf(f.r2) * 1.0001f;
+    const float ex = 4.f + 2.4e-7f * (fabsf(w.fx) + r / c), ey = 4.f + 2.4e-7f * (fabsf(w.fy) + r / f.cy);
+    w.rx = r / c + ex;
+    w.ry = r / f.cy + ey;
+    w.top = w.fy - ey;
     return w;
 }
 
@@ -79,6 +94,7 @@ struct FilterArgs {
     const DNode *nodes;
     const double2 *low;
     const IBox *ibox;
+    const float4 *cbox;
     uint32_t N;
     Frame f;
     ExactCtx ex;
@@ -93,51 +109,48 @@ struct FilterArgs {
  * keys. */
 template <class Emit>
 __device__ inline void walk_step(const FilterArgs &a, Walk &k, const WalkPoint &w, Emit emit) {
-    const uint32_t top = k.stack[--k.sp];
-    if (top & kKeptLeaf) {
-        emit(top & ~kKeptLeaf, k.kept);
-        ++k.kept;
-        return;
-    }
+    const uint32_t e = k.stack[--k.sp], top = e & ~kWalkStart;
     const uint4 chv = *reinterpret_cast<const uint4 *>(a.nodes[top].child);
-    const uint32_t ch[4] = {chv.x, chv.y, chv.z, chv.w};
-    IBox box[4];
-    uint2 tail[4]; /* gid; type, level */
+    const uint2 tail = *reinterpret_cast<const uint2 *>(&a.nodes[top].gid); /* gid; type, level */
+    const IBox box = a.ibox[top];
+    float4 fb[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        box[i] = a.ibox[ch[i]];
-        tail[i] = *reinterpret_cast<const uint2 *>(&a.nodes[ch[i]].gid);
-    }
-#pragma unroll
-    for (int i = 3; i >= 0; --i) {
-        const uint32_t type = tail[i].y & 0xffu;
+    for (int i = 0; i < 4; ++i) fb[i] = a.cbox[4 * (size_t)top + i];
+    const uint32_t type = tail.y & 0xffu;
+    if (!(e & kWalkStart)) {
         /* nothing at or above the object's latitude */
-        if (box[i].w < w.Y - 1 && (type == kLeaf || type == kBranch)) continue;
-        int in = fx_box_screen(box[i], w.X, w.Y, w.sc, a.f.cy);
+        if (box.w < w.Y - 1 && (type == kLeaf || type == kBranch)) return;
+        int in = fx_box_screen(box, w.X, w.Y, w.sc, a.f.cy);
         if (in < 0) {
             atomicAdd(&a.cnt->box_band, 1u);
-            const double2 lo = a.low[ch[i]];
-            in = box_exact(lo.x, lo.y, kdbl(a.nodes[ch[i]].khx), kdbl(a.nodes[ch[i]].khy), w.px, w.py, a.ex) ? 1 : 0;
+            const double2 lo = a.low[top];
+            in = box_exact(lo.x, lo.y, kdbl(a.nodes[top].khx), kdbl(a.nodes[top].khy), w.px, w.py, a.ex) ? 1 : 0;
         }
-        if (!in) continue;
+        if (!in) return;
         if (type == kLeaf) {
             bool keep;
-            if (w.Y < box[i].y - 1) {
+            if (w.Y < box.y - 1) {
                 keep = true;
-            } else if (w.Y > box[i].y + 1 && w.Y < box[i].w - 1 && (w.X < box[i].x - 1 || w.X > box[i].x + 1)) {
-                keep = w.X < box[i].x;
+            } else if (w.Y > box.y + 1 && w.Y < box.w - 1 && (w.X < box.x - 1 || w.X > box.x + 1)) {
+                keep = w.X < box.x;
             } else {
-                const double2 lo = a.low[ch[i]];
-                keep = dkey(w.py) < dkey(lo.y) || (dkey(w.py) < a.nodes[ch[i]].khy && dkey(w.px) < dkey(lo.x));
+                const double2 lo = a.low[top];
+                keep = dkey(w.py) < dkey(lo.y) || (dkey(w.py) < a.nodes[top].khy && dkey(w.px) < dkey(lo.x));
             }
-            if (!keep) continue;
-            if (k.sp < kStackMax) k.stack[k.sp++] = tail[i].x | kKeptLeaf;
-            else atomicOr(&a.cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
-        } else if (type == kBranch && k.sp < kStackMax) {
-            k.stack[k.sp++] = ch[i];
-        } else {
-            atomicOr(&a.cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
+            if (keep) emit(tail.x, k.kept++);
+            return;
         }
+        if (type != kBranch) {
+            atomicOr(&a.cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
+            return;
+        }
+    }
+    const uint32_t ch[4] = {chv.x, chv.y, chv.z, chv.w};
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+        if (fb[i].x - w.fx > w.rx || w.fx - fb[i].z > w.rx || fb[i].y - w.fy > w.ry || fb[i].w < w.top) continue;
+        if (k.sp < kStackMax) k.stack[k.sp++] = ch[i];
+        else atomicOr(&a.cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
     }
 }
 
@@ -192,7 +205,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, C
             lv = a.obj[pid].y;
             w = walk_point(a.sxy[i], a.sipos[i], a.sc[i], a.f);
             k.sp = 1;
-            k.stack[0] = lv;
+            k.stack[0] = lv | kWalkStart;
             while (k.sp > 0)
                 walk_step(a, k, w, [&](uint32_t gid, uint32_t j) {
                     if (j < (uint32_t)kQInline) row[j] = gid;
@@ -225,7 +238,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, C
                 /* the rare object with more: walked again for the rest */
                 k.sp = 1;
                 k.kept = 0;
-                k.stack[0] = lv;
+                k.stack[0] = lv | kWalkStart;
                 while (k.sp > 0)
                     walk_step(a, k, w, [&](uint32_t gid, uint32_t j) {
                         if (j >= (uint32_t)kQInline && j < n) put(gid, j);
@@ -274,6 +287,22 @@ struct TargetScan {
     }
 };
 
+__global__ void __launch_bounds__(256) k_child_boxes(const DNode *__restrict__ nodes, const IBox *__restrict__ ibox,
+                                                     uint32_t S, float4 *__restrict__ cbox) {
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
+        if (nodes[s].type != kBranch) continue;
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t ch = nodes[s].child[i];
+            if (ch < S) cbox[4 * (size_t)s + i] = f_box(ibox[ch]);
+        }
+    }
+}
+
+cudaError_t launch_child_boxes(glint_ctx *c) {
+    k_child_boxes<<<grid_for(c->S, 256), 256, 0, c->stream>>>(c->d_nodes, c->d_ibox, c->S, c->d_cbox);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_filter(glint_ctx *c) {
     cudaStream_t s = c->stream;
     const uint32_t N = c->N, G = c->G;
@@ -286,6 +315,7 @@ cudaError_t launch_filter(glint_ctx *c) {
     a.nodes = c->d_nodes;
     a.low = c->d_low;
     a.ibox = c->d_ibox;
+    a.cbox = c->d_cbox;
     a.N = N;
     a.f = c->frame;
     a.ex = make_exact(c);

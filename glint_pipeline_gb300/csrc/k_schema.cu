@@ -206,6 +206,7 @@ struct ApplyArgs {
     DNode *nodes;
     double2 *low;
     IBox *ibox;
+    float4 *cbox;
     Frame fr;
     const uint8_t *flags;
     const uint32_t *newgid;
@@ -263,7 +264,9 @@ __device__ inline void apply_split(const ApplyArgs &a, uint32_t p, const uint4 c
         c.khy = dkey(hy);
         c.kmx = dkey(__dmul_rn(__dadd_rn(lx, hx), 0.5));
         c.kmy = dkey(__dmul_rn(__dadd_rn(ly, hy), 0.5));
-        a.ibox[ch[k]] = fx_box(lx, ly, hx, hy, a.fr);
+        const IBox box = fx_box(lx, ly, hx, hy, a.fr);
+        a.ibox[ch[k]] = box;
+        a.cbox[4 * (size_t)p + k] = f_box(box);
         c.child[0] = c.child[1] = c.child[2] = c.child[3] = 0;
         c.gid = gg[k];
         c.type = kLeaf;
@@ -440,6 +443,7 @@ cudaError_t launch_schema_update(glint_ctx *c, cudaStream_t s, void *scan_tmp) {
     a.nodes = c->d_nodes;
     a.low = c->d_low;
     a.ibox = c->d_ibox;
+    a.cbox = c->d_cbox;
     a.fr = c->frame;
     a.flags = c->d_split;
     a.newgid = c->d_newgid;

@@ -429,6 +429,7 @@ extern "C" glint_status glint_snapshot_load(const char *path, int device, glint_
     }
     const bool read_ok = r.ok;
     fclose(r.f);
+    if (e == cudaSuccess && read_ok) e = launch_child_boxes(c);
     /* counters and host-side state */
     if (e == cudaSuccess && read_ok) {
         e = cudaMemcpy(c->d_cnt, &h.counters, sizeof(DevCounters), cudaMemcpyHostToDevice);

@@ -33,7 +33,6 @@ namespace glint {
 
 constexpr int kIdThreads = 256;
 constexpr int kIdWarps = kIdThreads / 32;
-constexpr uint8_t kStampEmit = 4;
 /* Records per lane in flight: with full lanes two are enough, and the registers
  * they save hold 40 warps per SM instead of 32 (four: 171 us at 1M objects, 2^26
  * buckets; two: 147; one: 145; two and spans of 512 or 2048: 148 and 192) */
@@ -68,7 +67,8 @@ __device__ inline void load_stamps(const uint8_t *stamp, uint64_t wbase, uint8_t
     __syncwarp();
 }
 
-template <uint32_t kSpan>
+/* kStamps: an entry that the step touched has its stamp, else its tag */
+template <uint32_t kSpan, bool kStamps>
 __global__ void __launch_bounds__(kIdThreads) k_expire_count(uint8_t *__restrict__ stamp,
                                                              uint32_t *__restrict__ newline,
                                                              TRec *__restrict__ tab, uint64_t B, uint32_t min_plus1,
@@ -91,17 +91,27 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_count(uint8_t *__restrict
     }
     load_stamps<kSpan>(stamp, wbase, sst[wid]);
     /* the span's buckets whose record is needed, 16 per lane at a time */
-    uint32_t n = 0;
+    uint32_t n = 0, kept = 0;
 #pragma unroll
     for (uint32_t i0 = 0; i0 < kSpan; i0 += 512) {
         const uint32_t off = i0 + lane * 16;
         uint32_t bits = 0;
         if (off < kSpan && wbase + off < B) {
             const uint4 v = *reinterpret_cast<const uint4 *>(&sst[wid][off]);
-            bits = ~(byte_bits(v.x, 0) | (byte_bits(v.y, 0) << 4) | (byte_bits(v.z, 0) << 8) | (byte_bits(v.w, 0) << 12));
-            /* every slot of a line that received a pair */
+            const uint32_t empty =
+                byte_bits(v.x, 0) | (byte_bits(v.y, 0) << 4) | (byte_bits(v.z, 0) << 8) | (byte_bits(v.w, 0) << 12);
+            bits = ~empty & 0xffffu;
+            if (kStamps) {
+                /* entries that stay need nothing of their records */
+                const uint32_t now = kStampTouched + st_now;
+                const uint32_t stay = byte_bits(v.x, now) | (byte_bits(v.y, now) << 4) | (byte_bits(v.z, now) << 8) |
+                                      (byte_bits(v.w, now) << 12);
+                kept += __popc(stay);
+                bits &= ~stay;
+            }
+            /* every empty slot of a line that received a pair */
             const uint32_t lines = (snl[wid][off >> 7] >> ((off >> 2) & 31)) & 0xfu;
-            bits |= ((lines & 1u) | ((lines & 2u) << 3) | ((lines & 4u) << 6) | ((lines & 8u) << 9)) * 0xfu;
+            bits |= ((lines & 1u) | ((lines & 2u) << 3) | ((lines & 4u) << 6) | ((lines & 8u) << 9)) * 0xfu & empty;
             const uint64_t left = B - (wbase + off);
             bits &= left < 16 ? (1u << left) - 1u : 0xffffu;
         }
@@ -116,7 +126,7 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_count(uint8_t *__restrict
         for (; bits; bits &= bits - 1) slist[wid][at++] = (uint16_t)(off + __ffs(bits) - 1);
     }
     __syncwarp();
-    uint32_t emit = 0, taken = 0, active = 0;
+    uint32_t emit = 0, taken = kept, active = kept;
     bool changed = false;
     for (uint32_t r0 = 0; r0 < n; r0 += 32 * kIdIlp) {
         uint32_t off[kIdIlp];
@@ -166,14 +176,14 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_count(uint8_t *__restrict
                     nr.mbr[0] = nr.mbr[1] = nr.mbr[2] = nr.mbr[3] = 0;
                 }
                 r = nr;
-                sst[wid][off[u]] = kStampOld;
+                sst[wid][off[u]] = kStamps ? (uint8_t)(kStampTouched + st_now) : (uint8_t)kStampOld;
                 changed = true;
                 continue;
             }
             if (sst[wid][off[u]] == kStampEmpty) continue;
             ++taken;
             const unsigned long long w1 = rec[u].y;
-            if ((uint32_t)(w1 >> 32) == st_now) {
+            if (!kStamps && (uint32_t)(w1 >> 32) == st_now) {
                 ++active;
                 continue;
             }
@@ -296,9 +306,13 @@ template <uint32_t kSpan>
 static void identify_passes(glint_ctx *c) {
     cudaStream_t s = c->stream;
     const unsigned tiles = (unsigned)c->n_tiles;
-    k_expire_count<kSpan><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_newline, c->d_tab, c->B,
-                                                       c->cfg.min_meet_time + 1, c->d_tile_cnt, c->d_fpos, c->N,
-                                                       c->d_cnt);
+    const uint32_t min_plus1 = c->cfg.min_meet_time + 1;
+    if (c->B <= kStampTouchBuckets)
+        k_expire_count<kSpan, true><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_newline, c->d_tab, c->B, min_plus1,
+                                                                 c->d_tile_cnt, c->d_fpos, c->N, c->d_cnt);
+    else
+        k_expire_count<kSpan, false><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_newline, c->d_tab, c->B, min_plus1,
+                                                                  c->d_tile_cnt, c->d_fpos, c->N, c->d_cnt);
     if (tiles <= kOwnScanTiles) {
         k_expire_emit<kSpan, true><<<tiles, kIdThreads, 0, s>>>(c->d_stamp, c->d_tab, c->d_tile_cnt, c->d_tile_off,
                                                                 c->d_log, c->log_cap, c->d_cnt);

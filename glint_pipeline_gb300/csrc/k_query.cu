@@ -21,8 +21,8 @@
  *
  * By bucket (k_search_count, k_search_emit), for the rest: the listed ids
  * become a bitmap of N bits; pass 1 reads the stamp byte of every bucket and
- * the record of occupied buckets (its tag says whether the last step touched
- * it), and counts matching sides per 8192-bucket tile; an exclusive scan gives
+ * the record of occupied buckets, and counts matching sides per 8192-bucket
+ * tile; an exclusive scan gives
  * each tile its offset; pass 2 writes the records of tiles that have any.  A
  * warp lists the occupied buckets of its span first, so that its lanes all
  * have a record to read.
@@ -48,7 +48,6 @@ struct SearchArgs {
     const TRec *tab;
     const uint8_t *stamp;
     uint64_t B;
-    uint8_t st;              /* tag of entries touched at the last step */
     uint32_t cur_time;
     uint32_t min_plus1;
     const uint32_t *bits;
@@ -67,10 +66,11 @@ __device__ inline bool listed(const SearchArgs &a, uint32_t p) {
     return p < a.N && ((a.bits[p >> 5] >> (p & 31)) & 1u);
 }
 
-/* matching sides of a record (its words w0, w1) touched at the last step: bit
- * 0 the lower id, bit 1 the higher id */
+/* matching sides of a record (its words w0, w1): bit 0 the lower id, bit 1 the
+ * higher id.  Between steps every entry of the table is active: identify took
+ * out the ones that the step did not touch. */
 __device__ inline uint32_t search_sides(const SearchArgs &a, const ulonglong2 &r) {
-    if (r.x == kEmptyW0 || (r.x & kNewFlag) || (uint32_t)(r.y >> 32) != a.st) return 0;
+    if (r.x == kEmptyW0 || (r.x & kNewFlag)) return 0;
     if (a.cur_time - (uint32_t)r.y < a.min_plus1) return 0;
     return (listed(a, pair_a(r.x)) ? 1u : 0u) | (listed(a, pair_b(r.x)) ? 2u : 0u);
 }
@@ -93,7 +93,7 @@ __device__ inline uint32_t list_occupied(const SearchArgs &a, uint64_t wbase, ui
         uint32_t bits = 0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const uint32_t m = __vcmpeq4(w[k], kStampOld * 0x01010101u) & 0x08040201u;
+            const uint32_t m = __vcmpne4(w[k], 0u) & 0x08040201u;
             bits |= ((m | (m >> 8) | (m >> 16) | (m >> 24)) & 0xfu) << (4 * k);
         }
         uint32_t incl = __popc(bits);
@@ -223,7 +223,7 @@ __device__ inline void found_contact(const ObjectSearch &o, uint32_t p, uint32_t
     for (uint32_t d = 0; d < span; ++d) {
         const ulonglong2 k = *reinterpret_cast<const ulonglong2 *>(&o.r.tab[slot]);
         if (k.x == pw) {
-            if ((uint32_t)(k.y >> 32) != o.s.st || o.s.cur_time - (uint32_t)k.y < o.s.min_plus1) return;
+            if (o.s.cur_time - (uint32_t)k.y < o.s.min_plus1) return;
             const uint32_t i = atomicAdd(o.n_found, 1u);
             if (i < kFoundMax) o.found[i] = slot * 2 + (pair_a(pw) == p ? 0u : 1u);
             return;
@@ -323,7 +323,6 @@ SearchArgs search_args(const glint_ctx *c, const uint32_t *bits) {
     a.tab = c->d_tab;
     a.stamp = c->d_stamp;
     a.B = c->B;
-    a.st = stamp_of(c->step_index);
     a.cur_time = c->last_time;
     a.min_plus1 = c->cfg.min_meet_time + 1;
     a.bits = bits;

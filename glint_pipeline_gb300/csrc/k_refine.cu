@@ -88,7 +88,7 @@ RefineArgs refine_args(glint_ctx *c) {
     a.qlist = c->d_qlist;
     a.extra = c->d_rextra;
     a.tab = c->d_tab;
-    a.stamp = c->d_stamp;
+    a.stamp = c->B <= kStampTouchBuckets ? c->d_stamp : nullptr;
     a.newlist = c->d_new;
     a.B = c->B;
     a.Bm = c->Bm;
@@ -152,6 +152,7 @@ __device__ inline void touch_box(TRec &r, const float2 &A, const float2 &Bp) {
 }
 
 __global__ void __launch_bounds__(256) k_insert(const NewEntry *__restrict__ list, TRec *tab, uint32_t *newline,
+                                                uint8_t *stamp,
                                                 uint64_t B, uint64_t Bm, uint64_t new_cap,
                                                 const float2 *__restrict__ fpos, uint32_t N,
                                                 DevCounters *cnt) {
@@ -195,7 +196,8 @@ __global__ void __launch_bounds__(256) k_insert(const NewEntry *__restrict__ lis
                     /* the carried pair's own committed entry */
                     const uint32_t pa = pair_a(plain), pb = pair_b(plain);
                     if (pa < N && pb < N) touch_box(tab[slot], fpos[pa], fpos[pb]);
-                    rec_set_tag(tab[slot], st);
+                    if (stamp) stamp[slot] = (uint8_t)(kStampTouched + st);
+                    else rec_set_tag(tab[slot], st);
                     done = true;
                     break;
                 }
@@ -234,7 +236,8 @@ cudaError_t launch_insert(glint_ctx *c, uint32_t cur_time) {
      * balance it (5.4 against 7.7 ms at 10M objects), fewer for a small
      * context's new-pair capacity */
     const unsigned blocks = (unsigned)std::min<uint64_t>(152u * 128u, std::max<uint64_t>(152u, c->new_cap / 2048));
-    k_insert<<<blocks, 256, 0, c->stream>>>(c->d_new, c->d_tab, c->d_newline, c->B, c->Bm, c->new_cap, c->d_fpos, c->N,
+    k_insert<<<blocks, 256, 0, c->stream>>>(c->d_new, c->d_tab, c->d_newline,
+                                             c->B <= kStampTouchBuckets ? c->d_stamp : nullptr, c->B, c->Bm, c->new_cap, c->d_fpos, c->N,
                                              c->d_cnt);
     return cudaGetLastError();
 }

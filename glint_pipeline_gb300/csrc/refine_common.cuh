@@ -44,7 +44,7 @@ struct RefineArgs {
     const IBox *ibox;
     const uint2 *extra;        /* (leaf, chunk) items beyond each leaf's first chunk */
     TRec *tab;
-    uint8_t *stamp;
+    uint8_t *stamp;            /* null: a touch is a tag in the record */
     NewEntry *newlist;
     uint64_t B, Bm, new_cap;
     uint32_t cap;
@@ -78,7 +78,8 @@ __device__ inline bool table_touch_from(const RefineArgs &a, const QEntry &q, ui
                 m.w = max(m.w, hy);
                 *reinterpret_cast<uint4 *>(a.tab[slot].mbr) = m;
             }
-            rec_set_tag(a.tab[slot], tag);
+            if (a.stamp) a.stamp[slot] = (uint8_t)(kStampTouched + tag);
+            else rec_set_tag(a.tab[slot], tag);
             return false;
         }
         if (w0 == kEmptyW0) return true;

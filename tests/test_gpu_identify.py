@@ -1,6 +1,7 @@
 """Identify and the scans at the sizes where their tiles end: tables of one
 bucket more or less than a whole number of tiles, on both sides of the small
-table's shorter spans, and object counts around a scan tile's 4096."""
+table's shorter spans, and object counts around a scan tile's 4096; and both
+ways of touching an entry, over enough steps for both parities."""
 import numpy as np
 import pytest
 
@@ -15,6 +16,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n,buckets", [
     (4095, 1024 * 12 - 1), (4096, 1024 * 12), (4097, 1024 * 12 + 1), (8193, 30011),
     (4000, (1 << 23) - 1), (4000, 1 << 23), (4000, (1 << 23) + 8193),
+    (3000, 1 << 26), (3000, (1 << 26) + 1),  # touches by stamp, by tag
 ])
 def test_identify_matches_oracle(n, buckets):
     steps = 14

@@ -411,7 +411,6 @@ extern "C" glint_status glint_active_search(glint_ctx *c, const uint32_t *pids, 
     cudaSetDevice(c->device);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     const uint64_t words = ((uint64_t)c->N + 31) / 32;
-    if (e == cudaSuccess) e = grow(&c->d_qbits, c->qbits_cap, words);
     if (e == cudaSuccess) e = grow(&c->d_qpids, c->qpids_cap, std::max<uint64_t>(npids, 1));
     if (e == cudaSuccess) e = grow(&c->d_qout, c->qout_cap, std::max<uint64_t>(cap, 1));
     if (e == cudaSuccess && !c->d_qn) e = cudaMalloc((void **)&c->d_qn, sizeof(unsigned long long));
@@ -428,6 +427,7 @@ extern "C" glint_status glint_active_search(glint_ctx *c, const uint32_t *pids, 
         fetch();
     }
     /* by bucket, also when more entries were found than one block orders */
+    if (e == cudaSuccess && found == ~0ull) e = grow(&c->d_qbits, c->qbits_cap, words);
     if (e == cudaSuccess && found == ~0ull) {
         void *tmp = c->d_scan_tmp;
         auto scan = [tmp](const uint32_t *in, uint32_t *o, uint64_t m, cudaStream_t s) {

@@ -47,15 +47,8 @@ __global__ void __launch_bounds__(32 * kRefineWarps) k_refine_fp64(RefineArgs a)
     const LeafTile m = leaf_tile(smem_raw + (size_t)(threadIdx.x >> 5) * tile_warp_bytes(a.cap), a.cap);
     RefineTally t;
     uint32_t qn = 0;
-    const uint32_t nwork = a.cnt->n_leaf_work, n_extra = a.cnt->n_extra;
     const uint32_t tag = a.cnt->step_tag;
-    bool extra_done = n_extra == 0;
-    LeafOrigin o;
-    for (;;) {
-        uint32_t g, chunk;
-        if (!claim_item(a, nwork, n_extra, extra_done, g, chunk)) break;
-        refine_item<true>(a, g, chunk, m, o, t, qn, tag);
-    }
+    refine_items<true>(a, m, t, qn, tag);
     refine_flush<true>(a, m.Q, qn, tag, t);
 }
 

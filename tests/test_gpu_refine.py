@@ -46,3 +46,27 @@ def test_refine_matches_oracle(capacity, amplify, extent, sigma, chunk, precisio
     assert contacts > 0 and total > 0
     g.close()
     o.close()
+
+
+@pytest.mark.parametrize("precision_mode", [0, 1])
+@pytest.mark.parametrize("n,chunk", [(40, 0), (2000, 0), (6000, 0), (10000, 0), (16000, 0), (40000, 0),
+                                     (2000, 1), (6000, 2)])
+def test_items_by_number_and_by_cursor(n, chunk, precision_mode):
+    """Work items from a handful to several times the warps of a launch: four,
+    two and one warps an item, and items taken from the cursor.  About four
+    members a leaf, so that n / 4 leaves and their extra chunks cross 1216, 2432
+    and 4864."""
+    gen = TraceGenerator(0xA11 + n, n, 0, extent_m=6.0 * n ** 0.5, n_hotspots=5, sigma_m=1.2 * n ** 0.5, hotspot_frac=0.5)
+    box, pts = gen.box(), gen.steps(4)
+    args = dict(num_objects=n, num_meeting_buckets=1 << 20, grid_capacity=6, grid_amplify=2.0)
+    o = Oracle(make_config(**args), box, pts[0])
+    g = DeviceBench(Configuration(precision_mode=precision_mode, refine_chunk=chunk, **args), box, pts[0])
+    for t in range(4):
+        o.step(pts[t], t)
+        st = g.step(pts[t], t)
+        c = o.counts()
+        assert (st.checks, st.candidates, st.contacts) == (c.grid_check_counter, c.candidates, c.contacts), f"step {t}"
+        compare_meetings(o.meetings(), g.meetings(), t)
+    assert n < 1000 or int(st.contacts) > 0
+    g.close()
+    o.close()

@@ -135,10 +135,9 @@ struct GatherOut {
 };
 
 /* the object pid at place `at` of the segment of a leaf node that starts at s0 */
-__device__ inline void gather_one(const GatherOut &o, const Frame &f, const double2 *__restrict__ pts, uint32_t s0,
-                                  uint32_t at, uint32_t pid, uint32_t leaf) {
+__device__ inline void gather_one(const GatherOut &o, const Frame &f, const double2 p, uint32_t s0, uint32_t at,
+                                  uint32_t pid, uint32_t leaf) {
     const uint32_t i = s0 + at;
-    const double2 p = pts[pid];
     o.sxy[i] = p;
     bool clamped = false;
     const long long X = fx_coord(p.x, f.k, f.X0, &clamped);
@@ -152,42 +151,61 @@ __device__ inline void gather_one(const GatherOut &o, const Frame &f, const doub
     o.rank[pid] = make_uint2(at < o.cap ? i : i | kDropped, leaf);
 }
 
-/* bitonic sort of n (<= 1024) keys in a warp's shared buffer, padded with ~0u */
-__device__ inline void warp_bitonic(uint32_t *buf, uint32_t n) {
-    uint32_t P = 32;
-    while (P < n) P <<= 1;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t i = n + lane; i < P; i += 32) buf[i] = 0xffffffffu;
-    __syncwarp();
-    for (uint32_t k = 2; k <= P; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = lane; i < P; i += 32) {
-                uint32_t l = i ^ j;
-                if (l > i) {
-                    uint32_t a = buf[i], b = buf[l];
-                    bool up = (i & k) == 0;
-                    if ((a > b) == up) { buf[i] = b; buf[l] = a; }
-                }
-            }
-            __syncwarp();
-        }
+/* A warp's segment of up to 32 K different ids: each lane counts the ids below
+ * its own, which is their place.  One pass over the ids in shared memory, read
+ * four at a time by all lanes at once, with the points' loads in flight behind
+ * it; a bitonic network of the same segment is 15 to 28 stages, each waiting
+ * for the one before. */
+template <int K>
+__device__ inline void rank_sort(const GatherOut &o, const Frame &f, const double2 *__restrict__ pts, uint32_t *seg,
+                                 uint32_t *buf, uint32_t n, uint32_t s0, uint32_t leaf) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t v[K], r[K];
+    double2 p[K];
+#pragma unroll
+    for (int e = 0; e < K; ++e) {
+        const uint32_t i = lane + 32 * e;
+        v[e] = i < n ? seg[i] : 0xffffffffu;
+        buf[i] = v[e];
+        r[e] = 0;
     }
+#pragma unroll
+    for (int e = 0; e < K; ++e)
+        if (lane + 32 * e < n) p[e] = pts[v[e]];
+    __syncwarp();
+    for (uint32_t j = 0; j < n; j += 4) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(buf + j);
+#pragma unroll
+        for (int e = 0; e < K; ++e) r[e] += (q.x < v[e]) + (q.y < v[e]) + (q.z < v[e]) + (q.w < v[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < K; ++e)
+        if (lane + 32 * e < n) {
+            seg[r[e]] = v[e];
+            gather_one(o, f, p[e], s0, r[e], v[e], leaf);
+        }
 }
 
 constexpr int kSortWarps = 8;
-constexpr uint32_t kWarpSortMax = 1024;
+constexpr uint32_t kWarpSortMax = 128;
+constexpr uint32_t kRankSortMax = 512;
 
 /* One warp per leaf segment of up to kWarpSortMax objects: its ids in order,
- * and each object's gathered arrays while the ids are still at hand.  (As a
- * sort and a gather of their own: 31 + 37 us at 1M objects; together and
- * without FP64 instructions 49 us.) */
+ * and each object's gathered arrays while the ids are still at hand.  Bound:
+ * the scattered reads and writes by object id (about 100 bytes an object in
+ * 32-byte sectors), and at small maps the chain of dependent loads from the
+ * leaf to the point.  With a bitonic network: 1M objects 53 us, 20k 9.3, 2k
+ * 8.3; ranked by counting: 37, 5.9 and 4.6.  Segments up to 1024 a warp left
+ * 2M objects in dense spots waiting for a few warps: 249 us, 225 with the
+ * counting alone; from 129 on by whole blocks 84 (and 47 in the block kernel,
+ * 13 before; the line at 256: 115 and 36). */
 __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t *__restrict__ work,
                                                                   const uint32_t *__restrict__ grid_start,
                                                                   const uint32_t *__restrict__ grid_count,
                                                                   uint32_t *__restrict__ sorted,
                                                                   const double2 *const *in, GatherOut o,
                                                                   Frame f, const DevCounters *cnt) {
-    __shared__ uint32_t buf[kSortWarps][kWarpSortMax];
+    __shared__ __align__(16) uint32_t buf[kSortWarps][kWarpSortMax];
     const double2 *__restrict__ pts = *in;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nwork = cnt->n_leaf_work;
@@ -199,45 +217,26 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t
         uint32_t *seg = sorted + s0;
         const uint32_t leaf = o.obj[seg[0]].z; /* the node of grid g: one for all its objects */
         __syncwarp();
-        if (n <= 32) {
-            uint32_t v = lane < (int)n ? seg[lane] : 0xffffffffu;
-            /* register bitonic sort across the warp */
-            for (int k = 2; k <= 32; k <<= 1) {
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    uint32_t x = __shfl_xor_sync(0xffffffffu, v, j);
-                    bool up = (lane & k) == 0;
-                    bool lower = (lane & j) == 0;
-                    v = (lower == up) ? min(v, x) : max(v, x);
-                }
-                if (k >= (int)n) break; /* the padding sorts last: done */
-            }
-            if (lane < (int)n) {
-                seg[lane] = v;
-                gather_one(o, f, pts, s0, lane, v, leaf);
-            }
-        } else {
-            for (uint32_t i = lane; i < n; i += 32) buf[w][i] = seg[i];
-            __syncwarp();
-            warp_bitonic(buf[w], n);
-            for (uint32_t i = lane; i < n; i += 32) {
-                seg[i] = buf[w][i];
-                gather_one(o, f, pts, s0, i, buf[w][i], leaf);
-            }
-        }
+        if (n <= 32) rank_sort<1>(o, f, pts, seg, buf[w], n, s0, leaf);
+        else if (n <= 64) rank_sort<2>(o, f, pts, seg, buf[w], n, s0, leaf);
+        else rank_sort<4>(o, f, pts, seg, buf[w], n, s0, leaf);
         __syncwarp();
     }
 }
 
 constexpr uint32_t kBlockSortMax = 16384;
 
-/* one block per long segment (up to kBlockSortMax objects) */
+/* One block per longer segment (up to kBlockSortMax objects): ranked by
+ * counting up to kRankSortMax, with two or four threads an object, above that
+ * by a bitonic network (counting grows with the square of the length: the line
+ * at 1024 took 56 us where this takes 47, 2M objects in dense spots). */
 __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restrict__ big,
                                                         const uint32_t *__restrict__ grid_start,
                                                         const uint32_t *__restrict__ grid_count,
                                                         uint32_t *__restrict__ sorted,
                                                         const double2 *const *in, GatherOut o, Frame f,
                                                         DevCounters *cnt) {
-    extern __shared__ uint32_t sbuf[];
+    extern __shared__ __align__(16) uint32_t sbuf[];
     const double2 *__restrict__ pts = *in;
     const uint32_t nbig = cnt->n_big;
     for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
@@ -248,15 +247,35 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
              * follows in this step reads objects */
             if (threadIdx.x == 0) atomicOr(&cnt->error_flags, GLINT_EF_SEGMENT_TOO_LARGE);
             for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-                gather_one(o, f, pts, grid_start[g], i, sorted[grid_start[g] + i],
+                gather_one(o, f, pts[sorted[grid_start[g] + i]], grid_start[g], i, sorted[grid_start[g] + i],
                            o.obj[sorted[grid_start[g]]].z);
+            continue;
+        }
+        uint32_t *seg = sorted + grid_start[g];
+        const uint32_t leaf = o.obj[seg[0]].z;
+        __syncthreads();
+        if (n <= kRankSortMax) {
+            const uint32_t parts = n <= kRankSortMax / 2 ? 4 : 2;
+            const uint32_t i = threadIdx.x / parts, part = threadIdx.x % parts;
+            if (threadIdx.x < kRankSortMax) sbuf[threadIdx.x] = threadIdx.x < n ? seg[threadIdx.x] : 0xffffffffu;
+            __syncthreads();
+            const uint32_t v = sbuf[i];
+            double2 p = make_double2(0., 0.);
+            if (i < n) p = pts[v];
+            uint32_t r = 0;
+            for (uint32_t j = 4 * part; j < n; j += 4 * parts) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(sbuf + j);
+                r += (q.x < v) + (q.y < v) + (q.z < v) + (q.w < v);
+            }
+            for (uint32_t d = 1; d < parts; d <<= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
+            if (i < n && part == 0) {
+                seg[r] = v;
+                gather_one(o, f, p, grid_start[g], r, v, leaf);
+            }
             continue;
         }
         uint32_t P = 1024;
         while (P < n) P <<= 1;
-        uint32_t *seg = sorted + grid_start[g];
-        const uint32_t leaf = o.obj[seg[0]].z;
-        __syncthreads();
         for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) sbuf[i] = i < n ? seg[i] : 0xffffffffu;
         __syncthreads();
         for (uint32_t k = 2; k <= P; k <<= 1) {
@@ -274,7 +293,7 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
         }
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
             seg[i] = sbuf[i];
-            gather_one(o, f, pts, grid_start[g], i, sbuf[i], leaf);
+            gather_one(o, f, pts[sbuf[i]], grid_start[g], i, sbuf[i], leaf);
         }
         __syncthreads();
     }
@@ -335,7 +354,7 @@ cudaError_t launch_partition(glint_ctx *c) {
     o.cap = c->cap;
     k_segsort_warp<<<grid_for(N, 16 * kSortWarps, 152u * 8u), 32 * kSortWarps, 0, s>>>(
         c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_in, o, c->frame, c->d_cnt);
-    k_segsort_block<<<152, 1024, kBlockSortMax * sizeof(uint32_t), s>>>(
+    k_segsort_block<<<304, 1024, kBlockSortMax * sizeof(uint32_t), s>>>(
         c->d_big, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_in, o, c->frame, c->d_cnt);
     return cudaGetLastError();
 }

@@ -101,14 +101,15 @@ struct FilterArgs {
     DevCounters *cnt;
 };
 
-/* One step of a walk: the node on top is opened, or the kept leaf on top is
+/* One step of a walk (of the start node only the children in `share` are
+ * taken): the node on top is opened, or the kept leaf on top is
  * given to emit(gid, ordinal).  The box test is screened on the fixed-point
  * boxes; only a box within the guard band of the reach takes the reference's
  * FP64 box distance.  The top/right rule is decided on the fixed-point
  * coordinates where they are more than a unit apart, else on the doubles'
  * keys. */
 template <class Emit>
-__device__ inline void walk_step(const FilterArgs &a, Walk &k, const WalkPoint &w, Emit emit) {
+__device__ inline void walk_step(const FilterArgs &a, Walk &k, const WalkPoint &w, uint32_t share, Emit emit) {
     const uint32_t e = k.stack[--k.sp], top = e & ~kWalkStart;
     const uint4 chv = *reinterpret_cast<const uint4 *>(a.nodes[top].child);
     const uint2 tail = *reinterpret_cast<const uint2 *>(&a.nodes[top].gid); /* gid; type, level */
@@ -146,9 +147,10 @@ __device__ inline void walk_step(const FilterArgs &a, Walk &k, const WalkPoint &
         }
     }
     const uint32_t ch[4] = {chv.x, chv.y, chv.z, chv.w};
+    if (!(e & kWalkStart)) share = 15u;
 #pragma unroll
     for (int i = 3; i >= 0; --i) {
-        if (fb[i].x - w.fx > w.rx || w.fx - fb[i].z > w.rx || fb[i].y - w.fy > w.ry || fb[i].w < w.top) continue;
+        if (!(share >> i & 1u) || fb[i].x - w.fx > w.rx || w.fx - fb[i].z > w.rx || fb[i].y - w.fy > w.ry || fb[i].w < w.top) continue;
         if (k.sp < kStackMax) k.stack[k.sp++] = ch[i];
         else atomicOr(&a.cnt->error_flags, GLINT_EF_DFS_OVERFLOW);
     }
@@ -159,6 +161,11 @@ __device__ inline void walk_step(const FilterArgs &a, Walk &k, const WalkPoint &
  * consecutive ranks at a time, queues its border objects in shared memory and
  * walks them 32 at a time, so that every lane of a walk has an object. */
 constexpr int kWalkWarps = 4;
+/* Maps of up to eight ranks for each of 24 warps an SM are read eight ranks at a
+ * time, larger ones 32: a warp with at most eight border objects gives each four
+ * lanes.  20k objects 15.1 -> 11.2 us, 2k 10.7 -> 8.0; read 16 at a time 100k
+ * gained 1 us, and sixteen regions at once, which share the SMs, lost 2%. */
+constexpr uint32_t kWalkSpread = 152 * 24;
 
 struct CheckLists {
     uint32_t *qstart, *qcount; /* each object's checks */
@@ -168,18 +175,18 @@ struct CheckLists {
     uint64_t cap;
 };
 
-__global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, CheckLists l) {
+__global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, CheckLists l, uint32_t span) {
     __shared__ uint32_t sbuf[kWalkWarps][64];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
-    const uint32_t stride = gridDim.x * kWalkWarps * 32;
-    uint32_t base = (blockIdx.x * kWalkWarps + wid) * 32;
+    const uint32_t stride = gridDim.x * kWalkWarps * span;
+    uint32_t base = (blockIdx.x * kWalkWarps + wid) * span;
     uint32_t nb = 0, nborder = 0;
     for (;;) {
         while (nb < 32 && base < a.N) {
             const uint32_t i = base + lane;
             bool border = false;
-            if (i < a.N) {
+            if (lane < (int)span && i < a.N) {
                 const uint32_t p = a.sorted[i];
                 const uint4 o = a.obj[p];
                 border = o.y != o.z;
@@ -193,21 +200,25 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, C
             __syncwarp();
         }
         if (nb == 0) break;
-        /* the queue's last objects */
+        /* the queue's last objects; of few, two or four lanes have one and
+         * share the children of its start, in order */
         const uint32_t take = nb < 32 ? nb : 32;
-        const bool mine = (uint32_t)lane < take;
+        const uint32_t parts = take <= 8 ? 4u : take <= 16 ? 2u : 1u;
+        const uint32_t obj = lane / parts, sub = lane % parts;
+        const uint32_t share = parts == 4 ? 1u << sub : parts == 2 ? 3u << 2 * sub : 15u;
+        const bool mine = obj < take;
         uint32_t pid = 0, lv = 0, row[kQInline];
         Walk k;
         WalkPoint w;
         if (mine) {
-            const uint32_t i = sbuf[wid][nb - take + lane];
+            const uint32_t i = sbuf[wid][nb - take + obj];
             pid = a.sorted[i];
             lv = a.obj[pid].y;
             w = walk_point(a.sxy[i], a.sipos[i], a.sc[i], a.f);
             k.sp = 1;
             k.stack[0] = lv | kWalkStart;
             while (k.sp > 0)
-                walk_step(a, k, w, [&](uint32_t gid, uint32_t j) {
+                walk_step(a, k, w, share, [&](uint32_t gid, uint32_t j) {
                     if (j < (uint32_t)kQInline) row[j] = gid;
                 });
         }
@@ -219,16 +230,22 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, C
             const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
+        const uint32_t head = lane - sub, tail = head + parts - 1;
         uint32_t at = 0;
         if (lane == 31 && incl) at = atomicAdd(&a.cnt->cross_checks, incl);
         at = __shfl_sync(0xffffffffu, at, 31) + incl - n;
+        /* the object's run: from its first lane's to its last lane's end */
+        const uint32_t from = __shfl_sync(0xffffffffu, at, head), to = __shfl_sync(0xffffffffu, at + n, tail);
         if (mine) {
-            if ((uint64_t)at + n > l.cap) {
+            uint32_t all = to - from;
+            if ((uint64_t)from + all > l.cap) {
                 atomicOr(&a.cnt->error_flags, GLINT_EF_CHECKS_OVERFLOW);
-                n = 0;
+                all = n = 0;
             }
-            l.qstart[pid] = at;
-            l.qcount[pid] = n;
+            if (sub == 0) {
+                l.qstart[pid] = from;
+                l.qcount[pid] = all;
+            }
             auto put = [&](uint32_t gid, uint32_t j) {
                 l.qlist[at + j] = gid;
                 l.qslot[at + j] = atomicAdd(&l.tcount[gid], 1u);
@@ -240,7 +257,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, C
                 k.kept = 0;
                 k.stack[0] = lv | kWalkStart;
                 while (k.sp > 0)
-                    walk_step(a, k, w, [&](uint32_t gid, uint32_t j) {
+                    walk_step(a, k, w, share, [&](uint32_t gid, uint32_t j) {
                         if (j >= (uint32_t)kQInline && j < n) put(gid, j);
                     });
             }
@@ -327,7 +344,8 @@ cudaError_t launch_filter(glint_ctx *c) {
     l.qslot = c->d_qslot;
     l.tcount = c->d_tcount;
     l.cap = c->check_cap;
-    k_filter_walk<<<grid_for(N, 32 * kWalkWarps, 152u * 16u), 32 * kWalkWarps, 0, s>>>(a, l);
+    const uint32_t span = N <= 8 * kWalkSpread ? 8u : 32u;
+    k_filter_walk<<<grid_for(N, span * kWalkWarps, 152u * 16u), 32 * kWalkWarps, 0, s>>>(a, l, span);
     TargetScan ts;
     ts.start = ScanStore{c->d_tstart, true};
     ts.grid_count = c->d_grid_count;

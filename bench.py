@@ -350,10 +350,9 @@ def run_form(args, mode, N, local, pg, world, box, first, pb, ob, dbuf, step_byt
 
 # DRAM bytes per step of each stage's kernels (dram__bytes_read.sum +
 # dram__bytes_write.sum) at 10M objects and 2^30 buckets, the tuned form:
-# from a full capture of each kernel on the 2M-object case scaled by the
-# stage's units, and from the one-pass launch list of the 10M step where
-# noted (profiles/); other workloads report null
-TRAFFIC_10M_2P30 = {"refine": 43.0e9, "identify": 50.6e9, "insert": 26.5e9}
+# from the one-pass launch list of the 10M step (profiles/); other workloads
+# report null
+TRAFFIC_10M_2P30 = {"refine": 40.1e9, "identify": 50.8e9, "insert": 20.5e9}
 
 
 def step_bytes_8d(N, per):
@@ -373,9 +372,9 @@ def roofline(form, N, buckets=None, mode=None):
     hbm = pk.get("hbm_gbs")
     peak = hbm if hbm else 6800.0
     stages = {k: v for k, v in form["stage_ms"].items() if k in ("partition", "filter", "refine", "insert", "identify")}
-    # the dominant kernel is refine's (k_refine_fp32 in the tuned form: 35% of
+    # the dominant kernel is refine's (k_refine_fp32 in the tuned form: 34% of
     # the step's kernel time in the ncu launch list, k_expire_count next at
-    # 26%); by stage, refine and identify take turns as the slowest
+    # 32%); by stage, refine and identify take turns as the slowest
     top = "refine"
     slowest = max(stages, key=stages.get)
     ms = stages[top]

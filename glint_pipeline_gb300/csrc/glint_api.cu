@@ -26,6 +26,7 @@ void refine_set_attributes(uint32_t cap);
 void refine_prec_set_attributes(uint32_t cap);
 size_t refine_smem_bytes(uint32_t cap);
 uint64_t identify_tiles(uint64_t B);
+uint32_t identify_launches(uint64_t tiles);
 cudaError_t noalloc_setup(int device);
 /* stamps cover a whole number of identify tiles (the padding stays empty) */
 inline uint64_t stamp_bytes(uint64_t B) { return (B + 8191) / 8192 * 8192 + 64; }
@@ -801,7 +802,7 @@ static void fill_stats(glint_ctx *c, glint_step_stats *st) {
     st->error_flags = h.error_flags;
     /* kernels per step: begin 1, partition 5, filter 3, refine 1, insert 1,
      * identify 3 (2 for small tables) + keys 1, schema update 4, tail 1 */
-    st->launches = 1 + 5 + 3 + 1 + 1 + 4 + (c->cfg.dynamic_schema ? 4 : 0) + 1;
+    st->launches = 1 + 5 + 3 + 1 + 1 + identify_launches(c->n_tiles) + 1 + (c->cfg.dynamic_schema ? 4 : 0) + 1;
     st->meeting_log_size = h.log_head;
     st->kv_count = h.kv_count;
     st->flushed = c->last_flushed ? 1u : 0u;

@@ -110,7 +110,6 @@ constexpr unsigned long long kEmptyW0 = ~0ull;
 constexpr unsigned long long kPairMask = ~kNewFlag;
 
 /* the touch tag of a committed record */
-__device__ inline uint32_t rec_tag(const TRec &r) { return (uint32_t)(r.w1 >> 32); }
 __device__ inline void rec_set_tag(TRec &r, uint32_t tag) { reinterpret_cast<uint32_t *>(&r.w1)[1] = tag; }
 
 __host__ __device__ inline unsigned long long pair_word(uint32_t a, uint32_t b) {

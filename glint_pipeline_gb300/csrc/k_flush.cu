@@ -24,10 +24,11 @@
  *
  * Device form of the sorts (the reference uses thrust): the STR sorts are
  * stable LSD radix sorts (k_sort.cu).  The key sorts exploit the key layout:
- * keys group by (part, sid, pid), so objects are radix-sorted by that triple,
- * each object's keys get a contiguous segment (a scan of the key counts), the
- * keys are scattered into their segments and each segment (a few keys, at
- * most kSegBlockMax) is sorted by a warp or a block.
+ * keys group by (part, sid, pid), so objects, which come in pid order, are
+ * radix-sorted by a 16-bit class of part and sid (2 passes), each object's
+ * keys get a contiguous segment (a scan of the key counts), the keys are
+ * scattered into their segments and each segment (a few keys, at most
+ * kSegBlockMax) is sorted by part of a warp, a warp or a block.
  *
  * The reference's cuda_get_limit and get_o_limit fold a 1024-entry shared
  * reduction down to 64 partial results and then shuffle-reduce only the

@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(kIdThreads) k_expire_emit(uint8_t *__restrict_
 
 /* up to here a block's own sum is four loads per thread */
 constexpr unsigned kOwnScanTiles = 1024;
+uint32_t identify_launches(uint64_t tiles) { return tiles <= kOwnScanTiles ? 2u : 3u; }
 
 template <uint32_t kSpan>
 static void identify_passes(glint_ctx *c) {

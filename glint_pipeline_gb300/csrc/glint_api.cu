@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(64) k_step_tail(uint32_t N, const uint32_t *re
 }
 
 void free_all(glint_ctx *c) {
-    void *ptrs[] = {c->d_pts, c->d_in, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_cbox, c->d_obj, c->d_grid_count,
+    void *ptrs[] = {c->d_pts, c->d_in, c->d_sipos, c->d_sfpos, c->d_sc, c->d_fpos, c->d_ibox, c->d_cbox, c->d_obj, c->d_seg, c->d_info, c->d_grid_node, c->d_grid_count,
                     c->d_grid_start, c->d_sorted, c->d_rank, c->d_sxy, c->d_sm, c->d_leaf_work,
                     c->d_nodes, c->d_low, c->d_sstack, c->d_gstack, c->d_split, c->d_evscan, c->d_cand, c->d_newgid,
                     c->d_evlist, c->d_evdata, c->d_evlevel, c->d_big, c->d_qcount,
@@ -416,6 +416,9 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     ALLOC(c->d_sc, N);
     ALLOC(c->d_fpos, N);
     ALLOC(c->d_obj, N);
+    ALLOC(c->d_seg, N);
+    ALLOC(c->d_info, N);
+    ALLOC(c->d_grid_node, G);
     ALLOC(c->d_grid_count, (size_t)G + 1);
     ALLOC(c->d_grid_start, (size_t)G + 1);
     ALLOC(c->d_sorted, N);

@@ -4,8 +4,11 @@
  *
  * HBM layout (N objects, G grid slots, S schema slots, B buckets):
  *   points      double2[N]   lon/lat as given, AoS 16 B per object
- *   obj         uint4[N]     leaf grid id, last_valid node, leaf node, place in the leaf, per object
+ *   obj         uint4[N]     in the last step's order: object, leaf grid id, last_valid node, place in the leaf
+ *   seg         uint2[N]     object and last_valid node, by leaf grid, in any order within a leaf
  *   sorted      u32[N]       object ids sorted by (grid id, object id): leaf member lists
+ *   info        uint2[N]     where an object's walk starts (kNoWalk: not a border object) and its
+ *                            leaf grid, in that order
  *   sxy         double2[N]   coordinates gathered in that order (leaf tiles)
  *   sipos, sc   [N]          fixed-point coordinates (i64 pair) and screening scale, same order
  *   sfpos, fpos float2[N]    FP32 coordinates (meeting boxes), sorted and by object id
@@ -101,6 +104,8 @@ constexpr uint64_t kStampTouchBuckets = 1ull << 26;
 
 /* a rank's mark: the object is past its leaf's buffer, which drops it */
 constexpr uint32_t kDropped = 0x80000000u;
+/* not a border object: its last_valid node is its leaf */
+constexpr uint32_t kNoWalk = 0xffffffffu;
 
 /* cross-leaf checks per refine work item (refine_common.cuh) */
 constexpr uint32_t kCrossChunk = 64;       /* default cross-leaf checks per refine work item */
@@ -199,8 +204,11 @@ struct glint_ctx {
 
     /* objects */
     double2 *d_pts = nullptr;              /* [N] the step's points, where they are not read in place */
-    uint4 *d_obj = nullptr;                /* [N] each object's leaf grid, last_valid node, leaf node and place in
-                                              its leaf's segment */
+    uint4 *d_obj = nullptr;                /* [N] in the last step's leaf-major order: object, leaf grid,
+                                              last_valid node and place in its leaf's segment */
+    uint2 *d_seg = nullptr;                /* [N] object and last_valid node by leaf grid, unsorted in a leaf */
+    uint2 *d_info = nullptr;               /* [N] leaf-major: the node a walk starts from (kNoWalk: none), leaf grid */
+    uint32_t *d_grid_node = nullptr;       /* [G] the leaf node of each grid that holds objects */
     bool input_device = false;             /* the step's input is device (not managed) memory */
     uint32_t *d_grid_count = nullptr;      /* [G+1] */
     uint32_t *d_grid_start = nullptr;      /* [G+1] */

@@ -90,7 +90,7 @@ struct FilterArgs {
     const double2 *sxy;
     const longlong2 *sipos;
     const float *sc;
-    const uint4 *obj;
+    const uint2 *info;
     const DNode *nodes;
     const double2 *low;
     const IBox *ibox;
@@ -187,10 +187,8 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, C
             const uint32_t i = base + lane;
             bool border = false;
             if (lane < (int)span && i < a.N) {
-                const uint32_t p = a.sorted[i];
-                const uint4 o = a.obj[p];
-                border = o.y != o.z;
-                if (!border) l.qcount[p] = 0;
+                border = a.info[i].x != kNoWalk;
+                if (!border) l.qcount[a.sorted[i]] = 0;
             }
             const unsigned m = __ballot_sync(0xffffffffu, border);
             if (border) sbuf[wid][nb + __popc(m & below)] = i;
@@ -213,7 +211,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_filter_walk(FilterArgs a, C
         if (mine) {
             const uint32_t i = sbuf[wid][nb - take + obj];
             pid = a.sorted[i];
-            lv = a.obj[pid].y;
+            lv = a.info[i].x;
             w = walk_point(a.sxy[i], a.sipos[i], a.sc[i], a.f);
             k.sp = 1;
             k.stack[0] = lv | kWalkStart;
@@ -328,7 +326,7 @@ cudaError_t launch_filter(glint_ctx *c) {
     a.sxy = c->d_sxy;
     a.sipos = c->d_sipos;
     a.sc = c->d_sc;
-    a.obj = c->d_obj;
+    a.info = c->d_info;
     a.nodes = c->d_nodes;
     a.low = c->d_low;
     a.ibox = c->d_ibox;

@@ -14,7 +14,7 @@
  * Here the leaf buffers are replaced by a stable sort of objects by
  * (grid id, object id): a count per grid, which gives every object a place in
  * its grid's segment, an exclusive scan, a scatter and a per-leaf sort of each
- * segment.  The first min(count, capacity) entries of a
+ * segment, which also gathers what the later stages read in that order.  The first min(count, capacity) entries of a
  * segment are exactly the reference's stored members, in the same order.
  */
 #include "scan.cuh"
@@ -26,6 +26,7 @@ constexpr int kMaxDepth = 64;
 __global__ void __launch_bounds__(256) k_descend(const double2 *const *in, const uint32_t *__restrict__ order,
                                                  uint32_t N, const DNode *__restrict__ nodes, uint32_t S, uint32_t G,
                                                  double xb, double yb, uint4 *__restrict__ obj,
+                                                 uint32_t *__restrict__ grid_node,
                                                  uint32_t *__restrict__ grid_count, DevCounters *cnt) {
     const double2 *__restrict__ pts = *in;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
@@ -66,18 +67,22 @@ __global__ void __launch_bounds__(256) k_descend(const double2 *const *in, const
         uint32_t at = 0;
         if ((threadIdx.x & 31) == leader) at = atomicAdd(&grid_count[gid], (uint32_t)__popc(peers));
         at = __shfl_sync(peers, at, leader);
-        /* one 16-byte record: objects come in leaf order, so each write is a
-         * memory transaction of its own */
-        obj[pid] = make_uint4(gid, lv, cur, at + __popc(peers & ((1u << (threadIdx.x & 31)) - 1u)));
+        at += __popc(peers & ((1u << (threadIdx.x & 31)) - 1u));
+        if (at == 0) grid_node[gid] = cur;
+        /* in the order of the launch, which is nearly the order that follows: by
+         * object id this store, the scatter's and the walk's loads were a sector
+         * an object each.  Descent, scatter and walk at 1M objects 48 + 10.3 + 93
+         * us, so 46 + 3.7 + 91; at 10M 0.65 + 0.11 + 1.28 ms, 0.54 + 0.04 + 1.16 */
+        obj[i] = make_uint4(pid, gid, lv == cur ? kNoWalk : lv, at);
     }
 }
 
 __global__ void __launch_bounds__(256) k_scatter(const uint4 *__restrict__ obj, uint32_t N,
                                                  const uint32_t *__restrict__ grid_start,
-                                                 uint32_t *__restrict__ sorted) {
-    for (uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x; pid < N; pid += gridDim.x * blockDim.x) {
-        const uint4 o = obj[pid];
-        sorted[grid_start[o.x] + o.w] = pid;
+                                                 uint2 *__restrict__ unsorted) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        const uint4 o = obj[i];
+        unsorted[grid_start[o.y] + o.w] = make_uint2(o.x, o.z);
     }
 }
 
@@ -130,14 +135,24 @@ struct GatherOut {
     double *sm;        /* null: not needed */
     float2 *fpos;      /* by object id */
     uint2 *rank;       /* by object id: sorted position and leaf node */
-    const uint4 *obj;
+    uint32_t *sorted;
+    uint2 *info;
+    const uint2 *unsorted;     /* object and walk start, by leaf */
+    const uint32_t *grid_node;
     uint32_t cap;
 };
 
-/* the object pid at place `at` of the segment of a leaf node that starts at s0 */
-__device__ inline void gather_one(const GatherOut &o, const Frame &f, const double2 p, uint32_t s0, uint32_t at,
-                                  uint32_t pid, uint32_t leaf) {
-    const uint32_t i = s0 + at;
+/* a segment: the leaf grid and node, and where it starts */
+struct Segment {
+    uint32_t g, leaf, s0;
+};
+
+/* object v (id and walk start) at place `at` of a segment */
+__device__ inline void gather_one(const GatherOut &o, const Frame &f, const double2 p, const Segment &s, uint32_t at,
+                                  const uint2 v) {
+    const uint32_t i = s.s0 + at, pid = v.x;
+    o.sorted[i] = pid;
+    o.info[i] = make_uint2(v.y, s.g);
     o.sxy[i] = p;
     bool clamped = false;
     const long long X = fx_coord(p.x, f.k, f.X0, &clamped);
@@ -148,7 +163,7 @@ __device__ inline void gather_one(const GatherOut &o, const Frame &f, const doub
     o.sfpos[i] = fp;
     o.fpos[pid] = fp;
     if (o.sm) o.sm[i] = metres_per_degree(p.y, f);
-    o.rank[pid] = make_uint2(at < o.cap ? i : i | kDropped, leaf);
+    o.rank[pid] = make_uint2(at < o.cap ? i : i | kDropped, s.leaf);
 }
 
 /* A warp's segment of up to 32 K different ids: each lane counts the ids below
@@ -157,33 +172,31 @@ __device__ inline void gather_one(const GatherOut &o, const Frame &f, const doub
  * it; a bitonic network of the same segment is 15 to 28 stages, each waiting
  * for the one before. */
 template <int K>
-__device__ inline void rank_sort(const GatherOut &o, const Frame &f, const double2 *__restrict__ pts, uint32_t *seg,
-                                 uint32_t *buf, uint32_t n, uint32_t s0, uint32_t leaf) {
+__device__ inline void rank_sort(const GatherOut &o, const Frame &f, const double2 *__restrict__ pts,
+                                 uint32_t *buf, uint32_t n, const Segment &s) {
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t v[K], r[K];
+    uint2 v[K];
+    uint32_t r[K];
     double2 p[K];
 #pragma unroll
     for (int e = 0; e < K; ++e) {
         const uint32_t i = lane + 32 * e;
-        v[e] = i < n ? seg[i] : 0xffffffffu;
-        buf[i] = v[e];
+        v[e] = i < n ? o.unsorted[s.s0 + i] : make_uint2(0xffffffffu, 0u);
+        buf[i] = v[e].x;
         r[e] = 0;
     }
 #pragma unroll
     for (int e = 0; e < K; ++e)
-        if (lane + 32 * e < n) p[e] = pts[v[e]];
+        if (lane + 32 * e < n) p[e] = pts[v[e].x];
     __syncwarp();
     for (uint32_t j = 0; j < n; j += 4) {
         const uint4 q = *reinterpret_cast<const uint4 *>(buf + j);
 #pragma unroll
-        for (int e = 0; e < K; ++e) r[e] += (q.x < v[e]) + (q.y < v[e]) + (q.z < v[e]) + (q.w < v[e]);
+        for (int e = 0; e < K; ++e) r[e] += (q.x < v[e].x) + (q.y < v[e].x) + (q.z < v[e].x) + (q.w < v[e].x);
     }
 #pragma unroll
     for (int e = 0; e < K; ++e)
-        if (lane + 32 * e < n) {
-            seg[r[e]] = v[e];
-            gather_one(o, f, p[e], s0, r[e], v[e], leaf);
-        }
+        if (lane + 32 * e < n) gather_one(o, f, p[e], s, r[e], v[e]);
 }
 
 constexpr int kSortWarps = 8;
@@ -202,24 +215,20 @@ constexpr uint32_t kRankSortMax = 512;
 __global__ void __launch_bounds__(32 * kSortWarps) k_segsort_warp(const uint32_t *__restrict__ work,
                                                                   const uint32_t *__restrict__ grid_start,
                                                                   const uint32_t *__restrict__ grid_count,
-                                                                  uint32_t *__restrict__ sorted,
                                                                   const double2 *const *in, GatherOut o,
                                                                   Frame f, const DevCounters *cnt) {
     __shared__ __align__(16) uint32_t buf[kSortWarps][kWarpSortMax];
     const double2 *__restrict__ pts = *in;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
     const uint32_t nwork = cnt->n_leaf_work;
     for (uint32_t li = blockIdx.x * kSortWarps + w; li < nwork; li += gridDim.x * kSortWarps) {
         const uint32_t g = work[li];
         const uint32_t n = grid_count[g];
         if (n > kWarpSortMax) continue;
-        const uint32_t s0 = grid_start[g];
-        uint32_t *seg = sorted + s0;
-        const uint32_t leaf = o.obj[seg[0]].z; /* the node of grid g: one for all its objects */
-        __syncwarp();
-        if (n <= 32) rank_sort<1>(o, f, pts, seg, buf[w], n, s0, leaf);
-        else if (n <= 64) rank_sort<2>(o, f, pts, seg, buf[w], n, s0, leaf);
-        else rank_sort<4>(o, f, pts, seg, buf[w], n, s0, leaf);
+        const Segment s = {g, o.grid_node[g], grid_start[g]};
+        if (n <= 32) rank_sort<1>(o, f, pts, buf[w], n, s);
+        else if (n <= 64) rank_sort<2>(o, f, pts, buf[w], n, s);
+        else rank_sort<4>(o, f, pts, buf[w], n, s);
         __syncwarp();
     }
 }
@@ -233,7 +242,6 @@ constexpr uint32_t kBlockSortMax = 16384;
 __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restrict__ big,
                                                         const uint32_t *__restrict__ grid_start,
                                                         const uint32_t *__restrict__ grid_count,
-                                                        uint32_t *__restrict__ sorted,
                                                         const double2 *const *in, GatherOut o, Frame f,
                                                         DevCounters *cnt) {
     extern __shared__ __align__(16) uint32_t sbuf[];
@@ -242,41 +250,37 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
     for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
         const uint32_t g = big[bi];
         const uint32_t n = grid_count[g];
+        const Segment s = {g, o.grid_node[g], grid_start[g]};
+        const uint2 *seg = o.unsorted + s.s0;
         if (n > kBlockSortMax) {
             /* reported; the arrays are filled all the same, so that what
              * follows in this step reads objects */
             if (threadIdx.x == 0) atomicOr(&cnt->error_flags, GLINT_EF_SEGMENT_TOO_LARGE);
-            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-                gather_one(o, f, pts[sorted[grid_start[g] + i]], grid_start[g], i, sorted[grid_start[g] + i],
-                           o.obj[sorted[grid_start[g]]].z);
+            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) gather_one(o, f, pts[seg[i].x], s, i, seg[i]);
             continue;
         }
-        uint32_t *seg = sorted + grid_start[g];
-        const uint32_t leaf = o.obj[seg[0]].z;
         __syncthreads();
         if (n <= kRankSortMax) {
             const uint32_t parts = n <= kRankSortMax / 2 ? 4 : 2;
             const uint32_t i = threadIdx.x / parts, part = threadIdx.x % parts;
-            if (threadIdx.x < kRankSortMax) sbuf[threadIdx.x] = threadIdx.x < n ? seg[threadIdx.x] : 0xffffffffu;
-            __syncthreads();
-            const uint32_t v = sbuf[i];
+            if (threadIdx.x < kRankSortMax) sbuf[threadIdx.x] = threadIdx.x < n ? seg[threadIdx.x].x : 0xffffffffu;
+            const uint2 me = i < n ? seg[i] : make_uint2(0u, 0u);
+            const uint32_t v = me.x;
             double2 p = make_double2(0., 0.);
             if (i < n) p = pts[v];
+            __syncthreads();
             uint32_t r = 0;
             for (uint32_t j = 4 * part; j < n; j += 4 * parts) {
                 const uint4 q = *reinterpret_cast<const uint4 *>(sbuf + j);
                 r += (q.x < v) + (q.y < v) + (q.z < v) + (q.w < v);
             }
             for (uint32_t d = 1; d < parts; d <<= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
-            if (i < n && part == 0) {
-                seg[r] = v;
-                gather_one(o, f, p, grid_start[g], r, v, leaf);
-            }
+            if (i < n && part == 0) gather_one(o, f, p, s, r, me);
             continue;
         }
         uint32_t P = 1024;
         while (P < n) P <<= 1;
-        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) sbuf[i] = i < n ? seg[i] : 0xffffffffu;
+        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) sbuf[i] = i < n ? seg[i].x : 0xffffffffu;
         __syncthreads();
         for (uint32_t k = 2; k <= P; k <<= 1) {
             for (uint32_t j = k >> 1; j > 0; j >>= 1) {
@@ -292,8 +296,14 @@ __global__ void __launch_bounds__(1024) k_segsort_block(const uint32_t *__restri
             }
         }
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            seg[i] = sbuf[i];
-            gather_one(o, f, pts[sbuf[i]], grid_start[g], i, sbuf[i], leaf);
+            const uint2 v = seg[i];
+            uint32_t lo = 0, hi = n; /* v's place: sbuf[lo] <= v < sbuf[hi] */
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) / 2;
+                if (sbuf[mid] <= v.x) lo = mid;
+                else hi = mid;
+            }
+            gather_one(o, f, pts[v.x], s, lo, v);
         }
         __syncthreads();
     }
@@ -332,7 +342,8 @@ cudaError_t launch_partition(glint_ctx *c) {
     const uint32_t N = c->N, G = c->G;
     /* the last step's leaf-major order is the descent's processing order */
     k_descend<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_in, c->d_sorted, N, c->d_nodes, c->S, G, c->x_buffer,
-                                                           c->y_buffer, c->d_obj, c->d_grid_count, c->d_cnt);
+                                                           c->y_buffer, c->d_obj, c->d_grid_node, c->d_grid_count,
+                                                           c->d_cnt);
     LeafScan ls;
     ls.start = ScanStore{c->d_grid_start, true};
     ls.work = c->d_leaf_work;
@@ -341,7 +352,7 @@ cudaError_t launch_partition(glint_ctx *c) {
     ls.warp_limit = kWarpSortMax;
     ls.cnt = c->d_cnt;
     scan_launch(ScanWords{c->d_grid_count, true}, ls, G, &c->d_cnt->grids_used, c->d_scan_tmp, s);
-    k_scatter<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_obj, N, c->d_grid_start, c->d_sorted);
+    k_scatter<<<grid_for(N, 256, 152u * 8u), 256, 0, s>>>(c->d_obj, N, c->d_grid_start, c->d_seg);
     GatherOut o;
     o.sxy = c->d_sxy;
     o.sipos = c->d_sipos;
@@ -350,12 +361,15 @@ cudaError_t launch_partition(glint_ctx *c) {
     o.sm = c->cfg.precision_mode == 1 ? nullptr : c->d_sm;
     o.fpos = c->d_fpos;
     o.rank = c->d_rank;
-    o.obj = c->d_obj;
+    o.sorted = c->d_sorted;
+    o.info = c->d_info;
+    o.unsorted = c->d_seg;
+    o.grid_node = c->d_grid_node;
     o.cap = c->cap;
     k_segsort_warp<<<grid_for(N, 16 * kSortWarps, 152u * 8u), 32 * kSortWarps, 0, s>>>(
-        c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_in, o, c->frame, c->d_cnt);
+        c->d_leaf_work, c->d_grid_start, c->d_grid_count, c->d_in, o, c->frame, c->d_cnt);
     k_segsort_block<<<304, 1024, kBlockSortMax * sizeof(uint32_t), s>>>(
-        c->d_big, c->d_grid_start, c->d_grid_count, c->d_sorted, c->d_in, o, c->frame, c->d_cnt);
+        c->d_big, c->d_grid_start, c->d_grid_count, c->d_in, o, c->frame, c->d_cnt);
     return cudaGetLastError();
 }
 

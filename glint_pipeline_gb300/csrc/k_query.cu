@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(128) k_search_objects(ObjectSearch o, const ui
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 32; i < npids; i += gridDim.x * blockDim.x / 32) {
         const uint32_t p = pids[i];
         if (p >= o.s.N) continue;
-        const uint32_t rank = a.rank[p].x, r = rank & ~kDropped, g = a.obj[p].x;
+        const uint32_t rank = a.rank[p].x, r = rank & ~kDropped, g = a.info[r].y;
         const uint32_t s0 = a.grid_start[g], k = min(a.grid_start[g + 1] - s0, a.cap);
         const bool stored = !(rank & kDropped);
         for (uint32_t j = lane; stored && j < k; j += 32) {

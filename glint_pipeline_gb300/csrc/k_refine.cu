@@ -74,7 +74,7 @@ RefineArgs refine_args(glint_ctx *c) {
     a.sfpos = c->d_sfpos;
     a.sc = c->d_sc;
     a.f = c->frame;
-    a.obj = c->d_obj;
+    a.info = c->d_info;
     a.rank = c->d_rank;
     a.qstart = c->d_qstart;
     a.qcount = c->d_qcount;

@@ -37,7 +37,7 @@ struct RefineArgs {
     const longlong2 *sipos;    /* fixed-point coordinates, leaf-major */
     const float2 *sfpos;       /* FP32 coordinates, leaf-major */
     const float *sc;           /* screening scale cx, leaf-major */
-    const uint4 *obj;          /* by object id: leaf grid, .. */
+    const uint2 *info;         /* by rank: .., leaf grid */
     const uint2 *rank;         /* by object id: leaf-major rank (kDropped: not stored), leaf node */
     const uint32_t *qstart, *qcount;
     const uint32_t *qlist;
@@ -168,7 +168,7 @@ __device__ inline bool queued_contact(const RefineArgs &a, QEntry &q, RefineTall
          * order; keep only one event */
         const uint32_t qid = (uint32_t)(q.prio >> 36) & 0x7ffffffu;
         const uint32_t mid = pair_a(q.pw) == qid ? pair_b(q.pw) : pair_a(q.pw);
-        if (has_check(a, mid, a.obj[qid].x) && pair_fp64(a, r2, r1)) return false;
+        if (has_check(a, mid, a.info[r1].y) && pair_fp64(a, r2, r1)) return false;
     }
     const float2 A = a.sfpos[r1], B = a.sfpos[r2];
     q.v = make_uint4(__float_as_uint(A.x), __float_as_uint(A.y), __float_as_uint(B.x), __float_as_uint(B.y));
@@ -516,7 +516,7 @@ __device__ inline void refine_item(const RefineArgs &a, uint32_t g, uint32_t chu
                     t.hits += hit ? 1 : 0;
                     /* mm's test comes first in the reference's order when
                      * mm < q; keep only one event */
-                    if (hit && dup && has_check(a, mm, a.obj[Q0].x)) {
+                    if (hit && dup && has_check(a, mm, a.info[R0].y)) {
                         const float cm = m.cb[j].x;
                         const float d2 = screen_q(f, P.x - X, P.y - Y, cm);
                         const float b2 = pair_band(f, cm, fmaxf(o.Mx, fabsf(X)), fmaxf(o.My, fabsf(Y)));

@@ -381,8 +381,10 @@ __device__ inline float f_of_d(double d) {
     return (float)d;
 }
 
-/* metres per unit along x at latitude lat, FP32 (within 9u of exact): the
- * angle from the pole as an integer, converted with one rounding */
+/* metres per unit along x at latitude lat, FP32 (within 9u of exact), without
+ * its sign, which is negative beyond 90 degrees: distances square it and bands
+ * and ranges want its size.  The angle from the pole as an integer, converted
+ * with one rounding */
 __device__ inline float c_of_lat(double lat, const Frame &f) {
     bool clamped = false;
     long long a = fx_round(lat, f.k, &clamped);
@@ -390,7 +392,7 @@ __device__ inline float c_of_lat(double lat, const Frame &f) {
     const long long ninety = 90ll << f.k;
     if (a == ninety && fabs(lat) == 90.0) a = 89ll << f.k;
     const float t = fx_to_f((ninety - a) >> f.ksh);
-    return clamped ? __int_as_float(0x7fc00000) : sinf(t * f.kang) * f.kc;
+    return clamped ? __int_as_float(0x7fc00000) : fabsf(sinf(t * f.kang) * f.kc);
 }
 
 /* metres per degree of longitude at latitude lat in FP64, 1 / L to a few

@@ -1,0 +1,48 @@
+"""Contacts where the longitude scale is unusual: beyond 90 degrees of latitude,
+where it is negative."""
+import numpy as np
+import pytest
+
+from glint_pipeline_gb300 import Configuration, DeviceBench
+from oracle.bindings import Oracle, make_config
+from test_gpu_parity import compare_meetings
+
+pytestmark = pytest.mark.gpu
+
+PI = 3.14159265  # the reference's (util/util.h:38)
+METRES = 40076000.0 / 360.0  # a degree at the equator
+
+
+def run(box, pts, steps, precision_mode, **args):
+    args = dict(num_objects=len(pts), num_meeting_buckets=1 << 20, min_meet_time=1, **args)
+    o = Oracle(make_config(**args), box, pts)
+    g = DeviceBench(Configuration(precision_mode=precision_mode, **args), box, pts)
+    far = pts.copy()  # last step: everyone apart, so that the contacts are reported
+    far[:, 1] = box[1] + (box[3] - box[1]) * (np.arange(len(pts)) + 0.5) / len(pts)
+    cross = contacts = 0
+    for t in range(steps + 1):
+        p = pts if t < steps else far
+        o.step(p, t)
+        st = g.step(p, t)
+        c = o.counts()
+        assert (st.checks, st.candidates, st.contacts) == (c.grid_check_counter, c.candidates, c.contacts), f"step {t}"
+        compare_meetings(o.meetings(), g.meetings(), t)
+        if t < steps:
+            cross, contacts = max(cross, int(st.cross_checks)), max(contacts, int(st.contacts))
+    g.close()
+    o.close()
+    return cross, contacts
+
+
+@pytest.mark.parametrize("precision_mode", [0, 1])
+def test_latitudes_beyond_ninety(precision_mode):
+    """A map across 90 degrees; the objects lie about the boundary between two
+    leaves that start above it."""
+    rng = np.random.default_rng(90)
+    n = 1200
+    pts = np.empty((n, 2))
+    pts[:, 0] = 0.5 + rng.uniform(-0.02, 0.02, n)
+    pts[:, 1] = 90.3 + rng.uniform(-0.0005, 0.0005, n)
+    pts[0], pts[1] = (0.01, 89.6), (0.99, 90.55)
+    cross, contacts = run(np.array([0.0, 89.5, 1.0, 90.6]), pts, 3, precision_mode, grid_capacity=600)
+    assert cross > 0 and contacts > 100

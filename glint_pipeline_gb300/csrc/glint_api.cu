@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <vector>
 
 #include "glint_internal.cuh"
@@ -240,6 +241,8 @@ Frame make_frame(const glint_box &mbr, const glint_schema_node &root, double r, 
     f.a0 = std::isfinite(mid) ? (90.0 - mid) * kPIh / 180.0 : 0.0;
     f.s0 = std::sin(f.a0);
     f.c0 = std::cos(f.a0);
+    /* near a pole the expansion's remainder is not small beside the sin */
+    if (!(std::fabs(f.s0) >= 0.1)) f.a0 = std::numeric_limits<double>::quiet_NaN();
     return f;
 }
 

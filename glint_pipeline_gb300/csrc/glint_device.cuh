@@ -318,7 +318,7 @@ struct Frame {
     float r2;            /* r^2 */
     float band0;         /* 64 u r^2 */
     float band1;         /* 4 r */
-    double a0, s0, c0;   /* an angle near the map's middle latitude, its sin and cos */
+    double a0, s0, c0;   /* the angle of the map's middle latitude (NaN: no expansion), its sin and cos */
 };
 
 /* a node box in fixed point: low x, low y, high x, high y */
@@ -395,12 +395,15 @@ __device__ inline float c_of_lat(double lat, const Frame &f) {
     return clamped ? __int_as_float(0x7fc00000) : fabsf(sinf(t * f.kang) * f.kc);
 }
 
-/* metres per degree of longitude at latitude lat in FP64, 1 / L to a few
- * 2^-50: the FP64 form of the refine stage decides with it outside a band of
- * 2^-36, and takes the reference's own L inside.  Within 0.02 rad (127 km) of
- * the frame's middle the sin is its Taylor expansion there to the fifth
- * power (remainder below 0.02^6 / 720 = 9e-14): 12 FP64 operations where the
- * library's sin and L's divisions are about 60. */
+/* metres per degree of longitude at latitude lat in FP64, 1 / L to 2^-43: the
+ * FP64 form of the refine stage decides with it outside a band of 2^-36, and
+ * takes the reference's own L inside.  Within 0.02 rad (127 km) of the frame's
+ * middle the sin is its Taylor expansion there to the fifth power: 12 FP64
+ * operations where the library's sin and L's divisions are about 60.  Its
+ * remainder is 0.02^6 / 720 = 9e-14 of the sin at the middle, s0, and 0.02^7 /
+ * 5040 = 3e-16.  Frames with |s0| below 0.1 (the middle within 5.7 degrees of
+ * a pole) have no expansion (a0 is NaN): elsewhere the sin itself is at least
+ * 0.8 |s0|, and the relative error at most 1.2e-13. */
 __device__ inline double metres_per_degree(double lat, const Frame &f) {
     const double la = fabs(lat) == 90.0 ? 89.0 : fabs(lat);
     const double x = __dmul_rn(__dsub_rn(90.0, la), kPI / 180.0), d = __dsub_rn(x, f.a0);

@@ -141,9 +141,10 @@ __device__ inline bool has_check(const RefineArgs &a, uint32_t obj, uint32_t gid
 
 /* The FP64 form's test: the squared distance in metres, in FP64 without the
  * reference's two divisions and square root (about 8 FP64 operations instead
- * of 45; FP64 issues at 1/64 of the FP32 rate).  Its error is a few 2^-52 of
- * the result, the band around r^2 is 2^-36 of it, so outside the band its
- * decision is the reference's; inside, the reference's own expression
+ * of 45; FP64 issues at 1/64 of the FP32 rate).  Its error is at most
+ * 2^-41 of the result (the longitude scale's 2^-43 twice, metres_per_degree,
+ * and a few 2^-52), the band around r^2 is 2^-36 of it, so outside the band
+ * its decision is the reference's; inside, the reference's own expression
  * decides.  The band contains every pair that point_le_exact re-takes with
  * the correctly rounded sin (|d - r| <= 2^-38 r), so that count stays. */
 __device__ inline bool pair_fp64(const RefineArgs &a, uint32_t r1, uint32_t r2) {

@@ -1,5 +1,6 @@
 """Contacts where the longitude scale is unusual: beyond 90 degrees of latitude,
-where it is negative."""
+where it is negative, and close to a pole, where it is small beside its value at
+the map's middle."""
 import numpy as np
 import pytest
 
@@ -46,3 +47,23 @@ def test_latitudes_beyond_ninety(precision_mode):
     pts[0], pts[1] = (0.01, 89.6), (0.99, 90.55)
     cross, contacts = run(np.array([0.0, 89.5, 1.0, 90.6]), pts, 3, precision_mode, grid_capacity=600)
     assert cross > 0 and contacts > 100
+
+
+@pytest.mark.parametrize("precision_mode", [0, 1])
+def test_pole_beside_a_lower_middle(precision_mode):
+    """Pairs 4e-12 to 7.5e-12 of the reach inside it, 640 m from the pole on a
+    map whose middle is 1.149 degrees away."""
+    pairs, r = 60, 0.5
+    x = 1.0e-4 + np.arange(pairs) * (2 * r / (METRES * 180 / PI))  # angles from the pole
+    lat = 90.0 - x * 180 / PI
+    delta = np.linspace(4.0e-12, 7.5e-12, pairs)
+    dx = r * (1 - delta) / (np.sin((90.0 - lat) * (PI / 180)) * METRES)
+    pts = np.empty((2 * pairs + 8, 2))
+    pts[0:2 * pairs:2, 0] = 0.0
+    pts[1:2 * pairs:2, 0] = dx
+    pts[0:2 * pairs:2, 1] = pts[1:2 * pairs:2, 1] = lat
+    mid = 90.0 - 0.02005 * 180 / PI
+    box = np.array([0.0, 2 * mid - 89.999, 40.0, 89.999])
+    pts[2 * pairs:, 0], pts[2 * pairs:, 1] = 39.0, box[1] + 0.1 * (1 + np.arange(8))
+    _, contacts = run(box, pts, 3, precision_mode, grid_capacity=len(pts) - 4, reach_distance=r)
+    assert contacts == pairs

@@ -384,14 +384,21 @@ __device__ inline float f_of_d(double d) {
 /* metres per unit along x at latitude lat, FP32 (within 9u of exact), without
  * its sign, which is negative beyond 90 degrees: distances square it and bands
  * and ranges want its size.  The angle from the pole as an integer, converted
- * with one rounding */
+ * with one rounding; below 2^25 units, where a unit and a half (the latitude's
+ * rounding and the shift) is not small beside it, from the latitude itself */
+constexpr long long kPoleUnits = 1ll << 25;
 __device__ inline float c_of_lat(double lat, const Frame &f) {
     bool clamped = false;
     long long a = fx_round(lat, f.k, &clamped);
     a = a < 0 ? -a : a;
     const long long ninety = 90ll << f.k;
     if (a == ninety && fabs(lat) == 90.0) a = 89ll << f.k;
-    const float t = fx_to_f((ninety - a) >> f.ksh);
+    const long long n = (ninety - a) >> f.ksh;
+    float t = fx_to_f(n);
+    if (n < kPoleUnits && n > -kPoleUnits) {
+        const double la = fabs(lat) == 90.0 ? 89.0 : fabs(lat);
+        t = scalbnf((float)__dmul_rn(__dsub_rn(90.0, la), f.S), -f.ksh);
+    }
     return clamped ? __int_as_float(0x7fc00000) : fabsf(sinf(t * f.kang) * f.kc);
 }
 

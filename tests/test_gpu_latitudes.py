@@ -1,6 +1,6 @@
 """Contacts where the longitude scale is unusual: beyond 90 degrees of latitude,
 where it is negative, and close to a pole, where it is small beside its value at
-the map's middle."""
+the map's middle and beside the fixed-point unit."""
 import numpy as np
 import pytest
 
@@ -67,3 +67,23 @@ def test_pole_beside_a_lower_middle(precision_mode):
     pts[2 * pairs:, 0], pts[2 * pairs:, 1] = 39.0, box[1] + 0.1 * (1 + np.arange(8))
     _, contacts = run(box, pts, 3, precision_mode, grid_capacity=len(pts) - 4, reach_distance=r)
     assert contacts == pairs
+
+
+@pytest.mark.parametrize("precision_mode", [0, 1])
+def test_pole_of_a_whole_globe(precision_mode):
+    """Pairs just beyond the reach, 1.7 m from the pole, where a latitude half a
+    unit off in the globe's fixed-point frame is 1.5e-5 of the distance to the
+    pole off."""
+    pairs, r = 12, 10.0
+    unit = 2.0 ** -31
+    lat = 90.0 - (np.round(np.linspace(1.47e-5, 1.53e-5, pairs) / unit) + 0.5) * unit
+    dx = r * (1 + np.linspace(1e-7, 2e-6, pairs)) / (np.sin((90.0 - lat) * (PI / 180)) * METRES)
+    assert dx.max() < 355.0
+    pts = np.empty((2 * pairs + 8, 2))
+    pts[0:2 * pairs:2, 0] = -dx / 2
+    pts[1:2 * pairs:2, 0] = dx / 2
+    pts[0:2 * pairs:2, 1] = pts[1:2 * pairs:2, 1] = lat
+    pts[2 * pairs:, 0], pts[2 * pairs:, 1] = 39.0, -0.1 * (1 + np.arange(8))
+    _, contacts = run(np.array([-180.0, -90.0, 180.0, 90.0]), pts, 2, precision_mode, grid_capacity=len(pts) - 4,
+                      reach_distance=r)
+    assert contacts > 0

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "glint_internal.cuh"
+#include "step_points.h"
 
 namespace glint {
 void partition_set_attributes();
@@ -633,12 +634,11 @@ glint_status glint_get_capacities(const glint_ctx *c, uint32_t *sc, uint32_t *gc
 
 namespace glint {
 
-/* A step's points: host points are copied into the context's buffer; points
- * in device memory on a 16-byte boundary are read in place (a copy of theirs
- * was 10 us of a 1M-object step's 700); others are copied too. */
+/* A step's points: read in place where they may be (a copy of theirs was 10 us
+ * of a 1M-object step's 700), else copied into the context's buffer. */
 cudaError_t step_input(glint_ctx *c, const double *points, bool host) {
     c->h_input->pts = c->d_pts;
-    if (!host && c->input_device && ((uintptr_t)points & 15) == 0) {
+    if (!host && c->points_in_place) {
         c->h_input->pts = reinterpret_cast<const double2 *>(points);
         return cudaSuccess;
     }
@@ -713,7 +713,7 @@ bool device_points(glint_ctx *c, const void *p) {
         c->last_error = "step input: not device memory";
         return false;
     }
-    c->input_device = at.type == cudaMemoryTypeDevice;
+    c->points_in_place = points_in_place(at, c->device, p);
     return true;
 }
 
@@ -972,10 +972,9 @@ glint_status glint_get_buckets(glint_ctx *c, uint64_t *keys, uint32_t *starts, f
 } /* extern "C" */
 
 namespace glint {
-/* the step on device points, never through the captured graph (whose input
- * buffer is fixed) */
-glint_status enqueue_device_step_plain(glint_ctx *c, const double *d_points, uint32_t cur_time) {
-    c->input_device = true; /* the pipe's own buffers */
+/* the step on the pipe's own device buffers, which are read in place */
+glint_status enqueue_pipe_step(glint_ctx *c, const double *d_points, uint32_t cur_time) {
+    c->points_in_place = true;
     return enqueue_step(c, d_points, false, cur_time);
 }
 } // namespace glint

@@ -176,7 +176,7 @@ struct StepTimers {
     bool created = false;
 };
 
-glint_status enqueue_device_step_plain(glint_ctx *c, const double *d_points, uint32_t cur_time);
+glint_status enqueue_pipe_step(glint_ctx *c, const double *d_points, uint32_t cur_time);
 /* true (and last_error set) when the context was turned to serving only */
 bool serve_only_refused(glint_ctx *c, const char *what);
 
@@ -209,7 +209,7 @@ struct glint_ctx {
     uint2 *d_seg = nullptr;                /* [N] object and last_valid node by leaf grid, unsorted in a leaf */
     uint2 *d_info = nullptr;               /* [N] leaf-major: the node a walk starts from (kNoWalk: none), leaf grid */
     uint32_t *d_grid_node = nullptr;       /* [G] the leaf node of each grid that holds objects */
-    bool input_device = false;             /* the step's input is device (not managed) memory */
+    bool points_in_place = false;          /* the step's device points are read where they lie (step_points.h) */
     uint32_t *d_grid_count = nullptr;      /* [G+1] */
     uint32_t *d_grid_start = nullptr;      /* [G+1] */
     uint32_t *d_sorted = nullptr;          /* [N] leaf-major order; the next descent's processing order */

@@ -157,7 +157,7 @@ extern "C" glint_status glint_pipe_submit(glint_pipe *p, const double *points, u
     if (fs != GLINT_OK) return fs;
     /* 3. the step and the export of its meetings */
     cudaStreamWaitEvent(c->stream, p->copied[slot], 0);
-    const glint_status st = glint::enqueue_device_step_plain(c, p->d_in[slot], cur_time);
+    const glint_status st = glint::enqueue_pipe_step(c, p->d_in[slot], cur_time);
     if (st != GLINT_OK) return st;
     /* the staging buffer is free once its last copy to the host is done */
     if (p->used[slot]) cudaStreamWaitEvent(c->stream, p->fetched[slot], 0);

@@ -206,7 +206,9 @@ glint_status glint_step(glint_ctx *ctx, const double *points, uint32_t cur_time,
 /* the same with points already in device memory; enqueues the step on the
  * context's stream and returns without waiting.  d_points must be device (or
  * managed) memory, else GLINT_ERR_INVALID_ARGUMENT before anything is
- * enqueued */
+ * enqueued.  The step reads the points where they lie (16-byte aligned memory
+ * of the context's GPU) or copies them first (any other): leave them unchanged
+ * and allocated until the step has completed on the context's stream. */
 glint_status glint_step_device(glint_ctx *ctx, const double *d_points, uint32_t cur_time);
 /* waits for enqueued steps; stats of the last one (may be NULL) */
 glint_status glint_sync(glint_ctx *ctx, glint_step_stats *stats);
@@ -584,7 +586,8 @@ glint_status glint_precision_probe(glint_ctx *ctx, uint32_t stride, glint_precis
  * the refine stage, one refine launch over the work items of all regions in
  * precision_mode 1 (regions in mode 0 refine on their own streams), then
  * every region's remaining stages.  The graph takes the points' addresses when
- * it runs, so they may change from call to call.  The call returns
+ * it runs, so they may change from call to call; as in glint_step_device the
+ * points stay unchanged until the timestep has completed.  The call returns
  * without waiting (after the previous timestep is done); glint_batch_sync
  * waits for it and runs each region's automatic flush, filling stats[r] when
  * stats is not NULL.  glint_batch_region gives a region's context for its

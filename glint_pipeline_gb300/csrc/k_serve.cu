@@ -35,11 +35,10 @@
 #include <vector>
 
 #include "scan.cuh"
+#include "serve_queue.h"
 #include "store_codec.cuh"
 
 namespace glint {
-
-constexpr uint32_t kMaxHops = 8;
 
 struct SlotParam {
     uint32_t t_start, t_end, window, pad;
@@ -441,28 +440,6 @@ struct MarkOut {
 
 using namespace glint;
 
-struct PendingQuery {
-    uint64_t ticket;
-    std::vector<uint32_t> seeds;
-    uint32_t hops, t_start, t_end;
-};
-
-struct SlotState {
-    bool busy = false;
-    uint64_t ticket = 0;
-    uint32_t hops = 0, hop = 0, frontier = 0;
-    const uint32_t *front_ids = nullptr; /* device: the last hop's part of the result list, or the seeds */
-    uint64_t reached = 0; /* seeds and every hop's new objects so far */
-    std::vector<uint32_t> ids;
-    uint64_t hop_end[kMaxHops] = {};
-};
-
-struct FinishedQuery {
-    std::vector<uint32_t> ids;
-    uint64_t hop_end[kMaxHops];
-    uint64_t keys_scanned;
-};
-
 struct glint_server {
     glint_ctx *ctx = nullptr;
     uint32_t slots = 0;
@@ -614,6 +591,7 @@ extern "C" glint_status glint_server_submit(glint_server *v, const glint_query *
 
 static glint_status server_fail(glint_server *v, cudaError_t e, const char *where) {
     v->ctx->last_error = std::string("server ") + where + ": " + cudaGetErrorString(e);
+    cudaGetLastError(); /* a refused allocation is this call's error, not the next launch's */
     return e == cudaErrorMemoryAllocation ? GLINT_ERR_OUT_OF_MEMORY : GLINT_ERR_CUDA;
 }
 
@@ -647,27 +625,13 @@ extern "C" glint_status glint_server_step(glint_server *v, uint32_t *n_active, u
     }
     const size_t at_blocks = ctl.add(bd);
 
-    /* admission: queued queries into free slots; their seeds, each once, are
-     * their first frontier */
-    std::vector<uint32_t> admitted, seeds, sprefix(1, 0);
-    for (uint32_t k = 0; k < v->slots && !v->queue.empty(); ++k) {
-        SlotState &st = v->state[k];
-        if (st.busy) continue;
-        PendingQuery q = std::move(v->queue.front());
-        v->queue.pop_front();
-        std::sort(q.seeds.begin(), q.seeds.end());
-        q.seeds.erase(std::unique(q.seeds.begin(), q.seeds.end()), q.seeds.end());
-        while (!q.seeds.empty() && q.seeds.back() >= N) q.seeds.pop_back();
-        st = SlotState();
-        st.busy = true;
-        st.ticket = q.ticket;
-        st.hops = q.hops;
-        st.frontier = (uint32_t)q.seeds.size();
-        st.reached = st.frontier;
-        v->hparam[k] = SlotParam{q.t_start, q.t_end, (q.t_start == 0 && q.t_end == 0) ? 0u : 1u, 0u};
-        admitted.push_back(k);
-        seeds.insert(seeds.end(), q.seeds.begin(), q.seeds.end());
-        sprefix.push_back((uint32_t)seeds.size());
+    /* undone at every return before the round's launches have run */
+    Admission adm(v->queue, v->state);
+    adm.take(N);
+    const std::vector<uint32_t> &admitted = adm.slots, &seeds = adm.seeds, &sprefix = adm.sprefix;
+    for (size_t i = 0; i < admitted.size(); ++i) {
+        const PendingQuery &q = adm.query(i);
+        v->hparam[admitted[i]] = SlotParam{q.t_start, q.t_end, (q.t_start == 0 && q.t_end == 0) ? 0u : 1u, 0u};
     }
     const size_t at_seeds = ctl.add(seeds), at_sprefix = ctl.add(sprefix), at_admitted = ctl.add(admitted);
 
@@ -759,6 +723,7 @@ extern "C" glint_status glint_server_step(glint_server *v, uint32_t *n_active, u
         cudaMemcpyAsync(v->h_out, v->out, sizeof(unsigned long long) * (v->slots + (size_t)A + 1),
                         cudaMemcpyDeviceToHost, s);
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return server_fail(v, e, "hop");
+        adm.keep();
         const unsigned long long *off = v->h_out + v->slots;
         /* the new ids, in stages, to their queries */
         for (uint32_t i = 0; i < A; ++i)
@@ -860,7 +825,10 @@ extern "C" glint_status glint_query_batch(glint_ctx *c, const glint_query *qs, u
     std::vector<char> got(nq, 0);
     while (finished < nq) {
         const glint_status st = glint_server_step(v, nullptr, nullptr);
-        if (st != GLINT_OK) return st;
+        if (st != GLINT_OK) {
+            cancel_queries(tickets, v->queue, v->state, v->done);
+            return st;
+        }
         for (uint32_t q = 0; q < nq; ++q) {
             if (got[q]) continue;
             int done = 0;

@@ -382,7 +382,8 @@ __global__ void k_serve_seed(const uint32_t *__restrict__ seeds, const uint32_t 
     }
 }
 
-/* the marks of all active slots, slot after slot, as one scan: each word's
+/* the marks of the active slots, slot after slot, as one scan for each group of
+ * slots whose objects a 32-bit sum counts (mark_group): each word's
  * count of marks, then its ids at its place of the result list; a slot's first
  * place is where its ids start.  Pull hops read the reached sets as they stood
  * before the hop, so their marks join them here (a walk's marks are in). */
@@ -418,18 +419,22 @@ struct MarkOut {
     uint32_t *ids;             /* the result list */
     unsigned long long *off;   /* [A + 1] */
     uint32_t A;
-    __device__ void total(uint32_t, uint32_t sum) const { off[A] = sum; }
+    bool later;                /* off[0] holds the total of the groups of slots before this one */
+    __device__ unsigned long long before() const { return later ? off[0] : 0ull; }
+    __device__ void total(uint32_t, uint32_t sum) const { off[A] = before() + sum; }
     __device__ void store(uint32_t base, uint32_t n, const uint32_t (&v)[kScanItems],
                           const uint32_t (&o)[kScanItems]) const {
         if (base >= n) return;
         const uint32_t r = base / in.words, w0 = base - r * in.words;
-        if (w0 == 0) off[r] = o[0];
+        const unsigned long long b = before();
+        if (w0 == 0 && !(later && r == 0)) off[r] = b + o[0];
         const uint32_t *f = in.word(base);
         uint32_t *vis = visited + (size_t)in.active[r] * in.words + w0;
 #pragma unroll
         for (int k = 0; k < kScanItems; ++k) {
             if (!v[k]) continue;
-            uint32_t m = f[k], at = o[k];
+            uint32_t m = f[k];
+            unsigned long long at = b + o[k];
             vis[k] |= m;
             for (; m; m &= m - 1) ids[at++] = (w0 + k) * 32 + (uint32_t)__ffs(m) - 1;
         }
@@ -517,23 +522,21 @@ extern "C" glint_status glint_server_create(glint_ctx *c, uint32_t max_slots, gl
     cudaSetDevice(c->device);
     glint_server *v = new glint_server();
     v->ctx = c;
-    /* whole scan threads per slot */
-    v->words = (uint32_t)((((uint64_t)c->N + 31) / 32 + kScanItems - 1) / kScanItems * kScanItems);
+    static_assert(kScanItems == 8, "slot_words");
+    v->words = slot_words(c->N);
     /* admission by memory: a slot costs its two bitmaps and its part of the
      * two result lists */
     const size_t slot_bytes = sizeof(uint32_t) * (2 * (size_t)v->words + 2 * (size_t)c->N) + 64;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     const size_t fit = (free_b / 2) / slot_bytes;
-    /* the marks of all slots are one scan of 32-bit length */
-    const size_t most = std::max<size_t>(1, 0xf0000000ull / v->words);
-    v->slots = (uint32_t)std::min<size_t>(std::min<size_t>(max_slots, most), std::max<size_t>(fit, 1));
+    v->slots = (uint32_t)std::min<size_t>(max_slots, std::max<size_t>(fit, 1));
     const uint32_t S = v->slots;
     cudaError_t e = cudaSuccess;
     auto A = [&](void **p, size_t n) {
         if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1);
     };
-    const size_t scan_bytes = scan_tmp_bytes((size_t)v->words * S);
+    const size_t scan_bytes = scan_tmp_bytes((size_t)v->words * std::min(S, mark_group(c->N)));
     A((void **)&v->visited, sizeof(uint32_t) * (size_t)v->words * S);
     A((void **)&v->fresh, sizeof(uint32_t) * (size_t)v->words * S);
     A((void **)&v->ids[0], sizeof(uint32_t) * (size_t)c->N * S);
@@ -714,12 +717,16 @@ extern "C" glint_status glint_server_step(glint_server *v, uint32_t *n_active, u
             k_serve_pull<<<grid_for((uint64_t)b.A * ((N + 31) / 32), 8, 152u * 16u), 256, 0, s>>>(b);
         }
         MarkOut mo;
-        mo.in = MarkIn{v->fresh, a.active, v->words};
         mo.visited = v->visited;
         mo.ids = v->ids[v->side];
-        mo.off = v->out + v->slots;
-        mo.A = A;
-        scan_launch(mo.in, mo, v->words * A, nullptr, v->scan_tmp, s);
+        const uint32_t group = mark_group(N);
+        for (uint32_t r = 0; r < A; r += group) {
+            mo.in = MarkIn{v->fresh, a.active + r, v->words};
+            mo.off = v->out + v->slots + r;
+            mo.A = std::min(group, A - r);
+            mo.later = r != 0;
+            scan_launch(mo.in, mo, v->words * mo.A, nullptr, v->scan_tmp, s);
+        }
         cudaMemcpyAsync(v->h_out, v->out, sizeof(unsigned long long) * (v->slots + (size_t)A + 1),
                         cudaMemcpyDeviceToHost, s);
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return server_fail(v, e, "hop");

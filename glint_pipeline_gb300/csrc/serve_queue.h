@@ -15,6 +15,18 @@
 namespace glint {
 
 constexpr uint32_t kMaxHops = 8;
+/* seeds of one round, numbered in 32 bits by grids of up to 2^28 threads */
+constexpr uint64_t kMaxRoundSeeds = 0xf0000000ull;
+
+/* a slot's bitmap words: whole scan threads of eight */
+inline uint32_t slot_words(uint32_t N) { return (uint32_t)(((uint64_t)N + 255) / 256 * 8); }
+
+/* The slots whose marks one scan counts: each marks up to N objects, and the
+ * scan's sums, like its length, have 32 bits.  429 at 10M objects, 64 at 2^26 -
+ * 1: a round of the default server is one scan at every size. */
+inline uint32_t mark_group(uint32_t N) {
+    return (uint32_t)std::min<uint64_t>(0xffffffffull / std::max(N, 1u), 0xf0000000ull / std::max(slot_words(N), 8u));
+}
 
 struct PendingQuery {
     uint64_t ticket;
@@ -55,12 +67,14 @@ public:
         for (size_t i = taken_.size(); i-- > 0;) queue_.push_front(std::move(taken_[i]));
     }
 
-    /* seeds from N on are no objects */
-    void take(uint32_t N) {
+    /* seeds from N on are no objects; a query whose seeds would be too many
+     * beside the others' waits for the next round */
+    void take(uint32_t N, uint64_t max_seeds = kMaxRoundSeeds) {
         taken_.reserve(std::min(queue_.size(), state_.size()));
         slots.reserve(taken_.capacity());
         for (uint32_t k = 0; k < state_.size() && !queue_.empty(); ++k) {
             if (state_[k].busy) continue;
+            if (!seeds.empty() && seeds.size() + queue_.front().seeds.size() > max_seeds) break;
             taken_.push_back(std::move(queue_.front()));
             queue_.pop_front();
             PendingQuery &q = taken_.back();

@@ -60,6 +60,30 @@ int main() {
     CHECK(queue.size() == 2 && queue[0].ticket == 4);
     CHECK(state[0].ticket == 1 && state[2].ticket == 2 && state[3].ticket == 3);
 
+    /* a round's seeds and a scan's marks are counted in 32 bits */
+    {
+        std::deque<PendingQuery> q;
+        std::vector<SlotState> st(4);
+        fill(q);
+        Admission a(q, st);
+        a.take(50, 9); /* five seeds a query, three after sorting: 3 + 5, but not 6 + 5 */
+        CHECK(a.slots.size() == 2 && q.size() == 3 && q[0].ticket == 3);
+    }
+    {
+        std::deque<PendingQuery> q;
+        std::vector<SlotState> st(1);
+        fill(q);
+        Admission a(q, st);
+        a.take(50, 1); /* one query is always taken */
+        CHECK(a.slots.size() == 1);
+    }
+    for (uint32_t N : {1u, 31u, 1000u, 10000000u, (1u << 26) - 1}) {
+        const uint64_t g = mark_group(N);
+        CHECK(g >= 64 && g * N <= 0xffffffffull && g * slot_words(N) <= 0xf0000000ull);
+        CHECK((g + 1) * N > 0xffffffffull || (g + 1) * slot_words(N) > 0xf0000000ull);
+    }
+    CHECK(slot_words(1) == 8 && slot_words(256) == 8 && slot_words(257) == 16);
+
     std::unordered_map<uint64_t, FinishedQuery> done;
     done[2] = FinishedQuery();
     done[98] = FinishedQuery();

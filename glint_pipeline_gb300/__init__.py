@@ -162,8 +162,10 @@ class DeviceBench:
         (search_multi, cuda/geometry.cu:605-663), in bucket order."""
         p = np.ascontiguousarray(pids, dtype=np.uint32)
         n = ctypes.c_uint64()
-        # without a cap: room for a first guess, and once more where it is short
-        room = max(4096, 32 * p.shape[0]) if cap is None else int(cap)
+        # without a cap: room for a first guess, and once more where it is short.
+        # The guess is bounded: the room is also taken, and kept, on the device,
+        # and a kilobyte per listed object is 10 GB for 10M of them.
+        room = min(max(4096, 32 * p.shape[0]), 1 << 16) if cap is None else int(cap)
         while True:
             out = np.empty(room, dtype=SEARCH_DTYPE)
             st = self.lib.glint_active_search(self.h, p.ctypes.data_as(ctypes.c_void_p), p.shape[0],

@@ -1107,6 +1107,32 @@ def run_skew(args, local, K=None, W=None):
     return line
 
 
+def short_line(line):
+    """What the default run prints on standard output: the headline and one
+    number or two of each leg, about 3 KB.  The whole record (stages and
+    counters of every form, latencies per rate, per-step counts) is 24 KB,
+    more than a reader that keeps the end of the output may keep; it goes to
+    standard error."""
+    def pick(d, *names):
+        return {k: d[k] for k in names if k in d} if isinstance(d, dict) else d
+
+    out = {k: v for k, v in line.items()
+           if k not in ("roofline", "cpu_baseline", "parity", "serving", "compaction", "forms")}
+    out["roofline"] = pick(line["roofline"], "kernel", "kernel_stage", "slowest_stage", "bound", "achieved", "peak",
+                           "unit", "frac", "traffic", "traffic_unit", "algorithmic_bytes", "frac_step", "peak_source")
+    out["cpu_baseline"] = pick(line["cpu_baseline"], "value", "unit", "cores", "kind", "sample", "ms_per_step",
+                               "steps", "same_config")
+    out["parity"] = {k: dict(pick(v, "steps", "meetings"), mismatching_steps=v["mismatching_steps"][:16])
+                     for k, v in line["parity"].items()}
+    out["forms"] = {k: pick(v, "value", "ms_per_step", "error") for k, v in line["forms"].items()}
+    serve = line["serving"]
+    out["serving"] = dict(pick(serve, "rate_req_s", "qps", "p50_ms", "p99_ms", "queries", "finished", "error"),
+                          **{k: pick(serve[k], "p50_ms", "p99_ms") for k in ("two_hop_1k_seeds",) if k in serve}) \
+        if isinstance(serve, dict) else serve
+    out["compaction"] = pick(line["compaction"], "source_keys", "ms", "source_keys_per_s", "error")
+    return out
+
+
 def main():
     args = parse()
     rank, world, local, pg = dist_init()
@@ -1223,7 +1249,8 @@ def main():
                 "forms": dict({m: {k: v for k, v in f.items()} for m, f in forms.items()}, **other)}
         bad = {k: v["mismatching_steps"] for k, v in parity.items() if v.get("mismatching_steps")}
         line["parity_ok"] = not bad
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(short_line(line)), flush=True)
         if bad:
             # the line above carries the numbers; a run whose meetings differ fails
             print(f"meetings differ on steps {bad}", file=sys.stderr)

@@ -346,9 +346,9 @@ glint_status glint_create(const glint_config *cfg_in, const glint_box *mbr, cons
     cudaSetDevice(c->device);
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
-        /* the highest priority: the schema update's one-block stack replay
-         * needs 160 KB of shared memory on one SM, which identify's many
-         * short blocks would otherwise keep taking first */
+        /* the highest priority: two of the schema update's kernels are one
+         * block each, which would otherwise wait for a place among identify's
+         * many short blocks */
         int least = 0, greatest = 0;
         cudaDeviceGetStreamPriorityRange(&least, &greatest);
         e = cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, greatest);

@@ -116,11 +116,6 @@ struct NewEntry {
     unsigned long long prio;
 };
 
-struct SchemaEvent {
-    uint32_t node;
-    uint32_t kind;        /* 0 split, 1 merge */
-};
-
 /* one contact-tracing block (CTB) kept on the device: flushed, loaded from
  * files or compacted */
 struct StoreBlock {

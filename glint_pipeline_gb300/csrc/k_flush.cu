@@ -1269,9 +1269,9 @@ namespace glint {
  * each with its own mapping and device-wide wait (2M objects, 7M keys: 2.25 ms a
  * flush with them, 2.05 without); so did a merge (7.0 ms for 22M keys in three
  * blocks, 4.9 with one allocation of a pool and the oversize objects counted on
- * the device).  What the pool keeps of dropped blocks is
- * bounded by what flushes and merges hold for a moment anyway;
- * glint_serve_only empties it and it goes with the context. */
+ * the device).  Of dropped blocks the pool keeps at most twice the largest
+ * block's memory, which other allocations on the device do without until
+ * glint_serve_only empties it or the context goes. */
 cudaError_t store_block_alloc(glint_ctx *c, StoreBlock &b, size_t key_bytes, uint32_t C, uint64_t o_n) {
     cudaError_t e = cudaSuccess;
     if (!c->store_pool) {

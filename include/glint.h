@@ -56,7 +56,7 @@ typedef enum glint_status {
 #define GLINT_EF_SEGMENT_TOO_LARGE   0x0020u /* a leaf holds more objects than the sorter supports */
 #define GLINT_EF_DUPLICATE_NEW       0x0040u /* internal: a new key was inserted twice */
 #define GLINT_EF_DFS_OVERFLOW        0x0080u /* lookup depth beyond the supported tree depth */
-#define GLINT_EF_SCHEMA_WINDOW       0x0100u /* schema update took the slow path */
+#define GLINT_EF_SCHEMA_WINDOW       0x0100u /* no longer reported */
 #define GLINT_EF_TREE_DEPTH          0x0200u /* descent deeper than the supported tree depth */
 #define GLINT_EF_KV_OVERFLOW         0x0400u /* more keys pending than kv_capacity */
 #define GLINT_EF_STORE_DOMAIN        0x0800u /* a flush outside the reference's domain (see glint_flush) */
